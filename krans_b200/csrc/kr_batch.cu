@@ -131,8 +131,8 @@ struct BatchLaunch {
                  "krans_solve_batch: mixed precision needs matrices created with KRANS_CSR_FP32");
     const krans_mat *A = r.A;
     memset(&q, 0, sizeof q);
-    q.F = CsrView{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, tuned_lanes(A->ctx, A->m, A->nnz), A->ulen};
-    q.B = CsrView{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, tuned_lanes(A->ctx, A->n, A->nnz), A->ulenT};
+    q.F = csr_view(A, false);
+    q.B = csr_view(A, true);
     q.o = r.opts;
     q.o.team = KRANS_TEAM_CTA;
     int64_t kt = (r.opts.nullity_known >= 0) ? (int64_t)r.opts.nullity_known : r.opts.k;

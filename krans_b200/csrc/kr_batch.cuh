@@ -18,7 +18,7 @@ template <class Team> KR_DEV double team_max_residual(Team &tm, const CsrView &F
   for (int64_t i = 0; i < nf; i++) {
     const double *u = basis + i * ldb;
     double s2 = 0.0;
-    csr_mv(tm, F, F.v64, u, [&](int64_t, double s) { s2 += s * s; });
+    csr_mv<double>(tm, F, u, [&](int64_t, double s) { s2 += s * s; });
     mr = fmax(mr, sqrt(tm.sum1(s2)));
   }
   return mr;
@@ -130,9 +130,8 @@ __device__ __noinline__ void run_cta_request(TeamShared *sh, CyclicDesc *dp, con
     uint32_t dyn;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
     if (cta_cg_smem_bytes(rq.plan.ldm, rq.plan.ldn) <= (size_t)dyn) {
-      d.rp = reinterpret_cast<double2 *>(kr_dyn_smem);
-      d.Ap = reinterpret_cast<double *>(kr_dyn_smem + 16 * rq.plan.ldm);
-      d.tn = reinterpret_cast<double *>(kr_dyn_smem + 24 * rq.plan.ldm);
+      d.cgr = reinterpret_cast<double *>(kr_dyn_smem);
+      d.tn = reinterpret_cast<double *>(kr_dyn_smem + 8 * rq.plan.ldm);
     }
     rq.res->t_begin = globaltimer_ns();
   }

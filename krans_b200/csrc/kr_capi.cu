@@ -246,6 +246,48 @@ __global__ void gather_t_kernel(int64_t nnz, const int32_t *perm, const int32_t 
   }
 }
 
+// Sorted slices of a CSR operand (SlicedView): one block per window of
+// kSliceWindow rows ranks them by length, longest first (ties by row, so the
+// order is deterministic), and writes the slots' rows and the slices' widths.
+__global__ void __launch_bounds__(kSliceWindow) slice_sort_kernel(int64_t rows, const int32_t *rp, int32_t *row,
+                                                                  int32_t *width) {
+  __shared__ int32_t len[kSliceWindow];
+  const int t = threadIdx.x;
+  const int64_t w0 = (int64_t)blockIdx.x * kSliceWindow, i = w0 + t;
+  const int here = (int)imin64(kSliceWindow, rows - w0);
+  const int32_t mine = t < here ? rp[i + 1] - rp[i] : -1;
+  len[t] = mine;
+  __syncthreads();
+  int rank = 0;
+  for (int j = 0; j < kSliceWindow; j++)
+    rank += len[j] > mine || (len[j] == mine && j < t);
+  if (w0 + (rank & ~31) < rows) { // the last window's slices past the last row do not exist
+    row[w0 + rank] = t < here ? (int32_t)i : -1;
+    if ((rank & 31) == 0)
+      width[(w0 + rank) >> 5] = mine;
+  }
+}
+// the rounds of every slice, a warp per slice
+__global__ void slice_fill_kernel(int64_t slices, const int32_t *off, const int32_t *row, const int32_t *rp,
+                                  const int32_t *ci, const double *v, int32_t *sci, double *sv, float *sv32) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t s = w; s < slices; s += nw) {
+    const int32_t r = row[s * 32 + lane];
+    const int32_t b = r >= 0 ? rp[r] : 0, len = r >= 0 ? rp[r + 1] - b : 0;
+    const int32_t o0 = off[s], o1 = off[s + 1];
+    for (int32_t j = 0; j < o1 - o0; j++) {
+      const size_t k = (size_t)(o0 + j) * 32 + lane;
+      const double x = j < len ? v[b + j] : 0.0;
+      sci[k] = j < len ? ci[b + j] : 0;
+      sv[k] = x;
+      if (sv32)
+        sv32[k] = (float)x;
+    }
+  }
+}
+
 __global__ void rng_mt_kernel(RngState *st, double *out, int64_t n) { block_mt_normals(st, out, n); }
 __global__ void rng_philox_kernel(RngState *st, double *out, int64_t n) {
   const uint64_t key = st->philox_key, base = st->philox_ctr;
@@ -267,11 +309,30 @@ void preload_capi_kernels() {
                       (const void *)to_f32_kernel,      (const void *)col_count_kernel,
                       (const void *)scan_kernel,        (const void *)scatter_kernel,
                       (const void *)row_sort_kernel,    (const void *)row_of_kernel,
-                      (const void *)gather_t_kernel,    (const void *)rng_mt_kernel,
+                      (const void *)gather_t_kernel,    (const void *)slice_sort_kernel,
+                      (const void *)slice_fill_kernel,  (const void *)rng_mt_kernel,
                       (const void *)rng_philox_kernel,  (const void *)rng_philox_advance};
   for (const void *k : ks)
     preload(k);
 }
+
+// Room of an operand's sorted slices. A slice is as wide as its longest row;
+// within a window sorted by length, every slice after the first is no wider
+// than the shortest row before it, so the padding of a window is at most 32
+// times its longest row.
+struct SliceSize {
+  int32_t longest = 0;
+  int64_t window_max = 0, sum_max = 0;
+  void row(int64_t i, int32_t len) {
+    if (i % kSliceWindow == 0) {
+      sum_max += window_max;
+      window_max = 0;
+    }
+    window_max = std::max<int64_t>(window_max, len);
+    longest = std::max(longest, len);
+  }
+  int64_t padding() const { return 32 * (sum_max + window_max); }
+};
 
 static int grid_for(krans_ctx *ctx, int64_t n, int threads = 256) {
   int64_t b = (n + threads - 1) / threads;
@@ -509,10 +570,12 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   // columns (range, per-column counts for the transpose's uniform length)
   const int64_t L = m > 0 ? (int64_t)(row_ptr[1] - row_ptr[0]) : 0;
   bool uni = m > 0 && L > 0 && L <= 8;
+  SliceSize szA, szT; // room that sorted slices of A and of its transpose take
   for (int64_t i = 0; i < m; i++) {
     const int32_t len = row_ptr[i + 1] - row_ptr[i];
     KR_CHECK_ARG(len >= 0, "krans_csr_create: row_ptr not monotone");
     uni = uni && len == L;
+    szA.row(i, len);
   }
   std::vector<int32_t> cc((size_t)n, 0);
   for (int64_t k = 0; k < nnz; k++) {
@@ -522,8 +585,10 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   }
   const int32_t LT = n > 0 ? cc[0] : 0;
   bool uniT = n > 0 && LT > 0 && LT <= 8;
-  for (int64_t j = 0; uniT && j < n; j++)
-    uniT = cc[(size_t)j] == LT;
+  for (int64_t j = 0; j < n; j++) {
+    uniT = uniT && cc[(size_t)j] == LT;
+    szT.row(j, cc[(size_t)j]);
+  }
   if (!(flags & (KRANS_CSR_FP64 | KRANS_CSR_FP32)))
     flags |= KRANS_CSR_FP64;
   flags |= KRANS_CSR_FP64; // FP64 values are kept for every path (polish, residuals)
@@ -533,7 +598,15 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   const size_t sz_v = (size_t)std::max<int64_t>(nnz, 1) * 8, sz_v32 = (size_t)std::max<int64_t>(nnz, 1) * 4;
   // the stored arrays share one allocation (carved at 256-byte offsets)
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const size_t total = up(sz_rp) + 2 * up(sz_ci) + 2 * up(sz_v) + up(sz_rpT) + (f32 ? 2 * up(sz_v32) : 0);
+  // rows of exactly 2 entries are read with vector loads as they are
+  const bool sl = nnz > 0 && !(uni && L == 2) && szA.longest <= kSliceMaxLen;
+  const bool slT = nnz > 0 && !(uniT && LT == 2) && szT.longest <= kSliceMaxLen;
+  auto slice_bytes = [&](int64_t rows, const SliceSize &z) {
+    const size_t slots = (size_t)((rows + 31) / 32) * 32, e = (size_t)(nnz + z.padding());
+    return up(slots * 4) + up((slots / 32 + 1) * 4) + up(e * 4) + up(e * 8) + (f32 ? up(e * 4) : 0);
+  };
+  const size_t total = up(sz_rp) + 2 * up(sz_ci) + 2 * up(sz_v) + up(sz_rpT) + (f32 ? 2 * up(sz_v32) : 0) +
+                       (sl ? slice_bytes(m, szA) : 0) + (slT ? slice_bytes(n, szT) : 0);
   char *base = nullptr;
   int rc = dev_alloc(ctx, (void **)&base, total);
   if (rc != KRANS_OK)
@@ -561,15 +634,30 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
     A->v32 = (float *)take(sz_v32);
     A->vT32 = (float *)take(sz_v32);
   }
+  auto take_slices = [&](int64_t rows, const SliceSize &z, SlicedView &S) {
+    const size_t nsl = (size_t)((rows + 31) / 32), e = (size_t)(nnz + z.padding());
+    S.slices = (int32_t)nsl;
+    S.row = (int32_t *)take(nsl * 32 * 4);
+    S.off = (int32_t *)take((nsl + 1) * 4);
+    S.ci = (int32_t *)take(e * 4);
+    S.v64 = (double *)take(e * 8);
+    S.v32 = f32 ? (float *)take(e * 4) : nullptr;
+  };
+  if (sl)
+    take_slices(m, szA, A->sl);
+  if (slT)
+    take_slices(n, szT, A->slT);
   // scratch of the device transpose: stream-ordered, so releasing it does not
   // wait for the device, and the next matrix's host work overlaps this
   // matrix's transpose kernels
   cudaStream_t s = ctx->stream;
   int32_t *scratch = nullptr;
-  const size_t sz_scr = up(sz_rpT) + 3 * up(sz_ci);
+  const size_t sz_w = up((size_t)(std::max(m, n) / 32 + 1) * 4); // slice widths, one operand at a time
+  const size_t sz_scr = up(sz_rpT) + 3 * up(sz_ci) + sz_w;
   cudaError_t e = cudaMallocAsync((void **)&scratch, sz_scr, s);
   int32_t *cnt = scratch, *perm = (int32_t *)((char *)scratch + up(sz_rpT));
   int32_t *tmp = (int32_t *)((char *)perm + up(sz_ci)), *rowof = (int32_t *)((char *)tmp + up(sz_ci));
+  int32_t *width = (int32_t *)((char *)rowof + up(sz_ci));
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(A->rp, row_ptr, sz_rp, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && nnz)
@@ -597,6 +685,18 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
       to_f32_kernel<<<g, 256, 0, s>>>(nnz, A->v, A->v32);
       to_f32_kernel<<<g, 256, 0, s>>>(nnz, A->vT, A->vT32);
     }
+    auto fill = [&](int64_t rows, const int32_t *rp, const int32_t *ci, const double *v, const SlicedView &S) {
+      int32_t *off = const_cast<int32_t *>(S.off), *row = const_cast<int32_t *>(S.row);
+      slice_sort_kernel<<<(unsigned)((rows + kSliceWindow - 1) / kSliceWindow), kSliceWindow, 0, s>>>(rows, rp, row, width);
+      scan_kernel<<<1, 1024, 0, s>>>(S.slices, width, off);
+      slice_fill_kernel<<<grid_for(ctx, (int64_t)S.slices * 32), 256, 0, s>>>(
+          S.slices, off, row, rp, ci, v, const_cast<int32_t *>(S.ci), const_cast<double *>(S.v64),
+          const_cast<float *>(S.v32));
+    };
+    if (sl)
+      fill(m, A->rp, A->ci, A->v, A->sl);
+    if (slT)
+      fill(n, A->rpT, A->ciT, A->vT, A->slT);
   } else if (e == cudaSuccess) {
     e = cudaMemsetAsync(A->rpT, 0, sz_rpT, s);
   }

@@ -57,24 +57,24 @@ template <class Team, class KT> struct CyclicSolver {
   }
 
   // y = F x (FP64)
-  KR_DEV void mulF(const double *x, double *y) {
-    csr_mv(tm, d.F, d.F.v64, x,
+  __device__ __noinline__ void mulF(const double *x, double *y) {
+    csr_mv<double>(tm, d.F, x,
               [&](int64_t i, double s) { y[i] = s; });
     count_F();
     c.bytes += spmv_bytes(d.F.rows, d.F.cols, d.F.nnz, 8, 8, 8);
     tm.sync();
   }
-  KR_DEV void mulB(const double *x, double *y) {
-    csr_mv(tm, d.B, d.B.v64, x,
+  __device__ __noinline__ void mulB(const double *x, double *y) {
+    csr_mv<double>(tm, d.B, x,
               [&](int64_t i, double s) { y[i] = s; });
     count_B();
     c.bytes += spmv_bytes(d.B.rows, d.B.cols, d.B.nnz, 8, 8, 8);
     tm.sync();
   }
   // ||F x|| with y = F x stored (fused norm)
-  KR_DEV double mulF_norm(const double *x, double *y) {
+  __device__ __noinline__ double mulF_norm(const double *x, double *y) {
     double s2 = 0.0;
-    csr_mv(tm, d.F, d.F.v64, x, [&](int64_t i, double s) {
+    csr_mv<double>(tm, d.F, x, [&](int64_t i, double s) {
       y[i] = s;
       s2 += s * s;
     });
@@ -83,21 +83,21 @@ template <class Team, class KT> struct CyclicSolver {
     return sqrt(tm.sum1(s2)); // the reduction's barrier also publishes y
   }
 
-  KR_DEV double nrm2(int64_t len, const double *x) {
+  __device__ __noinline__ double nrm2(int64_t len, const double *x) {
     c.bytes += 8.0 * len;
     return team_nrm2(tm, len, x);
   }
-  KR_DEV void scale(int64_t len, double a, double *x) {
+  __device__ __noinline__ void scale(int64_t len, double a, double *x) {
     team_for(tm, len, [&](int64_t i) { x[i] *= a; });
     c.bytes += 16.0 * len;
     tm.sync();
   }
-  KR_DEV void copy(int64_t len, const double *s, double *dd) {
+  __device__ __noinline__ void copy(int64_t len, const double *s, double *dd) {
     team_for(tm, len, [&](int64_t i) { dd[i] = s[i]; });
     c.bytes += 16.0 * len;
     tm.sync();
   }
-  KR_DEV void random(double *out) {
+  __device__ __noinline__ void random(double *out) {
     team_random_normal(tm, d.rng, out, n);
     c.bytes += 8.0 * n;
   }
@@ -114,7 +114,7 @@ template <class Team, class KT> struct CyclicSolver {
     }
   }
   // one CGS pass of w (len) against ns stored vectors S (type TS)
-  template <class TS, class TW> KR_DEV void cgs_pass(int64_t len, const TS *S, int64_t ld, int ns, TW *w) {
+  template <class TS, class TW> __device__ __noinline__ void cgs_pass(int64_t len, const TS *S, int64_t ld, int ns, TW *w) {
     if (ns == 0)
       return;
     team_multidot(tm, len, S, ld, ns, w);
@@ -134,13 +134,70 @@ template <class Team, class KT> struct CyclicSolver {
     return sqrt(sum2 / (double)samples);
   }
 
-  // CG on (F F^T) w = rhs (CyclicLanczosSolver.cpp:48-113), no preconditioner.
-  // The callers only use F^T w, so this returns u = F^T w instead of w: u
-  // accumulates alpha_k F^T p_k, and F^T p_k is the vector the first SpMV of
-  // iteration k forms anyway. The m-vector w and the closing F^T w product
-  // are never needed (same value in exact arithmetic; rounding differs).
-  // r and p are stored interleaved, so the gather of r + beta p at each entry
-  // of F^T is one 16-byte load.
+  // What the first SpMV's epilogue of a CG iteration combines with its row sum.
+  struct TU {
+    double t, u;
+  };
+  // CG on (F F^T) w = rhs (CyclicLanczosSolver.cpp:48-113), without and with
+  // a preconditioner. The callers only use F^T w, so this returns u = F^T w
+  // instead of w, and it carries t = F^T p in place of the direction p
+  // (Craig's form of CG for A A^T, CGNE in Saad, Iterative Methods for Sparse
+  // Linear Systems, 2nd ed., 8.3.2): with p <- z + beta p,
+  //   t <- F^T z + beta t,  p . F F^T p = t . t,  u += alpha t,  r -= alpha F t,
+  // the same iterates in exact arithmetic. The m-vectors w, p and F F^T p do
+  // not exist, and an iteration is two SpMV passes with everything else in
+  // their prologues and epilogues, each ended by one reduction:
+  //   t_i = (F^T z)_i + beta t_i, u_i += alpha_prev t_i (old), sum t_i^2
+  //   r_i -= alpha (F t)_i, sum r_i^2
+  // Bound by the latency and sector rate of the gathers of one SM's L1/L2
+  // path (DRAM is idle: the vectors and matrices sit in L2). An iteration on an
+  // incidence matrix: 37.2 -> 24.5 us at 4000 columns on one block, 72.7 -> 51.7
+  // us at 13877 on two, 97 -> 73 us at 60000 on eight (with the sorted slices).
+  //
+  // One iteration's first pass: t and sum t^2 (the team's total; its barrier
+  // publishes t), with t and u by slot of F^T's sorted order in ts and us.
+  // `first`: ts and us are not read.
+  __device__ __noinline__ double cg_pass_t(const double *z, double *t, double *ts, double *us, double beta,
+                                           double alpha_prev, bool first) {
+    double tt = 0.0;
+    csr_mv_pre<double>(
+        tm, d.B, [&](int32_t cc) { return z[cc]; },
+        [&](int, int slot) { return first ? TU{0.0, 0.0} : TU{ts[slot], us[slot]}; },
+        [&](int row, int slot, double s, TU o) {
+          const double ti = s + beta * o.t;
+          t[row] = ti;
+          ts[slot] = ti;
+          us[slot] = o.u + alpha_prev * o.t;
+          tt += ti * ti;
+        });
+    count_B();
+    c.bytes += spmv_bytes(d.B.rows, d.B.cols, d.B.nnz, 8, 8, 8) + 24.0 * n;
+    return tm.sum1(tt);
+  }
+  // the second pass: r -= alpha F t, and this thread's share of sum r^2
+  __device__ __noinline__ double cg_pass_r(const double *t, double *r, double alpha) {
+    double rr = 0.0;
+    csr_mv_pre<double>(
+        tm, d.F, [&](int32_t cc) { return t[cc]; },
+        [&](int i, int) { return r[i]; },
+        [&](int i, int, double s, double ro) {
+          const double ri = ro - alpha * s;
+          r[i] = ri;
+          rr += ri * ri;
+        });
+    count_F();
+    c.bytes += spmv_bytes(d.F.rows, d.F.cols, d.F.nnz, 8, 8, 8) + 8.0 * m;
+    return rr;
+  }
+  // u by row; `pending`: with the last iteration's alpha t, which no further
+  // first pass applies
+  __device__ __noinline__ void cg_result(const double *ts, const double *us, bool pending, double alpha, double *u) {
+    const int32_t *row = d.B.sl.slices ? d.B.sl.row : nullptr;
+    team_for(tm, n, [&](int64_t p) { u[row ? row[p] : p] = pending ? us[p] + alpha * ts[p] : us[p]; });
+    c.bytes += 24.0 * n;
+    tm.sync();
+  }
+
   // `precond`: use the request's precond_aat (the candidate polish does; the
   // random-projector fallback of try_project_random does not,
   // CyclicLanczosSolver.cpp:140-214).
@@ -148,8 +205,7 @@ template <class Team, class KT> struct CyclicSolver {
                                      double *rnorm_out, bool precond = true) {
     if (precond && d.o.precond_aat != KRANS_PRECOND_NONE)
       return cg_pre(rhs, u, maxit, rel_tol, bd_tol, rnorm_out);
-    double2 *rp = d.rp;
-    double *Ap = d.Ap, *tn = d.tn;
+    double *r = d.cgr, *t = d.tn, *ts = d.cgts, *us = d.cgus;
     double rr = 0.0;
     team_for(tm, n, [&](int64_t i) { u[i] = 0.0; });
     team_for4(tm, m, [&](const int64_t *ix, int cnt) {
@@ -161,12 +217,12 @@ template <class Team, class KT> struct CyclicSolver {
 #pragma unroll
       for (int u4 = 0; u4 < 4; u4++)
         if (u4 < cnt) {
-          rp[ix[u4]] = make_double2(xv[u4], xv[u4]);
+          r[ix[u4]] = xv[u4];
           rr += xv[u4] * xv[u4];
         }
     });
     rr = tm.sum1(rr);
-    c.bytes += 24.0 * m + 8.0 * n;
+    c.bytes += 16.0 * m + 8.0 * n;
     const double rhsn = sqrt(rr > 0.0 ? rr : 0.0);
     *rnorm_out = rhsn;
     if (!(rhsn > 0.0) || !isfinite(rhsn))
@@ -179,70 +235,18 @@ template <class Team, class KT> struct CyclicSolver {
     *rnorm_out = rnorm;
     if (rnorm <= tol)
       return 0;
-    // p = r at entry. Each iteration first forms p <- r + beta p; that
-    // update is folded into the gather of the first SpMV (t = F^T p) and into
-    // the epilogue of the second (which stores p), so CG needs no separate
-    // pass over p (fma(beta, p, r) in both places: the same values).
     int64_t k = 0;
-    double beta = 0.0;
+    double beta = 0.0, alpha = 0.0;
+    bool started = false, pending = false; // us and ts hold values; us lacks alpha t of the last iteration
     for (; k < maxit && tm.ok(); ++k) {
-      const double bq = beta;
-      team_spmv_x(
-          tm, d.B.rows, d.B.rp, d.B.ci, d.B.v64,
-          [&](int32_t cc) {
-            const double2 q = rp[cc];
-            return q.x + bq * q.y;
-          },
-          d.B.lanes, d.B.ulen, [&](int64_t i, double s) { tn[i] = s; });
-      count_B();
-      c.bytes += spmv_bytes(d.B.rows, d.B.cols, d.B.nnz, 8, 16, 8);
-      tm.sync();
-      double pap = 0.0;
-      csr_mv(tm, d.F, d.F.v64, tn, [&](int64_t i, double s) {
-        const double2 q = rp[i];
-        const double pn = q.x + bq * q.y;
-        rp[i].y = pn;
-        Ap[i] = s;
-        pap += pn * s;
-      });
-      count_F();
-      c.bytes += spmv_bytes(d.F.rows, d.F.cols, d.F.nnz, 8, 8, 8) + 24.0 * m;
-      pap = tm.sum1(pap);
+      const double pap = cg_pass_t(r, t, ts, us, beta, alpha, k == 0);
+      started = true;
+      pending = false;
       if (!isfinite(pap) || fabs(pap) <= bd_tol)
         break;
-      const double alpha = rz / pap;
-      double rzn = 0.0;
-      team_for4(tm, m, [&](const int64_t *ix, int cnt) {
-        double rv[4], av[4];
-#pragma unroll
-        for (int u4 = 0; u4 < 4; u4++)
-          if (u4 < cnt) {
-            rv[u4] = rp[ix[u4]].x;
-            av[u4] = Ap[ix[u4]];
-          }
-#pragma unroll
-        for (int u4 = 0; u4 < 4; u4++)
-          if (u4 < cnt) {
-            const double ri = rv[u4] - alpha * av[u4];
-            rp[ix[u4]].x = ri;
-            rzn += ri * ri;
-          }
-      });
-      team_for4(tm, n, [&](const int64_t *ix, int cnt) {
-        double uv[4], tv[4];
-#pragma unroll
-        for (int u4 = 0; u4 < 4; u4++)
-          if (u4 < cnt) {
-            uv[u4] = u[ix[u4]];
-            tv[u4] = tn[ix[u4]];
-          }
-#pragma unroll
-        for (int u4 = 0; u4 < 4; u4++)
-          if (u4 < cnt)
-            u[ix[u4]] = uv[u4] + alpha * tv[u4];
-      });
-      rzn = tm.sum1(rzn); // its barrier also publishes r for the next gather
-      c.bytes += 24.0 * m + 24.0 * n;
+      alpha = rz / pap;
+      pending = true;
+      const double rzn = tm.sum1(cg_pass_r(t, r, alpha)); // its barrier also publishes r for the next gather
       if (!isfinite(rzn))
         break;
       rnorm = sqrt(rzn > 0.0 ? rzn : 0.0);
@@ -253,6 +257,8 @@ template <class Team, class KT> struct CyclicSolver {
       beta = rzn / fmax(1e-300, rz);
       rz = rzn;
     }
+    if (started)
+      cg_result(ts, us, pending, alpha, u);
     *rnorm_out = rnorm;
     return k;
   }
@@ -271,20 +277,20 @@ template <class Team, class KT> struct CyclicSolver {
     tm.sync();
   }
 
-  // z = M^-1 r into zp[i].x: Jacobi (z = r / diag(F F^T)) or precond_steps
+  // z = M^-1 r: Jacobi (z = r / diag(F F^T)) or precond_steps
   // steps of steepest descent on F F^T from z = 0 (the precond_AAt callback of
   // tests/test_cyclic_lanczos.cpp:339-377: residual and direction coincide at
   // the start of each step, so one vector q carries both)
-  __device__ __noinline__ void apply_precond(const double *r, double2 *zp) {
+  __device__ __noinline__ void apply_precond(const double *r, double *z) {
     if (d.o.precond_aat == KRANS_PRECOND_JACOBI) {
-      team_for(tm, m, [&](int64_t i) { zp[i].x = d.dinv[i] * r[i]; });
-      c.bytes += 32.0 * m;
+      team_for(tm, m, [&](int64_t i) { z[i] = d.dinv[i] * r[i]; });
+      c.bytes += 24.0 * m;
       tm.sync();
       return;
     }
     double *q = d.sd_q, *Oq = d.sd_Oq, *tn = d.tn;
     team_for(tm, m, [&](int64_t i) {
-      zp[i].x = 0.0;
+      z[i] = 0.0;
       q[i] = r[i];
     });
     c.bytes += 24.0 * m;
@@ -292,7 +298,7 @@ template <class Team, class KT> struct CyclicSolver {
     for (int it = 0; it < d.o.precond_steps && tm.ok(); it++) {
       mulB(q, tn);
       double acc[2] = {0.0, 0.0}; // q.Oq, q.q
-      csr_mv(tm, d.F, d.F.v64, tn, [&](int64_t i, double s) {
+      csr_mv<double>(tm, d.F, tn, [&](int64_t i, double s) {
         Oq[i] = s;
         const double qi = q[i];
         acc[0] += qi * s;
@@ -307,7 +313,7 @@ template <class Team, class KT> struct CyclicSolver {
       double q2 = 0.0;
       team_for(tm, m, [&](int64_t i) {
         const double qi = q[i];
-        zp[i].x += alpha * qi;
+        z[i] += alpha * qi;
         const double qn = qi - alpha * Oq[i];
         q[i] = qn;
         q2 += qn * qn;
@@ -320,13 +326,10 @@ template <class Team, class KT> struct CyclicSolver {
   }
 
   // Preconditioned CG (cg_normal_eq_prec, CyclicLanczosSolver.cpp:48-113):
-  // z = M^-1 r, rz = r.z, p = z, tolerance on sqrt(r.z); otherwise as cg()
-  // (u = F^T w returned, direction update folded into the SpMVs, z and p
-  // interleaved for the gather of z + beta p).
+  // z = M^-1 r, rz = r.z, p = z, tolerance on sqrt(r.z); otherwise as cg().
   __device__ __noinline__ int64_t cg_pre(const double *rhs, double *u, int64_t maxit, double rel_tol,
                                          double bd_tol, double *rnorm_out) {
-    double2 *zp = d.rp;
-    double *r = d.r_pre, *Ap = d.Ap, *tn = d.tn;
+    double *z = d.cgr, *r = d.r_pre, *t = d.cgt, *ts = d.cgts, *us = d.cgus;
     double rr = 0.0;
     team_for(tm, n, [&](int64_t i) { u[i] = 0.0; });
     team_for(tm, m, [&](int64_t i) {
@@ -340,15 +343,11 @@ template <class Team, class KT> struct CyclicSolver {
     *rnorm_out = rhsn;
     if (!(rhsn > 0.0) || !isfinite(rhsn))
       return 0;
-    apply_precond(r, zp);
+    apply_precond(r, z);
     double rz = 0.0;
-    team_for(tm, m, [&](int64_t i) {
-      const double z = zp[i].x;
-      zp[i].y = z;
-      rz += r[i] * z;
-    });
+    team_for(tm, m, [&](int64_t i) { rz += r[i] * z[i]; });
     rz = tm.sum1(rz);
-    c.bytes += 32.0 * m;
+    c.bytes += 16.0 * m;
     if (!(rz > 0.0) || !isfinite(rz))
       return 0;
     double rnorm = sqrt(rz);
@@ -357,40 +356,21 @@ template <class Team, class KT> struct CyclicSolver {
     if (rnorm <= tol)
       return 0;
     int64_t k = 0;
-    double beta = 0.0;
+    double beta = 0.0, alpha = 0.0;
+    bool started = false, pending = false;
     for (; k < maxit && tm.ok(); ++k) {
-      const double bq = beta;
-      team_spmv_x(
-          tm, d.B.rows, d.B.rp, d.B.ci, d.B.v64,
-          [&](int32_t cc) {
-            const double2 q = zp[cc];
-            return q.x + bq * q.y;
-          },
-          d.B.lanes, d.B.ulen, [&](int64_t i, double s) { tn[i] = s; });
-      count_B();
-      c.bytes += spmv_bytes(d.B.rows, d.B.cols, d.B.nnz, 8, 16, 8);
-      tm.sync();
-      double pap = 0.0;
-      csr_mv(tm, d.F, d.F.v64, tn, [&](int64_t i, double s) {
-        const double2 q = zp[i];
-        const double pn = q.x + bq * q.y;
-        zp[i].y = pn;
-        Ap[i] = s;
-        pap += pn * s;
-      });
-      count_F();
-      c.bytes += spmv_bytes(d.F.rows, d.F.cols, d.F.nnz, 8, 8, 8) + 24.0 * m;
-      pap = tm.sum1(pap);
+      const double pap = cg_pass_t(z, t, ts, us, beta, alpha, k == 0);
+      started = true;
+      pending = false;
       if (!isfinite(pap) || fabs(pap) <= bd_tol)
         break;
-      const double alpha = rz / pap;
-      team_for(tm, m, [&](int64_t i) { r[i] -= alpha * Ap[i]; });
-      team_for(tm, n, [&](int64_t i) { u[i] += alpha * tn[i]; });
-      c.bytes += 24.0 * m + 24.0 * n;
+      alpha = rz / pap;
+      pending = true;
+      (void)cg_pass_r(t, r, alpha);
       tm.sync();
-      apply_precond(r, zp);
+      apply_precond(r, z);
       double rzn = 0.0;
-      team_for(tm, m, [&](int64_t i) { rzn += r[i] * zp[i].x; });
+      team_for(tm, m, [&](int64_t i) { rzn += r[i] * z[i]; });
       rzn = tm.sum1(rzn); // its barrier also publishes z for the next gather
       c.bytes += 16.0 * m;
       if (!isfinite(rzn))
@@ -403,6 +383,8 @@ template <class Team, class KT> struct CyclicSolver {
       beta = rzn / fmax(1e-300, rz);
       rz = rzn;
     }
+    if (started)
+      cg_result(ts, us, pending, alpha, u);
     *rnorm_out = rnorm;
     return k;
   }
@@ -740,7 +722,7 @@ template <class Team, class KT> struct CyclicSolver {
   }
 
   // candidate v = sum_q coef_q Y[q] (CyclicLanczosSolver.cpp:496-503)
-  KR_DEV void form_candidate(const KT *Y, bool split, int l, int jb, int ny_used, double *v) {
+  __device__ __noinline__ void form_candidate(const KT *Y, bool split, int l, int jb, int ny_used, double *v) {
     for (int q = threadIdx.x; q < ny_used; q += blockDim.x)
       tm.sh->h[q] = coef(split, l, jb, q);
     __syncthreads();
@@ -808,7 +790,7 @@ template <class Team, class KT> struct CyclicSolver {
         ++tested;
         // residual, with F v stored as column g of the block right-hand side
         double s2 = 0.0;
-        csr_mv(tm, d.F, d.F.v64, vg, [&](int64_t i, double s) {
+        csr_mv<double>(tm, d.F, vg, [&](int64_t i, double s) {
           Hb[i * KR_NBP + g] = s;
           s2 += s * s;
         });
@@ -928,6 +910,27 @@ template <class Team, class KT> struct CyclicSolver {
     }
   }
 
+  // the Golub-Kahan products with their -beta x update: wx = F y - beta xp
+  // (sub: with the second term), wy = F^T x - beta yp
+  __device__ __noinline__ void gk_F(const KT *y, const KT *xp, bool sub, KT beta, KT *wx) {
+    using Acc = typename AccOf<KT>::T;
+    csr_mv_pre<KT>(
+        tm, d.F, [&](int32_t cc) { return y[cc]; }, [&](int i, int) { return sub ? xp[i] : KT(0); },
+        [&](int i, int, Acc s, KT x0) { wx[i] = sub ? (KT)(s - (Acc)beta * (Acc)x0) : (KT)s; });
+    count_F();
+    c.bytes += spmv_bytes(m, n, d.F.nnz, sizeof(KT), sizeof(KT), sizeof(KT)) + (sub ? sizeof(KT) * (double)m : 0.0);
+    tm.sync();
+  }
+  __device__ __noinline__ void gk_B(const KT *x, const KT *yp, KT beta, KT *wy) {
+    using Acc = typename AccOf<KT>::T;
+    csr_mv_pre<KT>(
+        tm, d.B, [&](int32_t cc) { return x[cc]; }, [&](int i, int) { return yp[i]; },
+        [&](int i, int, Acc s, KT y0) { wy[i] = (KT)(s - (Acc)beta * (Acc)y0); });
+    count_B();
+    c.bytes += spmv_bytes(n, m, d.B.nnz, sizeof(KT), sizeof(KT), sizeof(KT)) + sizeof(KT) * (double)n;
+    tm.sync();
+  }
+
   __device__ __noinline__ void run() {
     const krans_cyclic_opts &o = d.o;
     KT *Y = (KT *)d.Y, *X = (KT *)d.X, *wx = (KT *)d.wx, *wy = (KT *)d.wy;
@@ -982,37 +985,11 @@ template <class Team, class KT> struct CyclicSolver {
       for (int64_t j = 0; j < ncv && tm.ok(); ++j) {
         const bool from_y = nY > nX;
         if (from_y) {
-          const KT *yj = Y + (int64_t)(nY - 1) * ldn;
-          const KT *xp = X + (int64_t)(nX > 0 ? nX - 1 : 0) * ldm;
-          const KT bp = (KT)(nbeta > 0 ? beta_prev : 0.0);
-          const bool sub = nbeta > 0;
-          if constexpr (sizeof(KT) == 8) {
-            csr_mv(tm, d.F, d.F.v64, yj,
-                      [&](int64_t i, double s) { wx[i] = sub ? (KT)(s - (double)bp * (double)xp[i]) : (KT)s; });
-          } else {
-            csr_mv(tm, d.F, d.F.v32, yj,
-                      [&](int64_t i, float s) { wx[i] = sub ? (KT)(s - (float)bp * (float)xp[i]) : (KT)s; });
-          }
-          count_F();
-          c.bytes += spmv_bytes(m, n, d.F.nnz, sizeof(KT), sizeof(KT), sizeof(KT)) +
-                     (sub ? sizeof(KT) * (double)m : 0.0);
-          tm.sync();
+          gk_F(Y + (int64_t)(nY - 1) * ldn, X + (int64_t)(nX > 0 ? nX - 1 : 0) * ldm, nbeta > 0, (KT)beta_prev, wx);
           for (int pass = 0; pass < o.reorth; ++pass)
             cgs_pass(m, X, ldm, nX, wx);
         } else {
-          const KT *xj = X + (int64_t)(nX - 1) * ldm;
-          const KT *yp = Y + (int64_t)(nY - 1) * ldn;
-          const KT bp = (KT)beta_prev;
-          if constexpr (sizeof(KT) == 8) {
-            csr_mv(tm, d.B, d.B.v64, xj,
-                      [&](int64_t i, double s) { wy[i] = (KT)(s - (double)bp * (double)yp[i]); });
-          } else {
-            csr_mv(tm, d.B, d.B.v32, xj,
-                      [&](int64_t i, float s) { wy[i] = (KT)(s - (float)bp * (float)yp[i]); });
-          }
-          count_B();
-          c.bytes += spmv_bytes(n, m, d.B.nnz, sizeof(KT), sizeof(KT), sizeof(KT)) + sizeof(KT) * (double)n;
-          tm.sync();
+          gk_B(X + (int64_t)(nX - 1) * ldm, Y + (int64_t)(nY - 1) * ldn, (KT)beta_prev, wy);
           for (int pass = 0; pass < o.reorth; ++pass) {
             cgs_pass(n, d.basis, d.ldb, (int)nb, wy);
             cgs_pass(n, Y, ldn, nY, wy);

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/krans_cuda.h"
+#include "kr_types.cuh"
 
 #include <cstdlib>
 
@@ -76,6 +77,7 @@ struct krans_mat {
   float *v32 = nullptr, *vT32 = nullptr;
   int lanes = 1, lanesT = 1;
   int32_t ulen = 0, ulenT = 0; // uniform row length of A / A^T (0 = not uniform)
+  kr::SlicedView sl{}, slT{};  // sorted slices of A / A^T for the solvers (slices = 0: not kept)
   krans_spmv_tuning tune{}, tuneT{}; // standalone SpMV kernel of A / A^T (zero: automatic)
   char *base = nullptr;         // one device allocation holding every stored array
   size_t bytes = 0;
@@ -146,5 +148,13 @@ inline int tuned_lanes(const krans_ctx *ctx, int64_t rows, int64_t nnz) {
   while (b < 5 && mean > bound[b])
     b++;
   return ctx->tune.lanes[b];
+}
+// A (or its stored transpose) as the solvers' device code sees it
+inline CsrView csr_view(const krans_mat *A, bool trans) {
+  if (trans)
+    return CsrView{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, tuned_lanes(A->ctx, A->n, A->nnz), A->ulenT,
+                   A->slT};
+  return CsrView{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, tuned_lanes(A->ctx, A->m, A->nnz), A->ulen,
+                 A->sl};
 }
 } // namespace kr

@@ -38,20 +38,20 @@ template <class Team> struct LobpcgSolver {
 
   // ---- primitives ---------------------------------------------------------
   KR_DEV void mulA(const double *x, double *y) {
-    csr_mv(tm, d.F, d.F.v64, x, [&](int64_t i, double s) { y[i] = s; });
+    csr_mv<double>(tm, d.F, x, [&](int64_t i, double s) { y[i] = s; });
     c.spmv++;
     c.bytes += spmv_bytes(m, n, d.F.nnz, 8, 8, 8);
     tm.sync();
   }
   KR_DEV void mulAT(const double *x, double *y) {
-    csr_mv(tm, d.B, d.B.v64, x, [&](int64_t i, double s) { y[i] = s; });
+    csr_mv<double>(tm, d.B, x, [&](int64_t i, double s) { y[i] = s; });
     c.spmvT++;
     c.bytes += spmv_bytes(n, m, d.B.nnz, 8, 8, 8);
     tm.sync();
   }
   KR_DEV double normA(const double *x, double *y) { // ||A x||, y = A x
     double s2 = 0.0;
-    csr_mv(tm, d.F, d.F.v64, x, [&](int64_t i, double s) {
+    csr_mv<double>(tm, d.F, x, [&](int64_t i, double s) {
       y[i] = s;
       s2 += s * s;
     });
@@ -160,7 +160,7 @@ template <class Team> struct LobpcgSolver {
     for (int it = 0; it < d.o.precond_steps && tm.ok(); it++) {
       mulA(q, d.pc_tm);
       double acc[2] = {0.0, 0.0}; // q.Nq, q.q
-      csr_mv(tm, d.B, d.B.v64, d.pc_tm, [&](int64_t i, double s) {
+      csr_mv<double>(tm, d.B, d.pc_tm, [&](int64_t i, double s) {
         Nq[i] = s;
         const double qi = q[i];
         acc[0] += qi * s;

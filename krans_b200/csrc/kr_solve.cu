@@ -16,16 +16,6 @@ static inline int64_t round_up(int64_t x, int64_t a) { return kr_round_up(x, a);
 // Lay out (or, with base == nullptr, size) the workspace of one run.
 static size_t cyclic_layout(const CyclicPlan &p, char *base, CyclicDesc *d) { return cyclic_carve(p, base, d); }
 
-static CsrView view_of(const krans_mat *A, bool trans) {
-  CsrView v;
-  if (!trans) {
-    v = CsrView{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, tuned_lanes(A->ctx, A->m, A->nnz), A->ulen};
-  } else {
-    v = CsrView{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, tuned_lanes(A->ctx, A->n, A->nnz), A->ulenT};
-  }
-  return v;
-}
-
 // Reference k_target / early-exit rules (CyclicLanczosSolver.cpp:297-311).
 // Returns 1 when the run has nothing to do.
 static int cyclic_targets(const krans_cyclic_opts &o, int64_t m, int64_t n, int64_t *k_target,
@@ -65,7 +55,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
                       const krans_cyclic_opts &o, const double *init_right, int64_t k_target,
                       int64_t ncv, std::vector<krans_vec *> &found, RunOut *out,
                       const double *prefill = nullptr, int64_t nprefill = 0, double frob_init = 0.0) {
-  const CsrView F = view_of(A, trans), B = view_of(A, !trans);
+  const CsrView F = csr_view(A, trans), B = csr_view(A, !trans);
   const bool mixed = o.precision == KRANS_PREC_MIXED;
   if (mixed && !A->v32) {
     set_error("mixed precision needs a matrix created with KRANS_CSR_FP32");

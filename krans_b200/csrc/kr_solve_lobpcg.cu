@@ -187,8 +187,8 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
 
   LobpcgDesc d;
   memset(&d, 0, sizeof d);
-  d.F = CsrView{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, tuned_lanes(A->ctx, A->m, A->nnz), A->ulen};
-  d.B = CsrView{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, tuned_lanes(A->ctx, A->n, A->nnz), A->ulenT};
+  d.F = csr_view(A, false);
+  d.B = csr_view(A, true);
   d.o = o;
   d.k_target = k_target;
   d.bs = bs;
@@ -410,8 +410,8 @@ int lobpcg_async_plan(krans_ctx *ctx, const krans_request &r, LobpcgAsync **out,
   a->ncta = cluster ? std::min(4, std::max(2, ctx->tune.cluster_size)) : 1;
   LobpcgDesc &d = a->d;
   memset(&d, 0, sizeof d);
-  d.F = CsrView{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, tuned_lanes(ctx, A->m, A->nnz), A->ulen};
-  d.B = CsrView{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, tuned_lanes(ctx, A->n, A->nnz), A->ulenT};
+  d.F = csr_view(A, false);
+  d.B = csr_view(A, true);
   d.o = o;
   d.o.team = cluster ? KRANS_TEAM_GRID : KRANS_TEAM_CTA; // informational only
   d.k_target = k_target;

@@ -245,9 +245,9 @@ __global__ void __launch_bounds__(kSpmvThreads) spmv_lanes_kernel(int64_t rows, 
                                                                   const VT *val, const double *x, double *y,
                                                                   int lanes) {
   TeamFlatSpmv tm;
-  team_spmv_x(
-      tm, rows, rp, ci, val, [&](int32_t c) { return (VT)x[c]; }, lanes, 0,
-      [&](int64_t i, typename AccOf<VT>::T s) { y[i] = (double)s; });
+  team_spmv_lanes(
+      tm, rows, rp, ci, val, [&](int32_t c) { return (VT)x[c]; }, lanes, NoPrologue(),
+      [&](int64_t i, typename AccOf<VT>::T s, char) { y[i] = (double)s; });
 }
 
 // Rows per block of the row-tile kernel: about 80% of a tile of entries at

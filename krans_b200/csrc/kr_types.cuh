@@ -36,6 +36,23 @@ struct RngState {
   int32_t pad;
 };
 
+// The entries of a CSR operand with short rows, as the solvers' SpMV reads
+// them (team_spmv_sliced). Rows are sorted by length, longest first, inside
+// windows of kSliceWindow rows, and taken 32 at a time: slot p of the sorted
+// order is row row[p] (-1 past the last row), slice s holds slots 32 s .. 32 s
+// + 31, and round r (off[s] <= r < off[s + 1]) holds one entry of each of its
+// rows at 32 r + lane (column 0, value 0 where the row has ended).
+struct SlicedView {
+  int32_t slices; // 0: this operand has none
+  const int32_t *off, *row, *ci;
+  const double *v64;
+  const float *v32;
+};
+constexpr int kSliceWindow = 256;
+// Longest row that one lane sums alone: a longer one would hold up its warp
+// while the other lanes idle, and several lanes share a row.
+constexpr int kSliceMaxLen = 64;
+
 struct CsrView {
   int64_t rows, cols, nnz;
   const int32_t *rp, *ci;
@@ -43,6 +60,7 @@ struct CsrView {
   const float *v32;
   int lanes;    // threads per row in the SpMV
   int32_t ulen; // every row has exactly ulen entries (rp[i] = i*ulen), 0 if not
+  SlicedView sl;
 };
 
 struct CyclicDevResult {
@@ -69,9 +87,11 @@ struct CyclicDesc {
   double *y0, *v, *vp, *best_v, *tn; // n-vectors
   double *Vc;                        // KR_NBP candidate n-vectors (block polish)
   double *Hb, *Wb, *Rk, *Pk, *Ak, *Tk; // interleaved CG blocks: m x KR_NBP (Tk: n x KR_NBP)
-  double *tmv, *wm, *Ap;             // m-vectors
-  double2 *rp;                       // CG residual and direction, interleaved (m)
+  double *tmv, *wm;                  // m-vectors
+  double *cgr;                       // CG: the residual (preconditioned CG: z = M^-1 r) that F^T gathers (m)
+  double *cgts, *cgus;               // CG: F^T p and F^T w by slot of F^T's sorted order (n)
   double *r_pre, *dinv, *sd_q, *sd_Oq; // preconditioned CG: residual, Jacobi weights, SD vectors (m)
+  double *cgt;                         // preconditioned CG: F^T p (n; the SD steps work in tn)
   double *alpha, *beta;              // ncv + 2
   double *Tb, *Vt, *sv;              // tiny problem
   int32_t *ord;
@@ -98,10 +118,10 @@ struct CyclicPlan {
 
 __host__ __device__ inline int64_t kr_round_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
-// Shared-memory bytes that hold the CG vectors of a one-block solve (residual
-// and direction interleaved, F F^T p, F^T p): 16 ldm + 8 ldm + 8 ldn.
+// Shared-memory bytes that hold the gathered CG vectors of a one-block solve
+// (residual r, F^T p): 8 ldm + 8 ldn.
 __host__ __device__ inline size_t cta_cg_smem_bytes(int64_t ldm, int64_t ldn) {
-  return (size_t)(24 * ldm + 8 * ldn);
+  return (size_t)(8 * ldm + 8 * ldn);
 }
 
 struct Carver {
@@ -126,8 +146,8 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
   double *y0 = c.take<double>(p.ldn), *v = c.take<double>(p.ldn), *vp = c.take<double>(p.ldn);
   double *best_v = c.take<double>(p.ldn), *tn = c.take<double>(p.ldn);
   double *tmv = c.take<double>(p.ldm), *wm = c.take<double>(p.ldm);
-  double2 *rp = c.take<double2>(p.ldm);
-  double *Ap = c.take<double>(p.ldm);
+  double *cgr = c.take<double>(p.ldm);
+  double *cgts = c.take<double>(p.ldn), *cgus = c.take<double>(p.ldn);
   double *alpha = c.take<double>(p.ncv + 2), *beta = c.take<double>(p.ncv + 2);
   double *Tb = c.take<double>((p.ncv + 1) * p.ncv), *Vt = c.take<double>(p.ncv * p.ncv);
   double *sv = c.take<double>(p.ncv + 1);
@@ -138,12 +158,13 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
   CyclicDevResult *res = c.take<CyclicDevResult>(1);
   GridBarrierState *gb = c.take<GridBarrierState>(1);
   double *gpart = c.take<double>(2 * (p.grid_blocks > 1 ? p.grid_blocks : 1) * KR_RED_K);
-  double *r_pre = nullptr, *dinv = nullptr, *sd_q = nullptr, *sd_Oq = nullptr;
+  double *r_pre = nullptr, *dinv = nullptr, *sd_q = nullptr, *sd_Oq = nullptr, *cgt = nullptr;
   if (p.precond) {
     r_pre = c.take<double>(p.ldm);
     dinv = c.take<double>(p.ldm);
     sd_q = c.take<double>(p.ldm);
     sd_Oq = c.take<double>(p.ldm);
+    cgt = c.take<double>(p.ldn);
   }
   double *Vc = nullptr, *Hb = nullptr, *Wb = nullptr, *Rk = nullptr, *Pk = nullptr, *Ak = nullptr, *Tk = nullptr;
   if (p.block_polish) {
@@ -159,13 +180,13 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
     d->Y = Y; d->X = X; d->wx = wx; d->wy = wy;
     if (p.own_basis) d->basis = basis;
     d->y0 = y0; d->v = v; d->vp = vp; d->best_v = best_v; d->tn = tn;
-    d->tmv = tmv; d->wm = wm; d->rp = rp; d->Ap = Ap;
+    d->tmv = tmv; d->wm = wm; d->cgr = cgr; d->cgts = cgts; d->cgus = cgus;
     d->alpha = alpha; d->beta = beta; d->Tb = Tb; d->Vt = Vt; d->sv = sv; d->ord = ord;
     d->eig_cs = eig_cs; d->eig_pq = eig_pq; d->eig_ord = eig_ord;
     if (p.own_basis) { d->status = status; d->res = res; }
     d->gb = gb; d->gpart = gpart;
     d->Vc = Vc; d->Hb = Hb; d->Wb = Wb; d->Rk = Rk; d->Pk = Pk; d->Ak = Ak; d->Tk = Tk;
-    d->r_pre = r_pre; d->dinv = dinv; d->sd_q = sd_q; d->sd_Oq = sd_Oq;
+    d->r_pre = r_pre; d->dinv = dinv; d->sd_q = sd_q; d->sd_Oq = sd_Oq; d->cgt = cgt;
     d->ldn = p.ldn; d->ldm = p.ldm; d->ldb = p.ldb; d->cap = p.cap;
   }
   return c.off + 256;
