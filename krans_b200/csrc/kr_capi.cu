@@ -510,7 +510,7 @@ extern "C" int krans_selftest_barrier_timeout(krans_ctx *ctx, double timeout_ms,
     GridBarrierState gb;
     int status;
     int pad;
-    double gpart[2 * 2 * KR_RED_K];
+    double gpart[2 * 2 * KR_MDOT];
   };
   Probe *d = nullptr;
   int rc = dev_alloc(ctx, (void **)&d, sizeof(Probe));

@@ -19,6 +19,7 @@
 
 #define KR_DEV __device__ __forceinline__
 #define KR_MAX_WARPS 32
+#define KR_MAX_CLUSTER 16 // blocks of a cluster team
 #ifndef KR_RED_K
 #define KR_RED_K 8 // values per fused team reduction
 #endif
@@ -44,13 +45,16 @@ KR_DEV uint64_t globaltimer_ns() {
 // (the longest legitimate wait is a serial section on the leader block).
 constexpr uint64_t kBarrierTimeoutNs = 8ull * 1000ull * 1000ull * 1000ull;
 
+#define KR_RED_LD (KR_MAX_WARPS + 2) // row of warp partials: 8 rows of double pairs on distinct banks
+
 // Per-block shared memory used by the team primitives.
 struct TeamShared {
-  double red[2][KR_MAX_WARPS * KR_RED_K]; // double-buffered warp partials
-  double bc[KR_RED_K];                    // broadcast slots (grid reductions)
-  double h[160];                          // Gram-Schmidt coefficients
-  double cpart[2][KR_RED_K];              // cluster reductions: this block's partials
-  int ibuf[64];                           // small integer scratch
+  alignas(16) double red[2][KR_RED_K * KR_RED_LD]; // double-buffered warp partials, one row per value
+  alignas(16) double dots[KR_MDOT * KR_RED_LD];    // warp partials of team_multidot
+  double bc[2][KR_RED_K];                          // broadcast slots (grid reductions)
+  double h[160];                                   // Gram-Schmidt coefficients
+  double cpart[2][KR_MAX_CLUSTER][KR_MDOT];        // cluster reductions: every block's partials
+  int ibuf[64];                                    // small integer scratch
 };
 
 KR_DEV double warp_sum(double v) {
@@ -60,28 +64,71 @@ KR_DEV double warp_sum(double v) {
   return v;
 }
 
+// Warp totals of K values (K = 2, 4 or 8) by recursive halving: at each of the
+// first log2 K steps a lane keeps half of the values and gives the other half
+// away, then the butterfly goes on with one value. K + 5 - log2 K exchanges
+// instead of 5 K, and the same additions in the same tree as K butterflies (a
+// lane adds its partner's partial of the same value at offsets 16, 8, 4, 2, 1),
+// so the totals are the same to the last bit. Lane l returns the total of
+// value l / (32 / K).
+template <int K> KR_DEV double warp_sums(double (&v)[K]) {
+  static_assert(K == 2 || K == 4 || K == 8, "power of two");
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int half = K / 2; half > 0; half /= 2, o /= 2) {
+    const bool hi = lane & o;
+#pragma unroll
+    for (int k = 0; k < half; k++) {
+      const double keep = hi ? v[k + half] : v[k], give = hi ? v[k] : v[k + half];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  double t = v[0];
+  for (; o > 0; o /= 2)
+    t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
+// sum of a row of warp partials in warp order
+KR_DEV double sum_warps(const double *r, int nw) {
+  double s = 0.0;
+  int w = 0;
+#pragma unroll 8
+  for (; w + 1 < nw; w += 2) {
+    const double2 p = *reinterpret_cast<const double2 *>(r + w);
+    s += p.x;
+    s += p.y;
+  }
+  if (w < nw)
+    s += r[w];
+  return s;
+}
+
 // Block-level sum of K values; every thread receives the totals. Fixed order:
-// butterfly inside each warp, then warps summed in index order.
+// butterfly inside each warp, then warps summed in index order. One lane per
+// value sums the warps (all threads summing all values cost 2048 shared-memory
+// reads per block for K = 8, more than the rest of the reduction).
 template <int K>
 KR_DEV void block_sum(TeamShared *sh, int &buf, double (&v)[K]) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int k = 0; k < K; k++)
-    v[k] = warp_sum(v[k]);
   double *r = sh->red[buf];
-  if (lane == 0) {
+  if constexpr (K == 1) {
+    const double t = warp_sum(v[0]);
+    if (lane == 0)
+      r[wid] = t;
+    __syncthreads();
+    v[0] = sum_warps(r, nw);
+  } else {
+    const double t = warp_sums<K>(v);
+    if ((lane & (32 / K - 1)) == 0)
+      r[(lane / (32 / K)) * KR_RED_LD + wid] = t;
+    __syncthreads();
+    const double s = lane < K ? sum_warps(r + lane * KR_RED_LD, nw) : 0.0;
 #pragma unroll
     for (int k = 0; k < K; k++)
-      r[wid * KR_RED_K + k] = v[k];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    double s = 0.0;
-    for (int w = 0; w < nw; w++)
-      s += r[w * KR_RED_K + k];
-    v[k] = s;
+      v[k] = __shfl_sync(0xffffffffu, s, k);
   }
   buf ^= 1;
 }
@@ -109,6 +156,11 @@ struct TeamCta {
     sum<1>(v);
     return v[0];
   }
+  // h[q] = team total of this block's total s of value q (thread q < cnt); cnt <= KR_MDOT
+  KR_DEV void dots(int cnt, double s, double *h) {
+    if (threadIdx.x < (unsigned)cnt)
+      h[threadIdx.x] = s;
+  }
   // make values written by the leader block visible to the team
   KR_DEV void publish() { __syncthreads(); }
 };
@@ -117,7 +169,7 @@ struct TeamGrid {
   TeamShared *sh;
   int *err;
   GridBarrierState *gb;
-  double *gpart; // [2][gridDim.x][KR_RED_K]
+  double *gpart; // [2][gridDim.x][KR_MDOT]
   int buf;
   int gbuf;
   KR_DEV int64_t tid() const { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
@@ -147,9 +199,14 @@ struct TeamGrid {
           __threadfence();
           atomicAdd(&gb->gen, 1u);
         } else {
+          // poll the generation alone; the error word and the clock are looked
+          // at once in 64 polls (each costs a poll's time, and the wait is one
+          // poll when the blocks arrive together)
           const uint64_t t0 = globaltimer_ns();
           const uint64_t limit = gb->timeout_ns ? gb->timeout_ns : kBarrierTimeoutNs;
-          while (*vgen == g) {
+          for (unsigned polls = 1; *vgen == g; polls++) {
+            if (polls & 63)
+              continue;
             if (*verr != 0)
               break;
             if (globaltimer_ns() - t0 > limit) {
@@ -157,7 +214,6 @@ struct TeamGrid {
               atomicCAS(err, 0, KRANS_ERR_TIMEOUT);
               break;
             }
-            __nanosleep(40);
           }
         }
         __threadfence();
@@ -166,33 +222,46 @@ struct TeamGrid {
     __syncthreads();
   }
 
+  // sum over the blocks of partial `p` (stride KR_MDOT) by one warp, the same
+  // fixed order in every block
+  KR_DEV double sum_blocks(const double *p) const {
+    double s = 0.0;
+    for (unsigned b = threadIdx.x & 31; b < gridDim.x; b += 32)
+      s += __ldcg(p + (size_t)b * KR_MDOT);
+    return warp_sum(s);
+  }
   template <int K> KR_DEV void sum(double (&v)[K]) {
     block_sum<K>(sh, buf, v);
-    double *gp = gpart + (size_t)gbuf * gridDim.x * KR_RED_K;
+    double *gp = gpart + (size_t)gbuf * gridDim.x * KR_MDOT;
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int k = 0; k < K; k++)
-        gp[(size_t)blockIdx.x * KR_RED_K + k] = v[k];
+        gp[(size_t)blockIdx.x * KR_MDOT + k] = v[k];
     }
     sync();
-    // warp 0 of every block sums the block partials in the same fixed order
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        double s = 0.0;
-        for (unsigned b = lane; b < gridDim.x; b += 32)
-          s += __ldcg(gp + (size_t)b * KR_RED_K + k);
-        s = warp_sum(s);
-        if (lane == 0)
-          sh->bc[k] = s;
-      }
+    const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int k = wid; k < K; k += nw) {
+      const double s = sum_blocks(gp + k);
+      if ((threadIdx.x & 31) == 0)
+        sh->bc[gbuf][k] = s;
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; k++)
-      v[k] = sh->bc[k];
-    __syncthreads();
+      v[k] = sh->bc[gbuf][k];
+    gbuf ^= 1; // the next reduction writes the other slots, and the one after it is behind its barriers
+  }
+  KR_DEV void dots(int cnt, double s, double *h) {
+    double *gp = gpart + (size_t)gbuf * gridDim.x * KR_MDOT;
+    if (threadIdx.x < (unsigned)cnt)
+      gp[(size_t)blockIdx.x * KR_MDOT + threadIdx.x] = s;
+    sync();
+    const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int q = wid; q < cnt; q += nw) {
+      const double t = sum_blocks(gp + q);
+      if ((threadIdx.x & 31) == 0)
+        h[q] = t;
+    }
     gbuf ^= 1;
   }
   KR_DEV double sum1(double x) {
@@ -205,8 +274,9 @@ struct TeamGrid {
 
 // A thread-block cluster (up to 16 blocks on distinct SMs of one GPC) as a
 // team: hardware cluster barrier, reductions through distributed shared
-// memory (each block publishes its partial in its own shared memory, every
-// block sums the partials of ranks 0..size-1 in order).
+// memory (each block writes its partials into every block's shared memory
+// before the barrier, so that after it they are summed from local memory, in
+// the order of the ranks).
 struct TeamCluster {
   TeamShared *sh;
   int *err;
@@ -223,33 +293,45 @@ struct TeamCluster {
   KR_DEV int ncta() const { return (int)csize; }
   KR_DEV bool ok() const { return *(volatile int *)err == 0; }
   KR_DEV void sync() { cooperative_groups::this_cluster().sync(); }
+  // The partials of one reduction go to buffer cbuf of every block; the next
+  // reduction writes the other buffer, and the one after it is behind that
+  // reduction's cluster barrier, which no block passes before it has read.
   template <int K> KR_DEV void sum(double (&v)[K]) {
     block_sum<K>(sh, buf, v);
-    if (threadIdx.x == 0) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (threadIdx.x < csize) {
+      double *peer = cl.map_shared_rank(&sh->cpart[cbuf][rank][0], threadIdx.x);
 #pragma unroll
       for (int k = 0; k < K; k++)
-        sh->cpart[cbuf][k] = v[k];
+        peer[k] = v[k];
     }
-    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     cl.sync();
-    // every thread sums the ranks' partials in rank order straight from their
-    // shared memory (the same order as a sequential sum from rank 0). The
-    // next reduction writes the other buffer, and the one after it is behind
-    // that reduction's cluster barrier, which no block passes before all
-    // blocks have read this one.
     double t[K];
 #pragma unroll
     for (int k = 0; k < K; k++)
       t[k] = 0.0;
     for (unsigned r = 0; r < csize; r++) {
-      const double *peer = cl.map_shared_rank(&sh->cpart[cbuf][0], r);
 #pragma unroll
       for (int k = 0; k < K; k++)
-        t[k] += peer[k];
+        t[k] += sh->cpart[cbuf][r][k];
     }
 #pragma unroll
     for (int k = 0; k < K; k++)
       v[k] = t[k];
+    cbuf ^= 1;
+  }
+  KR_DEV void dots(int cnt, double s, double *h) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (threadIdx.x < (unsigned)cnt)
+      for (unsigned r = 0; r < csize; r++)
+        *cl.map_shared_rank(&sh->cpart[cbuf][rank][threadIdx.x], r) = s;
+    cl.sync();
+    if (threadIdx.x < (unsigned)cnt) {
+      double t = 0.0;
+      for (unsigned r = 0; r < csize; r++)
+        t += sh->cpart[cbuf][r][threadIdx.x];
+      h[threadIdx.x] = t;
+    }
     cbuf ^= 1;
   }
   KR_DEV double sum1(double x) {
@@ -293,29 +375,42 @@ template <class Team, class TX> KR_DEV double team_nrm2(Team &tm, int64_t len, c
 }
 
 // h[q] = <S_q, w> for q < ns (S columns at stride ld); results in tm.sh->h
-// (all threads of every block see them after the call).
+// (all threads of every block see them after the call). Groups of 8 columns
+// share one sweep over w; up to KR_MDOT columns share one team reduction (one
+// per group, with every thread summing every value, made the Gram-Schmidt passes
+// of small solves wait on reductions: a Golub-Kahan step of a 1000-unknown
+// solve took 34 us, and takes 15).
 template <class Team, class TS, class TW>
 KR_DEV void team_multidot(Team &tm, int64_t len, const TS *S, int64_t ld, int ns, const TW *w) {
   const int64_t nt = tm.nthreads();
-  for (int q0 = 0; q0 < ns; q0 += KR_RED_K) {
-    double acc[KR_RED_K];
-#pragma unroll
-    for (int k = 0; k < KR_RED_K; k++)
-      acc[k] = 0.0;
-    const int qn = min(KR_RED_K, ns - q0);
-#pragma unroll 4
-    for (int64_t i = tm.tid(); i < len; i += nt) {
-      const double wi = to_d(w[i]);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  double *part = tm.sh->dots;
+  for (int c0 = 0; c0 < ns; c0 += KR_MDOT) {
+    const int cnt = min(KR_MDOT, ns - c0);
+    for (int g = 0; g < cnt; g += KR_RED_K) {
+      double acc[KR_RED_K];
 #pragma unroll
       for (int k = 0; k < KR_RED_K; k++)
-        if (k < qn)
-          acc[k] += to_d(S[(int64_t)(q0 + k) * ld + i]) * wi;
+        acc[k] = 0.0;
+      const int qn = min(KR_RED_K, cnt - g);
+      const TS *Sg = S + (int64_t)(c0 + g) * ld;
+#pragma unroll 4
+      for (int64_t i = tm.tid(); i < len; i += nt) {
+        const double wi = to_d(w[i]);
+#pragma unroll
+        for (int k = 0; k < KR_RED_K; k++)
+          if (k < qn)
+            acc[k] += to_d(Sg[(int64_t)k * ld + i]) * wi;
+      }
+      const double t = warp_sums<KR_RED_K>(acc);
+      if ((lane & 3) == 0)
+        part[(g + (lane >> 2)) * KR_RED_LD + wid] = t;
     }
-    tm.template sum<KR_RED_K>(acc);
-    if (threadIdx.x < (unsigned)qn)
-      tm.sh->h[q0 + threadIdx.x] = acc[threadIdx.x];
+    __syncthreads();
+    const double s = threadIdx.x < (unsigned)cnt ? sum_warps(part + threadIdx.x * KR_RED_LD, nw) : 0.0;
+    tm.dots(cnt, s, tm.sh->h + c0);
+    __syncthreads();
   }
-  __syncthreads();
 }
 
 // w -= sum_q S_q * coef[q]  (coef in shared memory). The subtractions run in

@@ -49,7 +49,7 @@ static int coop_scratch(krans_ctx *ctx, int blocks, size_t part_doubles, char **
                         GridBarrierState **gb, double **gpart, int **status, double **part) {
   Carver c;
   c.take<GridBarrierState>(1);
-  c.take<double>(2 * (size_t)blocks * KR_RED_K);
+  c.take<double>(2 * (size_t)blocks * KR_MDOT);
   c.take<int>(1);
   c.take<double>((int64_t)std::max<size_t>(part_doubles, 1));
   *bytes = c.off + 256;
@@ -59,7 +59,7 @@ static int coop_scratch(krans_ctx *ctx, int blocks, size_t part_doubles, char **
   Carver d;
   d.base = *ws;
   *gb = d.take<GridBarrierState>(1);
-  *gpart = d.take<double>(2 * (size_t)blocks * KR_RED_K);
+  *gpart = d.take<double>(2 * (size_t)blocks * KR_MDOT);
   *status = d.take<int>(1);
   *part = d.take<double>((int64_t)std::max<size_t>(part_doubles, 1));
   return KRANS_OK;

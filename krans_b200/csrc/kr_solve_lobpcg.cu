@@ -87,7 +87,7 @@ static size_t lobpcg_layout(int64_t m, int64_t n, int64_t bs, int64_t k, int64_t
   t.status = c.take<int32_t>(1);
   t.res = c.take<LobpcgDevResult>(1);
   t.gb = c.take<GridBarrierState>(1);
-  t.gpart = c.take<double>(2 * std::max(ncta, 1) * KR_RED_K);
+  t.gpart = c.take<double>(2 * std::max(ncta, 1) * KR_MDOT);
   t.flag = c.take<int32_t>(4);
   t.dflag = c.take<double>(4);
   if (d) {

@@ -12,6 +12,7 @@
 #ifndef KR_RED_K
 #define KR_RED_K 8 // values per fused team reduction
 #endif
+#define KR_MDOT 32 // columns per reduction of team_multidot (stride of a block's reduction partials)
 #define KR_NBP 8 // right-hand sides of the block CG polish (one fused reduction)
 
 namespace kr {
@@ -157,7 +158,7 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
   int32_t *status = c.take<int32_t>(1);
   CyclicDevResult *res = c.take<CyclicDevResult>(1);
   GridBarrierState *gb = c.take<GridBarrierState>(1);
-  double *gpart = c.take<double>(2 * (p.grid_blocks > 1 ? p.grid_blocks : 1) * KR_RED_K);
+  double *gpart = c.take<double>(2 * (p.grid_blocks > 1 ? p.grid_blocks : 1) * KR_MDOT);
   double *r_pre = nullptr, *dinv = nullptr, *sd_q = nullptr, *sd_Oq = nullptr, *cgt = nullptr;
   if (p.precond) {
     r_pre = c.take<double>(p.ldm);
