@@ -1,13 +1,10 @@
-// Tall-skinny products of the block solver:
-//   team_gemm_tn:       C = A^T B (Cholesky QR of short blocks, projections),
-//                       FP64 tensor cores: shared-memory panels for long, wide
-//                       products (team_gemm_tn_panel), one warp per output
-//                       tile otherwise
-//   team_gram_sym_tiled: S = Z^T Z and G = Z^T (AZ), upper tiles, panels
-//   team_gram2_direct:  S = Z^T Z and G = Z^T (AZ) in one pass (short or
-//                       narrow blocks)
-//   team_gemm_nn:       out (-)= Z * Y[roff:roff+zc, 0:q] (n x q), FP64 tensor
-//                       cores, shared-memory tiles (team_combine, team_combine_sub)
+// Tall-skinny products of the block solver, on the FP64 tensor cores:
+//   team_tn_panels:     S = Z^T Z with G = Z^T (AZ), or C = A^T B: shared-memory
+//                       panels, for long, wide blocks
+//   team_gemm_tn_direct, team_gram2_direct: the same for short or narrow
+//                       blocks, one warp per output tile
+//   team_gemm_nn:       out (-)= Z * Y[roff:roff+zc, 0:q] (n x q), shared-memory
+//                       chunks (team_combine, team_combine_sub)
 // Sums run in a fixed order that depends only on the team size, so results
 // are deterministic for a given team size.
 #pragma once
@@ -158,253 +155,198 @@ KR_DEV void team_gram2_direct(Team &tm, int64_t n, const double *Z, const double
 }
 
 
-// S = Z^T Z and, when AZ is given, G = Z^T (AZ) (p x p) in one pass over Z
-// and AZ, on the FP64 tensor cores with shared-memory panels: the tiled form
-// of team_gram2_direct for long, wide blocks. Only the upper 64 x 64 tiles
-// are formed and mirrored, as the reference's form_gram does
-// (LOBPCGSolver.cpp:67-80: S(i,j) = S(j,i) = Z_i.Z_j, G(i,j) = G(j,i) =
-// Z_i.(AZ)_j for i <= j). Work items are (upper tile, fixed chunk of rows);
-// a block stages 32-row panels of the tile's columns of Z (and of AZ) in
-// shared memory, fetching the next panel into registers while the current
-// one is multiplied, and each of its 16 warps accumulates a 16 x 16 piece of
-// S (and of G). Partial tiles are summed in chunk order, so the result
-// depends only on the team size. `part` must hold (2 ncta + tiles) * 8192
-// doubles; needs 512 threads and gram_tiled_smem_bytes() of dynamic shared
-// memory.
-#define KR_GT 64 // tile edge of the panel products
-#define KR_GP 32 // rows per panel of the panel products
-__host__ __device__ constexpr size_t gram_tiled_smem_bytes() { return (size_t)3 * KR_GT * (KR_GP + 1) * 8; }
+#define KR_TN_ROWS 131072 // rows from which the panel form of the A^T B products runs
+#define KR_TN_COLS 32     // and columns
 
-template <class Team>
-KR_DEV void team_gram_sym_tiled(Team &tm, int64_t n, const double *Z, const double *AZ, int64_t ld, int p,
-                                double *S, double *G, double *part) {
+// ---- panel products -----------------------------------------------------------
+// Asynchronous copies into the shared-memory panels: `live` of the W doubles
+// (W = 1 or 2) from global memory, zeros for the rest.
+template <int W> KR_DEV void cp_async_f64(double *dst, const double *src, int live) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  if constexpr (W == 2)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(8 * live) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(8 * live) : "memory");
+}
+KR_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> KR_DEV void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+KR_DEV bool aligned16(const double *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Products of tall blocks over their rows, on the FP64 tensor cores:
+//   SYM:  S = Z^T Z and, when W is given, G = Z^T W (p x p): only the upper 64
+//         x 64 tiles are formed, and mirrored, as the reference's form_gram does
+//         (LOBPCGSolver.cpp:67-80: S(i,j) = S(j,i) = Z_i.Z_j, G(i,j) = G(j,i) =
+//         Z_i.(AZ)_j for i <= j);
+//   else: S = Z^T W (p x q).
+// Work items are (tile, chunk of rows). A block stages 32-row panels of the
+// tile's columns of Z (and W) in shared memory, the next panel on its way by
+// cp.async while one is multiplied; each of its 16 warps accumulates a 16 x 16 piece of S and of G (2 x
+// 2 DMMA 8x8 tiles each) and skips pieces below the diagonal or past the last
+// column. Partial tiles are summed in chunk order, so the result depends only
+// on the team size.
+// Bound by the DMMA pipe (36.9 TFLOP/s measured). The panel pitch of 36 doubles
+// puts the 8 x 4 fragment of a DMMA on distinct banks (33 cost four-way
+// conflicts and held the kernel to 11 TFLOP/s executed), and the pieces are
+// dealt to the warps so that the ones past an edge do not all fall to one of
+// the SM's four pipes. The chunk count fills two rounds of the team's blocks,
+// not a little more than two. At n = 4194304, counting 2 n p^2 a product: S and
+// G of p = 288 17.6 -> 35.5 TFLOP/s, of p = 96 9.8 -> 26.1; a 64 x 96
+// projection 11.4 -> 19.0. Narrow blocks on many thread blocks stay with the
+// direct forms: p = 36 at n = 50021 took 0.10 ms there and 0.16 ms in panels.
+// `part` must hold (2 ncta + tiles) * 4096 doubles, twice that with SYM; needs
+// 512 threads and tn_panel_smem_bytes() of dynamic shared memory.
+#define KR_GT 64 // tile edge
+#define KR_GP 32 // rows per panel
+#define KR_GL 36 // panel pitch
+#define KR_GS 2  // panels held: one multiplied, one on its way
+__host__ __device__ constexpr size_t tn_panel_smem_bytes() { return (size_t)KR_GS * 3 * KR_GT * KR_GL * 8; }
+
+template <bool SYM, class Team>
+KR_DEV void team_tn_panels(Team &tm, int64_t n, const double *Z, int p, const double *W, int q, int64_t ld, double *S,
+                           double *G, double *part) {
   extern __shared__ __align__(16) double kr_gemm_smem[];
-  typedef double Panel[KR_GP + 1];
-  Panel *sA = reinterpret_cast<Panel *>(kr_gemm_smem);
-  Panel *sB = sA + KR_GT, *sC = sB + KR_GT;
-  const bool withG = AZ != nullptr;
-  const int tp = (p + KR_GT - 1) / KR_GT, tu = tp * (tp + 1) / 2;
+  constexpr int PANEL = KR_GT * KR_GL, STAGE = 3 * PANEL;
+  constexpr int ITEM = (SYM ? 2 : 1) * KR_GT * KR_GT;
+  const bool two = SYM && W != nullptr; // S and G
+  const int tp = (p + KR_GT - 1) / KR_GT, tq = (q + KR_GT - 1) / KR_GT;
+  const int tiles = SYM ? tp * (tp + 1) / 2 : tp * tq;
   const int ncta = tm.ncta();
   const int64_t kblocks = (n + KR_GP - 1) / KR_GP;
-  const int nch = (int)imin64(imin64(ncta, kblocks > 0 ? kblocks : 1), (int64_t)(2 * ncta + tu - 1) / tu);
+  const int nch = (int)imin64(kblocks, 2 * ncta / tiles);
   const int nchunks = nch > 0 ? nch : 1;
   const int64_t kb_per = (kblocks + nchunks - 1) / nchunks; // panels per chunk
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int wr = (wid >> 2) * 16, wc = (wid & 3) * 16; // this warp's 16 x 16 piece
-  const int items = tu * nchunks;
-  constexpr int PER = 3 * KR_GT * KR_GP / 512; // elements per thread and panel (up to three operands)
+  const int wr = (wid >> 2) * 16, wc = ((wid + (wid >> 2)) & 3) * 16; // this warp's 16 x 16 piece
+  const int items = tiles * nchunks;
+  const bool vec = (ld & 1) == 0 && aligned16(Z) && (W == nullptr || aligned16(W));
   for (int it = tm.cta_rank(); it < items; it += ncta) {
-    const int tile = it % tu, ch = it / tu;
-    int tj = 0;
-    while ((tj + 1) * (tj + 2) / 2 <= tile)
-      tj++;
-    const int ti = tile - tj * (tj + 1) / 2; // ti <= tj
-    const bool diag = ti == tj;              // the B panel is the A panel
+    const int tile = it % tiles, ch = it / tiles;
+    int ti, tj;
+    if (SYM) {
+      tj = 0;
+      while ((tj + 1) * (tj + 2) / 2 <= tile)
+        tj++;
+      ti = tile - tj * (tj + 1) / 2; // ti <= tj
+    } else {
+      ti = tile % tp;
+      tj = tile / tp;
+    }
+    const bool diag = SYM && ti == tj; // the B panel is the A panel
     const int64_t kb0 = (int64_t)ch * kb_per, kb1 = imin64(kb0 + kb_per, kblocks);
+    // panel of 64 columns of X from column c0 (cols in all), rows 32 kb ..
+    auto panel = [&](double *dst, const double *X, int c0, int cols, int64_t kb) {
+      const int64_t r0 = kb * KR_GP;
+      if (vec) {
+#pragma unroll
+        for (int e = threadIdx.x; e < KR_GT * KR_GP / 2; e += 512) {
+          const int c = e / (KR_GP / 2), k = 2 * (e % (KR_GP / 2));
+          const int64_t left = n - (r0 + k);
+          const int live = c0 + c < cols && left > 0 ? (left > 1 ? 2 : 1) : 0;
+          cp_async_f64<2>(dst + c * KR_GL + k, live ? X + (int64_t)(c0 + c) * ld + r0 + k : X, live);
+        }
+      } else {
+#pragma unroll
+        for (int e = threadIdx.x; e < KR_GT * KR_GP; e += 512) {
+          const int c = e / KR_GP, k = e % KR_GP;
+          const int live = c0 + c < cols && r0 + k < n;
+          cp_async_f64<1>(dst + c * KR_GL + k, live ? X + (int64_t)(c0 + c) * ld + r0 + k : X, live);
+        }
+      }
+    };
+    auto stage = [&](int64_t kb) {
+      if (kb < kb1) {
+        double *st = kr_gemm_smem + (kb - kb0) % KR_GS * STAGE;
+        panel(st, Z, ti * KR_GT, p, kb);
+        if (SYM) {
+          if (!diag)
+            panel(st + PANEL, Z, tj * KR_GT, p, kb);
+          if (two)
+            panel(st + 2 * PANEL, W, tj * KR_GT, p, kb);
+        } else {
+          panel(st + PANEL, W, tj * KR_GT, q, kb);
+        }
+      }
+      cp_async_commit();
+    };
+    // this warp's piece holds an element that is wanted
+    const bool mine = ti * KR_GT + wr < p && tj * KR_GT + wc < (SYM ? p : q) && (!diag || wr <= wc);
     double aS[2][2][2], aG[2][2][2];
 #pragma unroll
     for (int x = 0; x < 2; x++)
 #pragma unroll
       for (int y = 0; y < 2; y++)
         aS[x][y][0] = aS[x][y][1] = aG[x][y][0] = aG[x][y][1] = 0.0;
-    double v[PER];
-    auto fetch = [&](int64_t kb) {
-      const int64_t r0 = kb * KR_GP;
 #pragma unroll
-      for (int q = 0; q < PER; q++) {
-        const int e = threadIdx.x + q * 512;
-        const int which = e / (KR_GT * KR_GP), rem = e % (KR_GT * KR_GP);
-        const int c = rem / KR_GP, k = rem % KR_GP;
-        const int64_t r = r0 + k;
-        double x = 0.0;
-        const bool used = which == 0 || (which == 1 && !diag) || (which == 2 && withG);
-        if (used && kb < kb1 && r < n) {
-          const int colx = (which == 0 ? ti : tj) * KR_GT + c;
-          if (colx < p)
-            x = (which == 2 ? AZ : Z)[(int64_t)colx * ld + r];
-        }
-        v[q] = x;
-      }
-    };
-    fetch(kb0);
+    for (int s = 0; s < KR_GS - 1; s++)
+      stage(kb0 + s);
     for (int64_t kb = kb0; kb < kb1; kb++) {
+      cp_async_wait<KR_GS - 2>();
+      __syncthreads(); // panel kb is there, and every warp has read panel kb - 1
+      stage(kb + KR_GS - 1);
+      if (mine) {
+        const double *st = kr_gemm_smem + (kb - kb0) % KR_GS * STAGE;
+        const double *fA = st + (wr + (lane >> 2)) * KR_GL + (lane & 3);
+        const double *fB = st + (diag ? 0 : PANEL) + (wc + (lane >> 2)) * KR_GL + (lane & 3);
+        const double *fC = st + 2 * PANEL + (wc + (lane >> 2)) * KR_GL + (lane & 3);
 #pragma unroll
-      for (int q = 0; q < PER; q++) {
-        const int e = threadIdx.x + q * 512;
-        const int which = e / (KR_GT * KR_GP), rem = e % (KR_GT * KR_GP);
-        (which == 0 ? sA : which == 1 ? sB : sC)[rem / KR_GP][rem % KR_GP] = v[q];
-      }
-      __syncthreads();
-      if (kb + 1 < kb1)
-        fetch(kb + 1);
-      const Panel *pB = diag ? sA : sB;
-#pragma unroll
-      for (int kk = 0; kk < KR_GP; kk += 4) {
-        double fa[2], fb[2];
-#pragma unroll
-        for (int x = 0; x < 2; x++)
-          fa[x] = sA[wr + 8 * x + (lane >> 2)][kk + (lane & 3)];
-#pragma unroll
-        for (int y = 0; y < 2; y++)
-          fb[y] = pB[wc + 8 * y + (lane >> 2)][kk + (lane & 3)];
-#pragma unroll
-        for (int x = 0; x < 2; x++)
-#pragma unroll
-          for (int y = 0; y < 2; y++)
-            dmma_8x8x4(aS[x][y][0], aS[x][y][1], fa[x], fb[y]);
-        if (withG) {
-          double fc[2];
-#pragma unroll
-          for (int y = 0; y < 2; y++)
-            fc[y] = sC[wc + 8 * y + (lane >> 2)][kk + (lane & 3)];
-#pragma unroll
-          for (int x = 0; x < 2; x++)
-#pragma unroll
-            for (int y = 0; y < 2; y++)
-              dmma_8x8x4(aG[x][y][0], aG[x][y][1], fa[x], fc[y]);
+        for (int kk = 0; kk < KR_GP; kk += 4) {
+          const double a0 = fA[kk], a1 = fA[kk + 8 * KR_GL];
+          const double b0 = fB[kk], b1 = fB[kk + 8 * KR_GL];
+          dmma_8x8x4(aS[0][0][0], aS[0][0][1], a0, b0);
+          dmma_8x8x4(aS[0][1][0], aS[0][1][1], a0, b1);
+          dmma_8x8x4(aS[1][0][0], aS[1][0][1], a1, b0);
+          dmma_8x8x4(aS[1][1][0], aS[1][1][1], a1, b1);
+          if (two) {
+            const double c0 = fC[kk], c1 = fC[kk + 8 * KR_GL];
+            dmma_8x8x4(aG[0][0][0], aG[0][0][1], a0, c0);
+            dmma_8x8x4(aG[0][1][0], aG[0][1][1], a0, c1);
+            dmma_8x8x4(aG[1][0][0], aG[1][0][1], a1, c0);
+            dmma_8x8x4(aG[1][1][0], aG[1][1][1], a1, c1);
+          }
         }
       }
-      __syncthreads();
     }
-    double *pt = part + (size_t)it * (2 * KR_GT * KR_GT);
+    cp_async_wait<0>();
+    __syncthreads(); // the next item's panels may be staged
+    if (mine) {
+      double *pt = part + (size_t)it * ITEM;
 #pragma unroll
-    for (int x = 0; x < 2; x++)
+      for (int x = 0; x < 2; x++)
 #pragma unroll
-      for (int y = 0; y < 2; y++) {
-        const int i = wr + 8 * x + (lane >> 2), j = wc + 8 * y + 2 * (lane & 3);
-        pt[i + j * KR_GT] = aS[x][y][0];
-        pt[i + (j + 1) * KR_GT] = aS[x][y][1];
-        pt[KR_GT * KR_GT + i + j * KR_GT] = aG[x][y][0];
-        pt[KR_GT * KR_GT + i + (j + 1) * KR_GT] = aG[x][y][1];
-      }
+        for (int y = 0; y < 2; y++) {
+          const int i = wr + 8 * x + (lane >> 2), j = wc + 8 * y + 2 * (lane & 3);
+          pt[i + j * KR_GT] = aS[x][y][0];
+          pt[i + (j + 1) * KR_GT] = aS[x][y][1];
+          if (two) {
+            pt[KR_GT * KR_GT + i + j * KR_GT] = aG[x][y][0];
+            pt[KR_GT * KR_GT + i + (j + 1) * KR_GT] = aG[x][y][1];
+          }
+        }
+    }
   }
   tm.sync();
   const int64_t nthr = tm.nthreads();
-  for (int64_t e = tm.tid(); e < (int64_t)p * p; e += nthr) {
+  for (int64_t e = tm.tid(); e < (int64_t)p * q; e += nthr) {
     const int i = (int)(e % p), j = (int)(e / p);
-    if (i > j)
+    if (SYM && i > j)
       continue;
     const int ti = i / KR_GT, tj = j / KR_GT, li = i % KR_GT, lj = j % KR_GT;
-    const int tile = tj * (tj + 1) / 2 + ti;
+    const int tile = SYM ? tj * (tj + 1) / 2 + ti : tj * tp + ti;
     double sv = 0.0, gv = 0.0;
     for (int ch = 0; ch < nchunks; ch++) {
-      const double *pt = part + (size_t)(tile + ch * tu) * (2 * KR_GT * KR_GT);
+      const double *pt = part + (size_t)(tile + ch * tiles) * ITEM;
       sv += __ldcg(pt + li + lj * KR_GT);
-      if (withG)
+      if (two)
         gv += __ldcg(pt + KR_GT * KR_GT + li + lj * KR_GT);
     }
     S[i + (size_t)j * p] = sv;
-    S[j + (size_t)i * p] = sv;
-    if (withG) {
-      G[i + (size_t)j * p] = gv;
-      G[j + (size_t)i * p] = gv;
+    if (SYM) {
+      S[j + (size_t)i * p] = sv;
+      if (two) {
+        G[i + (size_t)j * p] = gv;
+        G[j + (size_t)i * p] = gv;
+      }
     }
-  }
-  tm.sync();
-}
-
-// C = A^T B (a x b, leading dim a) for long, wide products: the general form
-// of team_gram_sym_tiled. Work items are (64 x 64 tile of C, fixed chunk of
-// rows); a block stages 32-row panels of the tile's columns of A and of B in
-// shared memory, fetching the next panel into registers while the current
-// one is multiplied, and each of its 16 warps accumulates a 16 x 16 piece of
-// the tile (2 x 2 DMMA 8x8 tiles). Partial tiles are summed in chunk order,
-// so the result depends only on the team size. `part` must hold
-// (2 ncta + tiles) * 4096 doubles, tiles = ceil(a/64) * ceil(b/64); needs 512
-// threads and gram_tiled_smem_bytes() of dynamic shared memory.
-template <class Team>
-KR_DEV void team_gemm_tn_panel(Team &tm, int64_t n, const double *A, int a, const double *B, int b, int64_t ld,
-                               double *C, double *part) {
-  extern __shared__ __align__(16) double kr_gemm_smem[];
-  typedef double Panel[KR_GP + 1];
-  Panel *sA = reinterpret_cast<Panel *>(kr_gemm_smem);
-  Panel *sB = sA + KR_GT;
-  const int ta = (a + KR_GT - 1) / KR_GT, tb = (b + KR_GT - 1) / KR_GT, tiles = ta * tb;
-  const int ncta = tm.ncta();
-  const int64_t kblocks = (n + KR_GP - 1) / KR_GP;
-  const int nch = (int)imin64(imin64(ncta, kblocks > 0 ? kblocks : 1), (int64_t)(2 * ncta + tiles - 1) / tiles);
-  const int nchunks = nch > 0 ? nch : 1;
-  const int64_t kb_per = (kblocks + nchunks - 1) / nchunks;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int wr = (wid >> 2) * 16, wc = (wid & 3) * 16;
-  const int items = tiles * nchunks;
-  constexpr int PER = 2 * KR_GT * KR_GP / 512; // elements per thread and panel (two operands)
-  for (int it = tm.cta_rank(); it < items; it += ncta) {
-    const int tile = it % tiles, ch = it / tiles;
-    const int ti = tile % ta, tj = tile / ta;
-    const int64_t kb0 = (int64_t)ch * kb_per, kb1 = imin64(kb0 + kb_per, kblocks);
-    double acc[2][2][2];
-#pragma unroll
-    for (int x = 0; x < 2; x++)
-#pragma unroll
-      for (int y = 0; y < 2; y++)
-        acc[x][y][0] = acc[x][y][1] = 0.0;
-    double v[PER];
-    auto fetch = [&](int64_t kb) {
-      const int64_t r0 = kb * KR_GP;
-#pragma unroll
-      for (int q = 0; q < PER; q++) {
-        const int e = threadIdx.x + q * 512;
-        const int which = e / (KR_GT * KR_GP), rem = e % (KR_GT * KR_GP);
-        const int c = rem / KR_GP, k = rem % KR_GP;
-        const int64_t r = r0 + k;
-        double x = 0.0;
-        if (kb < kb1 && r < n) {
-          const int colx = (which == 0 ? ti : tj) * KR_GT + c;
-          if (colx < (which == 0 ? a : b))
-            x = (which == 0 ? A : B)[(int64_t)colx * ld + r];
-        }
-        v[q] = x;
-      }
-    };
-    fetch(kb0);
-    for (int64_t kb = kb0; kb < kb1; kb++) {
-#pragma unroll
-      for (int q = 0; q < PER; q++) {
-        const int e = threadIdx.x + q * 512;
-        const int which = e / (KR_GT * KR_GP), rem = e % (KR_GT * KR_GP);
-        (which == 0 ? sA : sB)[rem / KR_GP][rem % KR_GP] = v[q];
-      }
-      __syncthreads();
-      if (kb + 1 < kb1)
-        fetch(kb + 1);
-#pragma unroll
-      for (int kk = 0; kk < KR_GP; kk += 4) {
-        double fa[2], fb[2];
-#pragma unroll
-        for (int x = 0; x < 2; x++)
-          fa[x] = sA[wr + 8 * x + (lane >> 2)][kk + (lane & 3)];
-#pragma unroll
-        for (int y = 0; y < 2; y++)
-          fb[y] = sB[wc + 8 * y + (lane >> 2)][kk + (lane & 3)];
-#pragma unroll
-        for (int x = 0; x < 2; x++)
-#pragma unroll
-          for (int y = 0; y < 2; y++)
-            dmma_8x8x4(acc[x][y][0], acc[x][y][1], fa[x], fb[y]);
-      }
-      __syncthreads();
-    }
-    double *pt = part + (size_t)it * (KR_GT * KR_GT);
-#pragma unroll
-    for (int x = 0; x < 2; x++)
-#pragma unroll
-      for (int y = 0; y < 2; y++) {
-        const int i = wr + 8 * x + (lane >> 2), j = wc + 8 * y + 2 * (lane & 3);
-        pt[i + j * KR_GT] = acc[x][y][0];
-        pt[i + (j + 1) * KR_GT] = acc[x][y][1];
-      }
-  }
-  tm.sync();
-  const int64_t nthr = tm.nthreads();
-  for (int64_t e = tm.tid(); e < (int64_t)a * b; e += nthr) {
-    const int i = (int)(e % a), j = (int)(e / a);
-    const int ti = i / KR_GT, tj = j / KR_GT, li = i % KR_GT, lj = j % KR_GT;
-    const int tile = tj * ta + ti;
-    double sv = 0.0;
-    for (int ch = 0; ch < nchunks; ch++)
-      sv += __ldcg(part + (size_t)(tile + ch * tiles) * (KR_GT * KR_GT) + li + lj * KR_GT);
-    C[i + (size_t)j * a] = sv;
   }
   tm.sync();
 }
@@ -418,8 +360,8 @@ KR_DEV void team_gemm_tn_panel(Team &tm, int64_t n, const double *A, int a, cons
 template <class Team>
 KR_DEV void team_gemm_tn(Team &tm, int64_t n, const double *A, int a, const double *B, int b, int64_t ld,
                          double *C, double *part) {
-  if (n >= 131072 && (a >= 32 || b >= 32))
-    team_gemm_tn_panel(tm, n, A, a, B, b, ld, C, part);
+  if (n >= KR_TN_ROWS && (a >= KR_TN_COLS || b >= KR_TN_COLS))
+    team_tn_panels<false>(tm, n, A, a, B, b, ld, C, nullptr, part);
   else
     team_gemm_tn_direct(tm, n, A, a, B, b, ld, C, part);
 }
@@ -430,15 +372,22 @@ KR_DEV void team_gemm_tn(Team &tm, int64_t n, const double *A, int a, const doub
 // leading dim ldy. On the FP64 tensor cores: a block takes 64-row tiles of
 // the tall operand (every 128-column group of the output for one tile before
 // the next tile, so the tile is read from HBM once); k runs in chunks of 16
-// staged in shared memory (the next chunk is fetched into registers while
-// the current one is multiplied); each of the 16 warps owns a 16 x 32 piece
-// of the 64 x 128 output group (2 x 4 DMMA 8x8 tiles). Each output is summed
-// in a fixed order, independent of the team. Needs 512 threads and
-// gemm_nn_smem_bytes() of dynamic shared memory.
+// staged in shared memory, the next on its way by cp.async across the ends of
+// tiles; each of the 16 warps owns a 16 x 32 piece of the 64 x 128 output
+// group (2 x 4 DMMA 8x8 tiles), dealt so that pieces past the last column fall
+// to the SM's four pipes alike. Each output is summed in a fixed order,
+// independent of the team. Bound by the DMMA pipe; both chunk pitches put a
+// fragment on distinct banks (4194304 x 288 times 288 x 96: 15.1 -> 25.8
+// TFLOP/s). Needs 512 threads and gemm_nn_smem_bytes() of dynamic shared memory.
 #define KR_NT 64  // rows per tile
 #define KR_NQ 128 // output columns per group
 #define KR_NK 16  // k per chunk
-__host__ __device__ constexpr size_t gemm_nn_smem_bytes() { return (size_t)(KR_NT + KR_NQ) * (KR_NK + 1) * 8; }
+#define KR_NZL (KR_NT + 4) // pitch of a k row of the Z chunk
+#define KR_NYL (KR_NK + 4) // pitch of a column of the Y chunk
+#define KR_NS 2            // chunks held: one multiplied, one on its way
+__host__ __device__ constexpr size_t gemm_nn_smem_bytes() {
+  return (size_t)KR_NS * (KR_NK * KR_NZL + KR_NQ * KR_NYL) * 8;
+}
 
 // Narrow form (q <= KR_NQ_DIRECT outputs): every thread takes whole rows and
 // sums over k in order on the CUDA cores, with no shared memory and no
@@ -479,89 +428,132 @@ KR_DEV void team_gemm_nn(Team &tm, int64_t n, const double *Z, int64_t ld, int z
     return;
   }
   extern __shared__ __align__(16) double kr_gemm_smem[];
-  double(*sZ)[KR_NK + 1] = reinterpret_cast<double(*)[KR_NK + 1]>(kr_gemm_smem);
-  double(*sY)[KR_NK + 1] = reinterpret_cast<double(*)[KR_NK + 1]>(kr_gemm_smem + KR_NT * (KR_NK + 1));
+  constexpr int STAGE = KR_NK * KR_NZL + KR_NQ * KR_NYL;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int wr = (wid >> 2) * 16, wc = (wid & 3) * 32; // this warp's 16 x 32 piece
+  const int wr = (wid >> 2) * 16, wc = ((wid + (wid >> 2)) & 3) * 32; // this warp's 16 x 32 piece
   const int64_t row_tiles = (n + KR_NT - 1) / KR_NT;
   const int col_groups = (q + KR_NQ - 1) / KR_NQ;
   const int nchunks = (zc + KR_NK - 1) / KR_NK;
-  constexpr int PZ = KR_NT * KR_NK / 512, PY = KR_NQ * KR_NK / 512;
-  for (int64_t rt = tm.cta_rank(); rt < row_tiles; rt += tm.ncta()) {
-    const int64_t r0 = rt * KR_NT;
-    for (int cg = 0; cg < col_groups; cg++) {
-      const int c0 = cg * KR_NQ;
-      double acc[2][4][2];
+  const bool vz = (ld & 1) == 0 && aligned16(Z);
+  const bool vy = ((ldy | roff) & 1) == 0 && aligned16(Y);
+  const int64_t ncta = tm.ncta(), rt0 = tm.cta_rank();
+  if (rt0 >= row_tiles)
+    return;
+  // steps of this block: (row tile, column group, chunk), chunk fastest
+  struct Step {
+    int64_t rt;
+    int cg, ch;
+  };
+  auto next = [&](Step &s) {
+    if (++s.ch == nchunks) {
+      s.ch = 0;
+      if (++s.cg == col_groups) {
+        s.cg = 0;
+        s.rt += ncta;
+      }
+    }
+  };
+  auto stage = [&](const Step &s, int slot) {
+    if (s.rt < row_tiles) {
+      double *sZ = kr_gemm_smem + slot * STAGE, *sY = sZ + KR_NK * KR_NZL;
+      const int64_t r0 = s.rt * KR_NT;
+      const int c0 = s.cg * KR_NQ, k0 = s.ch * KR_NK;
+      if (vz) {
+        const int kk = threadIdx.x / (KR_NT / 2), r = 2 * (threadIdx.x % (KR_NT / 2)); // 512 pairs
+        const int64_t left = n - (r0 + r);
+        const int live = k0 + kk < zc && left > 0 ? (left > 1 ? 2 : 1) : 0;
+        cp_async_f64<2>(sZ + kk * KR_NZL + r, live ? Z + (int64_t)(k0 + kk) * ld + r0 + r : Z, live);
+      } else {
+#pragma unroll
+        for (int e = threadIdx.x; e < KR_NT * KR_NK; e += 512) {
+          const int kk = e / KR_NT, r = e % KR_NT;
+          const int live = k0 + kk < zc && r0 + r < n;
+          cp_async_f64<1>(sZ + kk * KR_NZL + r, live ? Z + (int64_t)(k0 + kk) * ld + r0 + r : Z, live);
+        }
+      }
+      if (vy) {
+#pragma unroll
+        for (int e = threadIdx.x; e < KR_NQ * KR_NK / 2; e += 512) {
+          const int c = e / (KR_NK / 2), kk = 2 * (e % (KR_NK / 2));
+          const int left = zc - (k0 + kk);
+          const int live = c0 + c < q && left > 0 ? (left > 1 ? 2 : 1) : 0;
+          cp_async_f64<2>(sY + c * KR_NYL + kk, live ? Y + (int64_t)(roff + k0 + kk) + (int64_t)(c0 + c) * ldy : Y,
+                          live);
+        }
+      } else {
+#pragma unroll
+        for (int e = threadIdx.x; e < KR_NQ * KR_NK; e += 512) {
+          const int c = e / KR_NK, kk = e % KR_NK;
+          const int live = c0 + c < q && k0 + kk < zc;
+          cp_async_f64<1>(sY + c * KR_NYL + kk, live ? Y + (int64_t)(roff + k0 + kk) + (int64_t)(c0 + c) * ldy : Y,
+                          live);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  Step ahead{rt0, 0, 0};
+  for (int s = 0; s < KR_NS - 1; s++) {
+    stage(ahead, s);
+    next(ahead);
+  }
+  double acc[2][4][2];
+  int slot = 0;
+  for (Step now{rt0, 0, 0}; now.rt < row_tiles; next(now)) {
+    cp_async_wait<KR_NS - 2>();
+    __syncthreads(); // this chunk is there, and every warp has read the one before
+    stage(ahead, (slot + KR_NS - 1) % KR_NS);
+    next(ahead);
+    if (now.ch == 0) {
 #pragma unroll
       for (int x = 0; x < 2; x++)
 #pragma unroll
         for (int y = 0; y < 4; y++)
           acc[x][y][0] = acc[x][y][1] = 0.0;
-      double vz[PZ], vy[PY];
-      auto fetch = [&](int ch) {
-        const int k0 = ch * KR_NK;
-#pragma unroll
-        for (int p = 0; p < PZ; p++) {
-          const int e = threadIdx.x + p * 512, kk = e / KR_NT, r = e % KR_NT;
-          vz[p] = (r0 + r < n && k0 + kk < zc) ? Z[(int64_t)(k0 + kk) * ld + r0 + r] : 0.0;
-        }
-#pragma unroll
-        for (int p = 0; p < PY; p++) {
-          const int e = threadIdx.x + p * 512, c = e / KR_NK, kk = e % KR_NK;
-          vy[p] = (c0 + c < q && k0 + kk < zc) ? Y[(int64_t)(roff + k0 + kk) + (int64_t)(c0 + c) * ldy] : 0.0;
-        }
-      };
-      fetch(0);
-      for (int ch = 0; ch < nchunks; ch++) {
-#pragma unroll
-        for (int p = 0; p < PZ; p++) {
-          const int e = threadIdx.x + p * 512;
-          sZ[e % KR_NT][e / KR_NT] = vz[p];
-        }
-#pragma unroll
-        for (int p = 0; p < PY; p++) {
-          const int e = threadIdx.x + p * 512;
-          sY[e / KR_NK][e % KR_NK] = vy[p];
-        }
-        __syncthreads();
-        if (ch + 1 < nchunks)
-          fetch(ch + 1);
-        if (c0 + wc < q) { // warp-uniform: warps past the last column have nothing to do
-#pragma unroll
-          for (int kk = 0; kk < KR_NK; kk += 4) {
-            double fa[2], fb[4];
-#pragma unroll
-            for (int x = 0; x < 2; x++)
-              fa[x] = sZ[wr + 8 * x + (lane >> 2)][kk + (lane & 3)];
-#pragma unroll
-            for (int y = 0; y < 4; y++)
-              fb[y] = sY[wc + 8 * y + (lane >> 2)][kk + (lane & 3)];
-#pragma unroll
-            for (int x = 0; x < 2; x++)
-#pragma unroll
-              for (int y = 0; y < 4; y++)
-                dmma_8x8x4(acc[x][y][0], acc[x][y][1], fa[x], fb[y]);
-          }
-        }
-        __syncthreads();
-      }
-#pragma unroll
-      for (int x = 0; x < 2; x++)
-#pragma unroll
-        for (int y = 0; y < 4; y++) {
-          const int64_t i = r0 + wr + 8 * x + (lane >> 2);
-          const int j = c0 + wc + 8 * y + 2 * (lane & 3);
-          if (i < n) {
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-              if (j + h < q) {
-                double *o = out + (int64_t)(j + h) * ld + i;
-                *o = subtract ? *o - acc[x][y][h] : acc[x][y][h];
-              }
-          }
-        }
     }
+    const int c0 = now.cg * KR_NQ;
+    if (c0 + wc < q) { // warp-uniform: warps past the last column have nothing to do
+      const double *sZ = kr_gemm_smem + slot * STAGE, *sY = sZ + KR_NK * KR_NZL;
+      const double *fA = sZ + (lane & 3) * KR_NZL + wr + (lane >> 2);
+      const double *fB = sY + (wc + (lane >> 2)) * KR_NYL + (lane & 3);
+#pragma unroll
+      for (int kk = 0; kk < KR_NK; kk += 4) {
+        double fa[2], fb[4];
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+          fa[x] = fA[kk * KR_NZL + 8 * x];
+#pragma unroll
+        for (int y = 0; y < 4; y++)
+          fb[y] = fB[8 * y * KR_NYL + kk];
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+          for (int y = 0; y < 4; y++)
+            dmma_8x8x4(acc[x][y][0], acc[x][y][1], fa[x], fb[y]);
+      }
+      if (now.ch == nchunks - 1) {
+        const int64_t r0 = now.rt * KR_NT;
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+          for (int y = 0; y < 4; y++) {
+            const int64_t i = r0 + wr + 8 * x + (lane >> 2);
+            const int j = c0 + wc + 8 * y + 2 * (lane & 3);
+            if (i < n) {
+#pragma unroll
+              for (int h = 0; h < 2; h++)
+                if (j + h < q) {
+                  double *o = out + (int64_t)(j + h) * ld + i;
+                  *o = subtract ? *o - acc[x][y][h] : acc[x][y][h];
+                }
+            }
+          }
+      }
+    }
+    slot = (slot + 1) % KR_NS;
   }
+  cp_async_wait<0>();
+  __syncthreads(); // the next product may stage its chunks
 }
 
 // X[:, i] -= sum_j S[:, j] * Cc(j, i) for i < k, j < ns (X, S column-major
@@ -578,11 +570,6 @@ template <class Team>
 KR_DEV void team_combine(Team &tm, int64_t n, const double *Z, int64_t ld, int zc, const double *Y,
                          int ldy, int roff, int q, double *out) {
   team_gemm_nn(tm, n, Z, ld, zc, Y, ldy, roff, q, out, false);
-}
-
-// dynamic shared memory of a kernel that runs the block solver's products
-__host__ __device__ constexpr size_t lobpcg_dyn_smem_bytes() {
-  return gram_tiled_smem_bytes() > gemm_nn_smem_bytes() ? gram_tiled_smem_bytes() : gemm_nn_smem_bytes();
 }
 
 } // namespace kr

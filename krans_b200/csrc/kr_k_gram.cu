@@ -1,6 +1,6 @@
 // Kernel TU: the block solver's dense products on raw device arrays
 // (krans_block_gram, krans_block_gemm_tn, krans_block_combine): the same
-// device code as inside the LOBPCG kernel (team_gram_sym_tiled, team_gemm_tn,
+// device code as inside the LOBPCG kernel (team_tn_panels, team_gemm_tn,
 // team_gemm_nn), run by every block of a cooperative launch, so that they can
 // be tested and timed on their own.
 #include <algorithm>
@@ -15,7 +15,7 @@ __global__ void __launch_bounds__(512) block_gram_kernel(int64_t n, const double
                                                          GridBarrierState *gb, double *gpart, int *status) {
   __shared__ TeamShared sh;
   TeamGrid tm{&sh, status, gb, gpart, 0, 0};
-  team_gram_sym_tiled(tm, n, Z, W, ld, p, S, G, part);
+  team_tn_panels<true>(tm, n, Z, p, W, p, ld, S, G, part);
 }
 
 __global__ void __launch_bounds__(512) block_gemm_tn_kernel(int64_t n, const double *A, int a, const double *B,
@@ -112,7 +112,7 @@ extern "C" int krans_block_gram(krans_ctx *ctx, int64_t n, int64_t p, const doub
   KR_CUDA(cudaSetDevice(ctx->device));
   std::lock_guard<std::mutex> lk(ctx->mu);
   const void *k = (const void *)block_gram_kernel;
-  const int blocks = coop_blocks(k, ctx, gram_tiled_smem_bytes());
+  const int blocks = coop_blocks(k, ctx, tn_panel_smem_bytes());
   const int64_t tp = (p + KR_GT - 1) / KR_GT;
   const size_t part = (size_t)(2 * blocks + tp * (tp + 1) / 2) * 2 * KR_GT * KR_GT;
   char *ws = nullptr;
@@ -131,7 +131,7 @@ extern "C" int krans_block_gram(krans_ctx *ctx, int64_t n, int64_t p, const doub
   void *args[] = {(void *)&n, (void *)&Z, (void *)&W, (void *)&ld, (void *)&pi, (void *)&S, (void *)&G,
                   (void *)&pt, (void *)&gb, (void *)&gpart, (void *)&status};
   if (e == cudaSuccess)
-    e = timed_coop(k, blocks, args, gram_tiled_smem_bytes(), s, device_ms);
+    e = timed_coop(k, blocks, args, tn_panel_smem_bytes(), s, device_ms);
   int h_status = 0;
   if (e == cudaSuccess)
     e = cudaMemcpy(&h_status, status, sizeof(int), cudaMemcpyDeviceToHost);
@@ -153,7 +153,7 @@ extern "C" int krans_block_gemm_tn(krans_ctx *ctx, int64_t n, int64_t a, const d
   KR_CUDA(cudaSetDevice(ctx->device));
   std::lock_guard<std::mutex> lk(ctx->mu);
   const void *k = (const void *)block_gemm_tn_kernel;
-  const int blocks = coop_blocks(k, ctx, gram_tiled_smem_bytes());
+  const int blocks = coop_blocks(k, ctx, tn_panel_smem_bytes());
   // partials of both forms: the panel form's (2 blocks + tiles) 64 x 64 tiles,
   // the direct form's a x b per block
   const int64_t tiles = ((a + KR_GT - 1) / KR_GT) * ((b + KR_GT - 1) / KR_GT);
@@ -174,7 +174,7 @@ extern "C" int krans_block_gemm_tn(krans_ctx *ctx, int64_t n, int64_t a, const d
   void *args[] = {(void *)&n, (void *)&A, (void *)&ai, (void *)&B, (void *)&bi, (void *)&ld, (void *)&C,
                   (void *)&pt, (void *)&gb, (void *)&gpart, (void *)&status};
   if (e == cudaSuccess)
-    e = timed_coop(k, blocks, args, gram_tiled_smem_bytes(), s, device_ms);
+    e = timed_coop(k, blocks, args, tn_panel_smem_bytes(), s, device_ms);
   int h_status = 0;
   if (e == cudaSuccess)
     e = cudaMemcpy(&h_status, status, sizeof(int), cudaMemcpyDeviceToHost);

@@ -7,9 +7,9 @@
 
 namespace kr {
 
-cudaError_t launch_lobpcg_cluster(const LobpcgDesc *d_dev, int csize, cudaStream_t s) {
+cudaError_t launch_lobpcg_cluster(const LobpcgDesc &d, const LobpcgDesc *d_dev, int csize, cudaStream_t s) {
   const void *k = (const void *)lobpcg_cluster_kernel;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lobpcg_dyn_smem_bytes());
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLobpcgMaxDynSmem);
   if (e == cudaSuccess && csize > 8)
     e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess)
@@ -18,7 +18,7 @@ cudaError_t launch_lobpcg_cluster(const LobpcgDesc *d_dev, int csize, cudaStream
   cudaLaunchAttribute at[1];
   cfg.gridDim = dim3(csize);
   cfg.blockDim = dim3(512);
-  cfg.dynamicSmemBytes = lobpcg_dyn_smem_bytes();
+  cfg.dynamicSmemBytes = lobpcg_dyn_smem_bytes(d);
   cfg.stream = s;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = csize;

@@ -5,12 +5,12 @@
 
 namespace kr {
 
-cudaError_t launch_lobpcg_cta(const LobpcgDesc *d_dev, int threads, cudaStream_t s) {
+cudaError_t launch_lobpcg_cta(const LobpcgDesc &d, const LobpcgDesc *d_dev, int threads, cudaStream_t s) {
   static const cudaError_t attr = cudaFuncSetAttribute(
-      (const void *)lobpcg_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lobpcg_dyn_smem_bytes());
+      (const void *)lobpcg_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLobpcgMaxDynSmem);
   if (attr != cudaSuccess)
     return attr;
-  lobpcg_cta_kernel<<<1, threads, lobpcg_dyn_smem_bytes(), s>>>(d_dev);
+  lobpcg_cta_kernel<<<1, threads, lobpcg_dyn_smem_bytes(d), s>>>(d_dev);
   return cudaGetLastError();
 }
 

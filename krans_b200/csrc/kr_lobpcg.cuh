@@ -19,6 +19,19 @@
 
 namespace kr {
 
+// Dynamic shared memory of a LOBPCG launch: what the forms of the dense
+// products need that its sizes reach (blocks of up to pmax columns; products of
+// up to max(bs, k_target + 2) output columns). What is not taken stays L1 cache,
+// which the gathers of a one-block solve live on (n = 6000, 12 columns: 381 ms
+// with none taken, 417 ms with 110 KB).
+constexpr size_t kLobpcgMaxDynSmem =
+    tn_panel_smem_bytes() > gemm_nn_smem_bytes() ? tn_panel_smem_bytes() : gemm_nn_smem_bytes();
+inline size_t lobpcg_dyn_smem_bytes(const LobpcgDesc &d) {
+  if (d.F.cols >= KR_TN_ROWS && d.pmax >= KR_TN_COLS)
+    return kLobpcgMaxDynSmem;
+  return d.bs > KR_NQ_DIRECT || d.k_target + 2 > KR_NQ_DIRECT ? gemm_nn_smem_bytes() : 0;
+}
+
 template <class Team> struct LobpcgSolver {
   Team &tm;
   const LobpcgDesc &d;
@@ -341,8 +354,8 @@ template <class Team> struct LobpcgSolver {
 
   // one Cholesky-QR round: out = V chol(V^T V)^-T (V unchanged)
   __device__ __noinline__ bool cholqr_round(const double *V, int64_t k, double tol, double *out) {
-    if (n >= 131072 && k >= 32)
-      team_gram_sym_tiled(tm, n, V, nullptr, ldn, (int)k, d.Sj, nullptr, d.gram_part);
+    if (n >= KR_TN_ROWS && k >= KR_TN_COLS)
+      team_tn_panels<true>(tm, n, V, (int)k, nullptr, (int)k, ldn, d.Sj, nullptr, d.gram_part);
     else
       team_gemm_tn(tm, n, V, (int)k, V, (int)k, ldn, d.Sj, d.gram_part);
     gram_flops += 2.0 * (double)n * k * k;
@@ -442,8 +455,8 @@ template <class Team> struct LobpcgSolver {
 
   __device__ __noinline__ void form_gram(const double *Zb, const double *AZb, int p) {
     const uint64_t t0 = globaltimer_ns();
-    if (n >= 131072 && p >= 32) {
-      team_gram_sym_tiled(tm, n, Zb, AZb, ldn, p, d.S, d.G, d.gram_part); // both in one pass
+    if (n >= KR_TN_ROWS && p >= KR_TN_COLS) {
+      team_tn_panels<true>(tm, n, Zb, p, AZb, p, ldn, d.S, d.G, d.gram_part); // both in one pass
     } else {
       team_gram2_direct(tm, n, Zb, AZb, ldn, p, d.S, d.G, d.gram_part); // both in one pass
     }

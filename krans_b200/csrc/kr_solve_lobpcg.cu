@@ -317,8 +317,8 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
 // ---------------------------------------------------------------------------
 namespace kr {
 
-cudaError_t launch_lobpcg_cluster(const LobpcgDesc *d_dev, int csize, cudaStream_t s);
-cudaError_t launch_lobpcg_cta(const LobpcgDesc *d_dev, int threads, cudaStream_t s);
+cudaError_t launch_lobpcg_cluster(const LobpcgDesc &d, const LobpcgDesc *d_dev, int csize, cudaStream_t s);
+cudaError_t launch_lobpcg_cta(const LobpcgDesc &d, const LobpcgDesc *d_dev, int threads, cudaStream_t s);
 cudaError_t launch_basis_max_residual(const CsrView &F, const double *basis, int64_t ldb, const int64_t *nf,
                                       double *out, cudaStream_t s);
 
@@ -471,7 +471,7 @@ int lobpcg_async_launch(LobpcgAsync *a, cudaStream_t s) {
   if (e == cudaSuccess)
     e = cudaEventRecord(a->ev0, s);
   if (e == cudaSuccess)
-    e = a->ncta > 1 ? launch_lobpcg_cluster(a->d_desc, a->ncta, s) : launch_lobpcg_cta(a->d_desc, 512, s);
+    e = a->ncta > 1 ? launch_lobpcg_cluster(a->d, a->d_desc, a->ncta, s) : launch_lobpcg_cta(a->d, a->d_desc, 512, s);
   if (e == cudaSuccess)
     e = cudaEventRecord(a->ev1, s);
   if (e == cudaSuccess)
