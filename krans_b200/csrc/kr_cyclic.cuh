@@ -205,6 +205,8 @@ template <class Team, class KT> struct CyclicSolver {
                                      double *rnorm_out, bool precond = true) {
     if (precond && d.o.precond_aat != KRANS_PRECOND_NONE)
       return cg_pre(rhs, u, maxit, rel_tol, bd_tol, rnorm_out);
+    if (d.F.ulen != 2)
+      return cg_dir(rhs, u, maxit, rel_tol, bd_tol, rnorm_out);
     double *r = d.cgr, *t = d.tn, *ts = d.cgts, *us = d.cgus;
     double rr = 0.0;
     team_for(tm, n, [&](int64_t i) { u[i] = 0.0; });
@@ -259,6 +261,114 @@ template <class Team, class KT> struct CyclicSolver {
     }
     if (started)
       cg_result(ts, us, pending, alpha, u);
+    *rnorm_out = rnorm;
+    return k;
+  }
+
+  // The same with the direction p kept, for operators whose rows are not all of
+  // 2 entries. There the matrix outweighs the vectors (a row of 8 or 9 entries
+  // moves 100 bytes against 60 of r, p and F F^T p), and on the ill-conditioned
+  // planted kernels the two recurrences part: with this one a mixed solve stalls
+  // at cg_maxit and continues in FP64 as it always has. r and p are stored
+  // interleaved, so the gather of r + beta p at each entry of F^T is one 16-byte
+  // load; the update of p is folded into that gather and into the second SpMV's
+  // epilogue.
+  __device__ __noinline__ int64_t cg_dir(const double *rhs, double *u, int64_t maxit, double rel_tol, double bd_tol,
+                                         double *rnorm_out) {
+    double2 *rp = d.rp;
+    double *Ap = d.Ap, *tn = d.tn;
+    double rr = 0.0;
+    team_for(tm, n, [&](int64_t i) { u[i] = 0.0; });
+    team_for(tm, m, [&](int64_t i) {
+      const double x = rhs[i];
+      rp[i] = make_double2(x, x);
+      rr += x * x;
+    });
+    rr = tm.sum1(rr);
+    c.bytes += 24.0 * m + 8.0 * n;
+    const double rhsn = sqrt(rr > 0.0 ? rr : 0.0);
+    *rnorm_out = rhsn;
+    if (!(rhsn > 0.0) || !isfinite(rhsn))
+      return 0;
+    double rz = rr; // z = r without a preconditioner
+    if (!(rz > 0.0) || !isfinite(rz))
+      return 0;
+    double rnorm = sqrt(rz);
+    const double tol = fmax(rel_tol * rnorm, 1e-30);
+    *rnorm_out = rnorm;
+    if (rnorm <= tol)
+      return 0;
+    int64_t k = 0;
+    double beta = 0.0;
+    for (; k < maxit && tm.ok(); ++k) {
+      const double bq = beta;
+      csr_mv_pre<double>(
+          tm, d.B,
+          [&](int32_t cc) {
+            const double2 q = rp[cc];
+            return q.x + bq * q.y;
+          },
+          NoPrologue(), [&](int i, int, double s, char) { tn[i] = s; });
+      count_B();
+      c.bytes += spmv_bytes(d.B.rows, d.B.cols, d.B.nnz, 8, 16, 8);
+      tm.sync();
+      double pap = 0.0;
+      csr_mv_pre<double>(
+          tm, d.F, [&](int32_t cc) { return tn[cc]; }, [&](int i, int) { return rp[i]; },
+          [&](int i, int, double s, double2 q) {
+            const double pn = q.x + bq * q.y;
+            rp[i].y = pn;
+            Ap[i] = s;
+            pap += pn * s;
+          });
+      count_F();
+      c.bytes += spmv_bytes(d.F.rows, d.F.cols, d.F.nnz, 8, 8, 8) + 24.0 * m;
+      pap = tm.sum1(pap);
+      if (!isfinite(pap) || fabs(pap) <= bd_tol)
+        break;
+      const double alpha = rz / pap;
+      double rzn = 0.0;
+      team_for4(tm, m, [&](const int64_t *ix, int cnt) {
+        double rv[4], av[4];
+#pragma unroll
+        for (int u4 = 0; u4 < 4; u4++)
+          if (u4 < cnt) {
+            rv[u4] = rp[ix[u4]].x;
+            av[u4] = Ap[ix[u4]];
+          }
+#pragma unroll
+        for (int u4 = 0; u4 < 4; u4++)
+          if (u4 < cnt) {
+            const double ri = rv[u4] - alpha * av[u4];
+            rp[ix[u4]].x = ri;
+            rzn += ri * ri;
+          }
+      });
+      team_for4(tm, n, [&](const int64_t *ix, int cnt) {
+        double uv[4], tv[4];
+#pragma unroll
+        for (int u4 = 0; u4 < 4; u4++)
+          if (u4 < cnt) {
+            uv[u4] = u[ix[u4]];
+            tv[u4] = tn[ix[u4]];
+          }
+#pragma unroll
+        for (int u4 = 0; u4 < 4; u4++)
+          if (u4 < cnt)
+            u[ix[u4]] = uv[u4] + alpha * tv[u4];
+      });
+      rzn = tm.sum1(rzn); // its barrier also publishes r for the next gather
+      c.bytes += 24.0 * m + 24.0 * n;
+      if (!isfinite(rzn))
+        break;
+      rnorm = sqrt(rzn > 0.0 ? rzn : 0.0);
+      if (rnorm <= tol) {
+        ++k;
+        break;
+      }
+      beta = rzn / fmax(1e-300, rz);
+      rz = rzn;
+    }
     *rnorm_out = rnorm;
     return k;
   }

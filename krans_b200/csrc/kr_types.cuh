@@ -91,6 +91,8 @@ struct CyclicDesc {
   double *tmv, *wm;                  // m-vectors
   double *cgr;                       // CG: the residual (preconditioned CG: z = M^-1 r) that F^T gathers (m)
   double *cgts, *cgus;               // CG: F^T p and F^T w by slot of F^T's sorted order (n)
+  double2 *rp;                       // CG with a direction: residual and direction, interleaved (m)
+  double *Ap;                        // and F F^T p (m)
   double *r_pre, *dinv, *sd_q, *sd_Oq; // preconditioned CG: residual, Jacobi weights, SD vectors (m)
   double *cgt;                         // preconditioned CG: F^T p (n; the SD steps work in tn)
   double *alpha, *beta;              // ncv + 2
@@ -149,6 +151,8 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
   double *tmv = c.take<double>(p.ldm), *wm = c.take<double>(p.ldm);
   double *cgr = c.take<double>(p.ldm);
   double *cgts = c.take<double>(p.ldn), *cgus = c.take<double>(p.ldn);
+  double2 *rp = c.take<double2>(p.ldm);
+  double *Ap = c.take<double>(p.ldm);
   double *alpha = c.take<double>(p.ncv + 2), *beta = c.take<double>(p.ncv + 2);
   double *Tb = c.take<double>((p.ncv + 1) * p.ncv), *Vt = c.take<double>(p.ncv * p.ncv);
   double *sv = c.take<double>(p.ncv + 1);
@@ -182,6 +186,7 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
     if (p.own_basis) d->basis = basis;
     d->y0 = y0; d->v = v; d->vp = vp; d->best_v = best_v; d->tn = tn;
     d->tmv = tmv; d->wm = wm; d->cgr = cgr; d->cgts = cgts; d->cgus = cgus;
+    d->rp = rp; d->Ap = Ap;
     d->alpha = alpha; d->beta = beta; d->Tb = Tb; d->Vt = Vt; d->sv = sv; d->ord = ord;
     d->eig_cs = eig_cs; d->eig_pq = eig_pq; d->eig_ord = eig_ord;
     if (p.own_basis) { d->status = status; d->res = res; }
