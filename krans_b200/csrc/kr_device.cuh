@@ -374,37 +374,74 @@ template <class Team, class TX> KR_DEV double team_nrm2(Team &tm, int64_t len, c
   return sqrt(tm.sum1(s));
 }
 
+// This thread's share of <S_k, w> for K columns of S (stride ld), two rows at
+// a time: the 2 K + 2 loads are issued together before their products, which
+// keeps enough of them in flight whatever the compiler makes of the loop (left
+// to it, one build of the same source ran a Golub-Kahan step of 13877 incidence
+// columns on two blocks in 150 us and the next in 190; this form takes 122).
+// Columns from qn on repeat the last one (their sums are not used).
+template <int K, class Team, class TS, class TW>
+KR_DEV void dot_columns(Team &tm, int64_t len, const TS *S, int64_t ld, int qn, const TW *w, double (&acc)[K]) {
+  const int64_t nt = tm.nthreads();
+  const TS *col[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    acc[k] = 0.0;
+    col[k] = S + (int64_t)min(k, qn - 1) * ld;
+  }
+  int64_t i = tm.tid();
+  for (; i + nt < len; i += 2 * nt) {
+    TS s0[K], s1[K];
+    const TW w0 = w[i], w1 = w[i + nt];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      s0[k] = col[k][i];
+      s1[k] = col[k][i + nt];
+    }
+    const double d0 = to_d(w0), d1 = to_d(w1);
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      acc[k] += to_d(s0[k]) * d0;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      acc[k] += to_d(s1[k]) * d1;
+  }
+  if (i < len) {
+    const double d0 = to_d(w[i]);
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      acc[k] += to_d(col[k][i]) * d0;
+  }
+}
+
 // h[q] = <S_q, w> for q < ns (S columns at stride ld); results in tm.sh->h
 // (all threads of every block see them after the call). Groups of 8 columns
 // share one sweep over w; up to KR_MDOT columns share one team reduction (one
 // per group, with every thread summing every value, made the Gram-Schmidt passes
 // of small solves wait on reductions: a Golub-Kahan step of a 1000-unknown
-// solve took 34 us, and takes 15).
+// solve took 34 us, and takes 14).
 template <class Team, class TS, class TW>
 KR_DEV void team_multidot(Team &tm, int64_t len, const TS *S, int64_t ld, int ns, const TW *w) {
-  const int64_t nt = tm.nthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   double *part = tm.sh->dots;
   for (int c0 = 0; c0 < ns; c0 += KR_MDOT) {
     const int cnt = min(KR_MDOT, ns - c0);
     for (int g = 0; g < cnt; g += KR_RED_K) {
-      double acc[KR_RED_K];
-#pragma unroll
-      for (int k = 0; k < KR_RED_K; k++)
-        acc[k] = 0.0;
       const int qn = min(KR_RED_K, cnt - g);
       const TS *Sg = S + (int64_t)(c0 + g) * ld;
-#pragma unroll 4
-      for (int64_t i = tm.tid(); i < len; i += nt) {
-        const double wi = to_d(w[i]);
-#pragma unroll
-        for (int k = 0; k < KR_RED_K; k++)
-          if (k < qn)
-            acc[k] += to_d(Sg[(int64_t)k * ld + i]) * wi;
+      if (qn > KR_RED_K / 2) {
+        double acc[KR_RED_K];
+        dot_columns<KR_RED_K>(tm, len, Sg, ld, qn, w, acc);
+        const double t = warp_sums<KR_RED_K>(acc);
+        if ((lane & 3) == 0)
+          part[(g + (lane >> 2)) * KR_RED_LD + wid] = t;
+      } else {
+        double acc[KR_RED_K / 2];
+        dot_columns<KR_RED_K / 2>(tm, len, Sg, ld, qn, w, acc);
+        const double t = warp_sums<KR_RED_K / 2>(acc);
+        if ((lane & 7) == 0)
+          part[(g + (lane >> 3)) * KR_RED_LD + wid] = t;
       }
-      const double t = warp_sums<KR_RED_K>(acc);
-      if ((lane & 3) == 0)
-        part[(g + (lane >> 2)) * KR_RED_LD + wid] = t;
     }
     __syncthreads();
     const double s = threadIdx.x < (unsigned)cnt ? sum_warps(part + threadIdx.x * KR_RED_LD, nw) : 0.0;
