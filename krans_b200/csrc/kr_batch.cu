@@ -20,6 +20,11 @@
 namespace kr {
 
 
+std::atomic<int> &device_servers(int device) {
+  static std::atomic<int> live[64];
+  return live[device & 63];
+}
+
 static void mt_seed(RngState &s, uint32_t seed) {
   memset(&s, 0, sizeof s);
   s.mt[0] = seed;
@@ -1052,6 +1057,7 @@ int krans_server_create(krans_ctx *ctx, const krans_server_opts *opts, krans_ser
     delete s;
     return cuda_fail(e, "server streams", __FILE__, __LINE__);
   }
+  device_servers(ctx->device)++;
   s->worker = std::thread([s] { s->run(); });
   *out = s;
   return KRANS_OK;
@@ -1089,6 +1095,7 @@ int krans_server_destroy(krans_server *s) {
     cudaStreamDestroy(s->ctl);
   if (s->ctx_ready)
     cudaEventDestroy(s->ctx_ready);
+  device_servers(s->ctx->device)--;
   delete s;
   return KRANS_OK;
 }

@@ -67,6 +67,8 @@ struct krans_ctx {
   int partial_blocks = 0;
   krans_batch_tuning tune{16384, 120000, 8, {1, 2, 4, 8, 16, 32}}; // batched-launch knobs in effect
   std::mutex mu;
+  // blocks of a single solve's cluster: cyclic FP64, cyclic mixed, LOBPCG (-1: not asked yet; under mu)
+  int solo_cluster[3] = {-1, -1, -1};
 };
 
 struct krans_mat {
@@ -149,6 +151,22 @@ inline int tuned_lanes(const krans_ctx *ctx, int64_t rows, int64_t nnz) {
     b++;
   return ctx->tune.lanes[b];
 }
+// Team of a single solve by its size m + n (KRANS_TEAM_AUTO): one block below
+// the first line, a cluster of 16 blocks between them, the whole GPU from the
+// second on. One block costs the least per step and many blocks the least per
+// entry. Measured (ms), incidence matrices of mean degree 6, mixed precision, one
+// block / cluster / whole GPU: m + n = 4000: 22.8 / 25.4 / 44; 8000: 43 / 27.8 /
+// 48; 32000: 162 / 37 / 58; 64000: 377 / 58 / 67; 128000: - / 84 / 68. Block
+// LOBPCG: 5000: 98 / 76 / 96; 10000: 174 / 95 / 119; 30000: 390 / 113 / 128; 60000:
+// 839 / 155 / 147.
+constexpr int64_t kSoloClusterMin = 5000, kSoloGridMin = 100000;
+constexpr int64_t kSoloLobpcgClusterMin = 4000, kSoloLobpcgGridMin = 40000;
+// While a server lives on the device, a solve stays on one block up to here: the
+// server's resident launch leaves few SMs free, which one block finds and a
+// cluster or the whole GPU would have to wait for.
+constexpr int64_t kServedGridMin = 120000;
+// live servers of this process on a device
+std::atomic<int> &device_servers(int device);
 // A (or its stored transpose) as the solvers' device code sees it
 inline CsrView csr_view(const krans_mat *A, bool trans) {
   if (trans)

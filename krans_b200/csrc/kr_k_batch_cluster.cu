@@ -40,6 +40,20 @@ int cyclic_batch_cluster_max(bool mixed, int csize, int sms, size_t dyn_smem) {
   return maxc;
 }
 
+int cyclic_solo_cluster(bool mixed) {
+  for (int csize = 16; csize >= 8; csize /= 2) {
+    if (csize > 8)
+      cudaFuncSetAttribute(cl_kernel(mixed), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = cl_config(1, csize, 0, nullptr, at);
+    int fits = 0;
+    if (cudaOccupancyMaxActiveClusters(&fits, cl_kernel(mixed), &cfg) == cudaSuccess && fits > 0)
+      return csize;
+    cudaGetLastError();
+  }
+  return 0;
+}
+
 cudaError_t launch_cyclic_batch_cluster(bool mixed, int nclusters, int csize, size_t dyn_smem, cudaStream_t s,
                                         const CyclicRequestDev *reqs_large, int n_large, int *queue_large,
                                         char *ws_large, size_t stride_large, const CyclicRequestDev *reqs_small,

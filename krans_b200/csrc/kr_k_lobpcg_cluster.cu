@@ -29,6 +29,31 @@ cudaError_t launch_lobpcg_cluster(const LobpcgDesc &d, const LobpcgDesc *d_dev, 
   return cudaLaunchKernelEx(&cfg, lobpcg_cluster_kernel, d_dev);
 }
 
+int lobpcg_solo_cluster() {
+  const void *k = (const void *)lobpcg_cluster_kernel;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLobpcgMaxDynSmem);
+  for (int csize = 16; csize >= 8; csize /= 2) {
+    if (csize > 8)
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = dim3(csize);
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = kLobpcgMaxDynSmem;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = csize;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fits = 0;
+    if (cudaOccupancyMaxActiveClusters(&fits, k, &cfg) == cudaSuccess && fits > 0)
+      return csize;
+    cudaGetLastError();
+  }
+  return 0;
+}
+
 __global__ void __launch_bounds__(512) basis_max_residual_kernel(CsrView F, const double *basis, int64_t ldb,
                                                                  const int64_t *nf, double *out) {
   __shared__ TeamShared sh;

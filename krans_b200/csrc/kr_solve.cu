@@ -42,9 +42,9 @@ struct RunOut {
   int64_t fallback_from = 0; // vectors the mixed run had accepted
 };
 
-// One find_right_nullspace run on the device (a grid team, or one thread
-// block through the persistent batched kernel with a single request); the
-// basis rows are copied into new vectors owned by the caller.
+// One find_right_nullspace run on the device (a grid team, or one thread block
+// or one cluster through the persistent batched kernels with a single request);
+// the basis rows are copied into new vectors owned by the caller.
 // `prefill` (nprefill rows, stride round_up(n, 32)) and `frob_init` continue
 // an earlier run: its accepted vectors are copied into the basis first and
 // its ||A||_F estimate is kept. A MIXED run that stops short of k_target with
@@ -66,9 +66,17 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
   KR_CHECK_ARG(o.precond_aat >= KRANS_PRECOND_NONE && o.precond_aat <= KRANS_PRECOND_SD && o.precond_steps >= 1 &&
                    o.precond_steps <= 1000,
                "cyclic: precond_aat must be a KRANS_PRECOND_* value, precond_steps in [1, 1000]");
-  int team = o.team;
-  if (team == KRANS_TEAM_AUTO)
-    team = (F.rows + F.cols) < 120000 ? KRANS_TEAM_CTA : KRANS_TEAM_GRID;
+  int team = o.team, csize = 0; // csize: blocks of a cluster team, else 0
+  if (team == KRANS_TEAM_AUTO) {
+    const int64_t size = F.rows + F.cols;
+    const bool served = device_servers(ctx->device).load() > 0;
+    if (!served && size >= kSoloClusterMin && size < kSoloGridMin) {
+      if (ctx->solo_cluster[mixed] < 0)
+        ctx->solo_cluster[mixed] = cyclic_solo_cluster(mixed);
+      csize = ctx->solo_cluster[mixed];
+    }
+    team = size < (served ? kServedGridMin : kSoloGridMin) ? KRANS_TEAM_CTA : KRANS_TEAM_GRID;
+  }
   const bool grid = team == KRANS_TEAM_GRID;
   const int threads = 512;
   CyclicPlan p;
@@ -102,7 +110,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
     d_res = c.take<CyclicDevResult>(1);
     d_status = c.take<int32_t>(1);
     d_mr = c.take<double>(1);
-    d_queue = c.take<int>(1);
+    d_queue = c.take<int>(2);
     return c.off + 256;
   };
   const size_t bytes = layout(nullptr);
@@ -119,7 +127,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
   if (e == cudaSuccess)
     e = cudaMemsetAsync(d_status, 0, 4, s);
   if (e == cudaSuccess)
-    e = cudaMemsetAsync(d_queue, 0, 4, s);
+    e = cudaMemsetAsync(d_queue, 0, 8, s);
   CyclicDesc d;
   CyclicRequestDev q;
   if (grid) {
@@ -164,8 +172,10 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
   if (e == cudaSuccess)
     e = cudaEventRecord(e0, s);
   if (e == cudaSuccess)
-    e = grid ? launch_cyclic_grid(mixed, d, p.grid_blocks, threads, s)
-             : launch_cyclic_batch_cta(mixed, 1, threads,
+    e = grid    ? launch_cyclic_grid(mixed, d, p.grid_blocks, threads, s)
+        : csize ? launch_cyclic_batch_cluster(mixed, 1, csize, 0, s, d_req, 1, d_queue, slot, 0, nullptr, 0,
+                                              d_queue + 1, slot, 0, nullptr, 0)
+                : launch_cyclic_batch_cta(mixed, 1, threads,
                                        cta_cg_smem_bytes(p.ldm, p.ldn) <= cta_smem_cap()
                                            ? cta_cg_smem_bytes(p.ldm, p.ldn)
                                            : 0,

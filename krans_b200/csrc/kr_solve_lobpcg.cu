@@ -128,6 +128,11 @@ static const char *lobpcg_err_msg(int code) {
 
 } // namespace kr
 
+namespace kr {
+cudaError_t launch_lobpcg_cluster(const LobpcgDesc &d, const LobpcgDesc *d_dev, int csize, cudaStream_t s);
+int lobpcg_solo_cluster(); // as cyclic_solo_cluster
+} // namespace kr
+
 using namespace kr;
 
 extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng *rng,
@@ -180,10 +185,18 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
 
   const int64_t pmax = std::max<int64_t>(3 * bs, 2 * k_target + 2);
   int team = o.team;
-  if (team == KRANS_TEAM_AUTO)
-    team = (m + n) < 120000 ? KRANS_TEAM_CTA : KRANS_TEAM_GRID;
+  int csize = 0; // blocks of a cluster team, else 0
+  if (team == KRANS_TEAM_AUTO) {
+    const bool served = device_servers(ctx->device).load() > 0;
+    if (!served && m + n >= kSoloLobpcgClusterMin && m + n < kSoloLobpcgGridMin) {
+      if (ctx->solo_cluster[2] < 0)
+        ctx->solo_cluster[2] = lobpcg_solo_cluster();
+      csize = ctx->solo_cluster[2];
+    }
+    team = m + n < (served ? kServedGridMin : kSoloLobpcgGridMin) ? KRANS_TEAM_CTA : KRANS_TEAM_GRID;
+  }
   const int threads = 512;
-  const int ncta = team == KRANS_TEAM_GRID ? lobpcg_grid_blocks(ctx, threads) : 1;
+  const int ncta = team == KRANS_TEAM_GRID ? lobpcg_grid_blocks(ctx, threads) : csize ? csize : 1;
 
   LobpcgDesc d;
   memset(&d, 0, sizeof d);
@@ -231,7 +244,8 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
       e = cudaMemcpyAsync(d_desc, &d, sizeof d, cudaMemcpyHostToDevice, s);
   }
   if (e == cudaSuccess)
-    e = launch_lobpcg(team == KRANS_TEAM_GRID, d, d_desc, ncta, threads, s);
+    e = csize ? launch_lobpcg_cluster(d, d_desc, csize, s)
+              : launch_lobpcg(team == KRANS_TEAM_GRID, d, d_desc, ncta, threads, s);
   if (e == cudaSuccess)
     e = cudaEventRecord(e1, s);
   LobpcgDevResult R;

@@ -295,6 +295,9 @@ int cyclic_batch_cta_per_sm(bool mixed);
 cudaError_t launch_cyclic_batch_cta(bool mixed, int grid, int block, size_t dyn_smem, cudaStream_t s, const CyclicRequestDev *reqs, int count,
                                     int *queue, char *ws, size_t stride, const LaunchFeed *feed);
 int cyclic_batch_cluster_max(bool mixed, int csize, int sms, size_t dyn_smem);
+// blocks of the cluster that runs one solve on its own: 16, or 8 where the device
+// has no room for 16, or 0
+int cyclic_solo_cluster(bool mixed);
 cudaError_t launch_cyclic_batch_cluster(bool mixed, int nclusters, int csize, size_t dyn_smem, cudaStream_t s,
                                         const CyclicRequestDev *reqs_large, int n_large, int *queue_large,
                                         char *ws_large, size_t stride_large, const CyclicRequestDev *reqs_small,
