@@ -67,6 +67,11 @@ struct krans_ctx {
   int partial_blocks = 0;
   krans_batch_tuning tune{16384, 120000, 8, {1, 2, 4, 8, 16, 32}}; // batched-launch knobs in effect
   std::mutex mu;
+  // Kept scratch of the calls that work on the context's stream (see ws_take)
+  std::mutex ws_mu;
+  char *ws = nullptr;
+  size_t ws_bytes = 0;
+  bool ws_busy = false;
   // blocks of a single solve's cluster: cyclic FP64, cyclic mixed, LOBPCG (-1: not asked yet; under mu)
   int solo_cluster[3] = {-1, -1, -1};
 };
@@ -119,6 +124,25 @@ int spmv_rows_per_block(int64_t rows, int64_t nnz);
 // allocation with budget accounting
 int dev_alloc(krans_ctx *ctx, void **p, size_t bytes);
 void dev_free(krans_ctx *ctx, void *p, size_t bytes);
+// Scratch of one call on the context's stream, kept from call to call: a
+// cudaMalloc and cudaFree per call cost 0.3 ms and more (the three block products
+// of a 36-column block: 1.35 ms a round with them). One call holds it at a time,
+// another (a nested solve, another thread) gets an allocation of its own. What a
+// call has queued may still use it after ws_give: the next holder queues on the
+// same stream. At most kWsKeep bytes are kept; a call that needs more, or finds
+// the budget or the device short, allocates for itself, and dev_alloc gives idle
+// scratch back before it fails.
+constexpr size_t kWsKeep = (size_t)256 << 20;
+struct WsHold {
+  void *p = nullptr;
+  size_t bytes = 0;
+  enum { kNone, kKept, kOwn, kOwnAsync } mode = kNone;
+};
+// stream_ordered: an allocation of the call's own is freed in stream order (the
+// caller need not have waited for its kernels)
+int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, bool stream_ordered = false);
+void ws_give(krans_ctx *ctx, WsHold *w);
+bool ws_release(krans_ctx *ctx); // frees idle scratch; true if there was any
 // Stream-ordered forms (cudaMallocAsync / cudaFreeAsync on `s`): neither
 // waits for kernels running on other streams, unlike cudaFree, which waits
 // for the whole device. The served paths use them so that releasing one

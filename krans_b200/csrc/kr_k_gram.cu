@@ -45,19 +45,18 @@ static int coop_blocks(const void *k, krans_ctx *ctx, size_t smem) {
 }
 
 // workspace: grid barrier, reduction partials, status, Gram partials
-static int coop_scratch(krans_ctx *ctx, int blocks, size_t part_doubles, char **ws, size_t *bytes,
+static int coop_scratch(krans_ctx *ctx, int blocks, size_t part_doubles, WsHold *ws,
                         GridBarrierState **gb, double **gpart, int **status, double **part) {
   Carver c;
   c.take<GridBarrierState>(1);
   c.take<double>(2 * (size_t)blocks * KR_MDOT);
   c.take<int>(1);
   c.take<double>((int64_t)std::max<size_t>(part_doubles, 1));
-  *bytes = c.off + 256;
-  int rc = dev_alloc(ctx, (void **)ws, *bytes);
+  int rc = ws_take(ctx, c.off + 256, ws);
   if (rc != KRANS_OK)
     return rc;
   Carver d;
-  d.base = *ws;
+  d.base = (char *)ws->p;
   *gb = d.take<GridBarrierState>(1);
   *gpart = d.take<double>(2 * (size_t)blocks * KR_MDOT);
   *status = d.take<int>(1);
@@ -115,12 +114,11 @@ extern "C" int krans_block_gram(krans_ctx *ctx, int64_t n, int64_t p, const doub
   const int blocks = coop_blocks(k, ctx, tn_panel_smem_bytes());
   const int64_t tp = (p + KR_GT - 1) / KR_GT;
   const size_t part = (size_t)(2 * blocks + tp * (tp + 1) / 2) * 2 * KR_GT * KR_GT;
-  char *ws = nullptr;
-  size_t bytes = 0;
+  WsHold ws;
   GridBarrierState *gb;
   double *gpart, *pt;
   int *status;
-  int rc = coop_scratch(ctx, blocks, part, &ws, &bytes, &gb, &gpart, &status, &pt);
+  int rc = coop_scratch(ctx, blocks, part, &ws, &gb, &gpart, &status, &pt);
   if (rc != KRANS_OK)
     return rc;
   cudaStream_t s = ctx->stream;
@@ -135,7 +133,7 @@ extern "C" int krans_block_gram(krans_ctx *ctx, int64_t n, int64_t p, const doub
   int h_status = 0;
   if (e == cudaSuccess)
     e = cudaMemcpy(&h_status, status, sizeof(int), cudaMemcpyDeviceToHost);
-  dev_free(ctx, ws, bytes);
+  ws_give(ctx, &ws);
   if (e != cudaSuccess)
     return cuda_fail(e, "krans_block_gram", __FILE__, __LINE__);
   if (h_status != 0) {
@@ -158,12 +156,11 @@ extern "C" int krans_block_gemm_tn(krans_ctx *ctx, int64_t n, int64_t a, const d
   // the direct form's a x b per block
   const int64_t tiles = ((a + KR_GT - 1) / KR_GT) * ((b + KR_GT - 1) / KR_GT);
   const size_t part = std::max<size_t>((size_t)(2 * blocks + tiles) * KR_GT * KR_GT, (size_t)blocks * a * b);
-  char *ws = nullptr;
-  size_t bytes = 0;
+  WsHold ws;
   GridBarrierState *gb;
   double *gpart, *pt;
   int *status;
-  int rc = coop_scratch(ctx, blocks, part, &ws, &bytes, &gb, &gpart, &status, &pt);
+  int rc = coop_scratch(ctx, blocks, part, &ws, &gb, &gpart, &status, &pt);
   if (rc != KRANS_OK)
     return rc;
   cudaStream_t s = ctx->stream;
@@ -178,7 +175,7 @@ extern "C" int krans_block_gemm_tn(krans_ctx *ctx, int64_t n, int64_t a, const d
   int h_status = 0;
   if (e == cudaSuccess)
     e = cudaMemcpy(&h_status, status, sizeof(int), cudaMemcpyDeviceToHost);
-  dev_free(ctx, ws, bytes);
+  ws_give(ctx, &ws);
   if (e != cudaSuccess)
     return cuda_fail(e, "krans_block_gemm_tn", __FILE__, __LINE__);
   if (h_status != 0) {
@@ -197,12 +194,11 @@ extern "C" int krans_block_combine(krans_ctx *ctx, int64_t n, int64_t zc, int64_
   std::lock_guard<std::mutex> lk(ctx->mu);
   const void *k = (const void *)block_combine_kernel;
   const int blocks = coop_blocks(k, ctx, gemm_nn_smem_bytes());
-  char *ws = nullptr;
-  size_t bytes = 0;
+  WsHold ws;
   GridBarrierState *gb;
   double *gpart, *pt;
   int *status;
-  int rc = coop_scratch(ctx, blocks, 0, &ws, &bytes, &gb, &gpart, &status, &pt);
+  int rc = coop_scratch(ctx, blocks, 0, &ws, &gb, &gpart, &status, &pt);
   if (rc != KRANS_OK)
     return rc;
   cudaStream_t s = ctx->stream;
@@ -214,7 +210,7 @@ extern "C" int krans_block_combine(krans_ctx *ctx, int64_t n, int64_t zc, int64_
                   (void *)&out, (void *)&gb, (void *)&gpart, (void *)&status};
   if (e == cudaSuccess)
     e = timed_coop(k, blocks, args, gemm_nn_smem_bytes(), s, device_ms);
-  dev_free(ctx, ws, bytes);
+  ws_give(ctx, &ws);
   if (e != cudaSuccess)
     return cuda_fail(e, "krans_block_combine", __FILE__, __LINE__);
   return KRANS_OK;

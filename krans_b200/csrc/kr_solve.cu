@@ -114,11 +114,11 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
     return c.off + 256;
   };
   const size_t bytes = layout(nullptr);
-  char *ws = nullptr;
-  int rc = dev_alloc(ctx, (void **)&ws, bytes);
+  WsHold ws;
+  int rc = ws_take(ctx, bytes, &ws);
   if (rc != KRANS_OK)
     return rc;
-  layout(ws);
+  layout((char *)ws.p);
   cudaStream_t s = ctx->stream;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -193,11 +193,11 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (e != cudaSuccess) {
-    dev_free(ctx, ws, bytes);
+    ws_give(ctx, &ws);
     return cuda_fail(e, "cyclic solve launch", __FILE__, __LINE__);
   }
   if (out->r.status != KRANS_OK) {
-    dev_free(ctx, ws, bytes);
+    ws_give(ctx, &ws);
     set_error("cyclic solve: device status %d (a bounded device wait gave up)", out->r.status);
     return out->r.status;
   }
@@ -208,7 +208,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
     RunOut o2;
     rc = run_cyclic(ctx, A, trans, rng, o64, init_right, k_target, ncv, found, &o2, bsrc, out->r.n_found,
                     out->r.frob);
-    dev_free(ctx, ws, bytes);
+    ws_give(ctx, &ws);
     if (rc != KRANS_OK)
       return rc;
     const CyclicDevResult r1 = out->r;
@@ -239,7 +239,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
     }
   }
   cudaStreamSynchronize(s);
-  dev_free(ctx, ws, bytes);
+  ws_give(ctx, &ws);
   return rc;
 }
 

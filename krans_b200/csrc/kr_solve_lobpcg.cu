@@ -209,8 +209,8 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
   d.rng = rng->d;
   d.n_initial = n_initial;
   const size_t bytes = lobpcg_layout(m, n, bs, k_target, pmax, ncta, nullptr, nullptr);
-  char *ws = nullptr;
-  int rc = dev_alloc(ctx, (void **)&ws, bytes);
+  WsHold ws;
+  int rc = ws_take(ctx, bytes, &ws);
   if (rc != KRANS_OK)
     return rc;
   double **d_init = nullptr;
@@ -225,7 +225,7 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
       e = cudaMemcpyAsync(d_init, hinit.data(), sizeof(double *) * (size_t)n_initial, cudaMemcpyHostToDevice, s);
   }
   d.initial = d_init;
-  lobpcg_layout(m, n, bs, k_target, pmax, ncta, ws, &d);
+  lobpcg_layout(m, n, bs, k_target, pmax, ncta, (char *)ws.p, &d);
   LobpcgDesc *d_desc = nullptr;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -264,11 +264,11 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
   if (d_init)
     cudaFree(d_init);
   if (e != cudaSuccess) {
-    dev_free(ctx, ws, bytes);
+    ws_give(ctx, &ws);
     return cuda_fail(e, "lobpcg launch", __FILE__, __LINE__);
   }
   if (R.status != KRANS_OK) {
-    dev_free(ctx, ws, bytes);
+    ws_give(ctx, &ws);
     set_error("LOBPCG: device status %d (a bounded device wait gave up)", R.status);
     return R.status;
   }
@@ -287,7 +287,7 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
     result->phase_ms[i] = R.phase_ms[i];
   result->final_polish_ms = R.final_polish_ms;
   if (R.err_code != kLobErrNone) {
-    dev_free(ctx, ws, bytes);
+    ws_give(ctx, &ws);
     set_error("%s", lobpcg_err_msg(R.err_code));
     return KRANS_ERR_RUNTIME;
   }
@@ -309,7 +309,7 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
   }
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(s);
-  dev_free(ctx, ws, bytes);
+  ws_give(ctx, &ws);
   if (e != cudaSuccess)
     return cuda_fail(e, "lobpcg results", __FILE__, __LINE__);
   if (theta_out)
