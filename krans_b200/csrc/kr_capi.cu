@@ -364,7 +364,122 @@ __global__ void slice_fill_kernel(int64_t slices, const int32_t *off, const int3
   }
 }
 
-__global__ void rng_mt_kernel(RngState *st, double *out, int64_t n) { block_mt_normals(st, out, n); }
+__global__ void __launch_bounds__(1024) rng_mt_kernel(RngState *st, double *out, int64_t n) {
+  __shared__ uint32_t ring[6 * 624]; // 936 attempts a round
+  block_mt_normals(st, out, n, ring, 6);
+}
+// Long draws of the same sequence in three steps. One block runs the MT19937
+// recurrence alone and stores `states` states (the current one first); all SMs
+// then try the polar attempts in them and count the accepted ones per block, and
+// again, each block knowing the counts before it, write their normals; one block
+// takes over the new state. One block doing all of it spends most of its time in
+// log and square root on one SM's FP64 pipe. What is left is the serial
+// recurrence, one barrier per state: 24 vectors of 262144 take 5.4 ms (31 ms
+// with one block, one state and five barriers a round).
+constexpr int kMtTry = 256; // attempts per block
+__global__ void __launch_bounds__(640) rng_mt_states_kernel(const RngState *st, uint32_t *words, int64_t states,
+                                                            int64_t *last) {
+  __shared__ uint32_t ring[2][640]; // a word per thread; the last 16 are not used
+  const int i = threadIdx.x, at = min(i, 623);
+  if (i == 0)
+    *last = -1;
+  uint32_t v = st->mt[at];
+  ring[0][i] = v;
+  if (i < 624)
+    words[i] = v;
+  __syncthreads();
+  for (int64_t b = 1; b < states; b++) {
+    v = mt_next_word(ring[(b - 1) & 1], at);
+    ring[b & 1][i] = v;
+    __syncthreads();
+    if (i < 624)
+      words[b * 624 + i] = v;
+  }
+}
+__global__ void __launch_bounds__(kMtTry) rng_mt_count_kernel(const RngState *st, const uint32_t *words,
+                                                              int64_t states, int32_t *cnt) {
+  const int64_t t = (int64_t)blockIdx.x * kMtTry + threadIdx.x, w = st->idx + 4 * t;
+  double x, y, r2;
+  const int got = __syncthreads_count(w + 3 < states * 624 && polar_attempt(words + w, x, y, r2));
+  if (threadIdx.x == 0)
+    cnt[blockIdx.x] = got;
+}
+__global__ void __launch_bounds__(kMtTry) rng_mt_emit_kernel(const RngState *st, const uint32_t *words,
+                                                             int64_t states, const int32_t *cnt, double *out,
+                                                             int64_t n, int64_t *last, double *saved) {
+  __shared__ int s_warp[kMtTry / 32];
+  __shared__ int64_t s_before;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t first = st->has_saved ? 1 : 0; // out[0] is the carried value
+  const int64_t need = (n - first + 1) >> 1;   // pairs
+  // accepted attempts in the blocks before this one
+  int64_t sum = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += kMtTry)
+    sum += cnt[b];
+  for (int o = 16; o > 0; o >>= 1)
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (threadIdx.x == 0)
+    s_before = 0;
+  __syncthreads();
+  if (lane == 0)
+    atomicAdd((unsigned long long *)&s_before, (unsigned long long)sum);
+  const int64_t t = (int64_t)blockIdx.x * kMtTry + threadIdx.x, w = st->idx + 4 * t;
+  double x = 0.0, y = 0.0, r2 = 0.0;
+  const bool acc = w + 3 < states * 624 && polar_attempt(words + w, x, y, r2);
+  const unsigned bal = __ballot_sync(0xffffffffu, acc);
+  if (lane == 0)
+    s_warp[wid] = __popc(bal);
+  __syncthreads();
+  int64_t before = s_before + __popc(bal & ((1u << lane) - 1u));
+  for (int v = 0; v < wid; v++)
+    before += s_warp[v];
+  if (t == 0 && first && n > 0)
+    out[0] = st->saved;
+  if (acc && before < need) {
+    const double mult = polar_scale(r2);
+    const int64_t p = first + 2 * before;
+    out[p] = __dmul_rn(y, mult);
+    if (p + 1 < n)
+      out[p + 1] = __dmul_rn(x, mult);
+    if (before == need - 1) { // the draw ends here
+      *last = w + 3;
+      saved[0] = __dmul_rn(x, mult);
+    }
+  }
+}
+__global__ void __launch_bounds__(1024) rng_mt_finish_kernel(RngState *st, const uint32_t *words, int64_t states,
+                                                             const int32_t *cnt, int blocks, double *out, int64_t n,
+                                                             const int64_t *last, const double *saved) {
+  __shared__ uint32_t ring[6 * 624];
+  __shared__ int64_t s_got;
+  const int64_t first = st->has_saved ? 1 : 0, end = *last;
+  if (threadIdx.x == 0)
+    s_got = 0;
+  __syncthreads();
+  if (end < 0) { // the states ran out before the draw ended (their number allows for that in one of 1e9 draws)
+    int64_t sum = 0;
+    for (int b = threadIdx.x; b < blocks; b += blockDim.x)
+      sum += cnt[b];
+    atomicAdd((unsigned long long *)&s_got, (unsigned long long)sum);
+  }
+  __syncthreads();
+  const int64_t b = end < 0 ? states - 1 : end / 624;
+  for (int i = threadIdx.x; i < 624; i += blockDim.x)
+    st->mt[i] = words[b * 624 + i];
+  const bool odd = ((n - first) & 1) != 0; // the last pair's second value is carried over
+  if (threadIdx.x == 0) {
+    st->idx = end < 0 ? 624 : (int32_t)(end + 1 - b * 624);
+    st->has_saved = end >= 0 && odd;
+    if (end >= 0 && odd)
+      st->saved = saved[0];
+  }
+  __threadfence_block();
+  __syncthreads();
+  if (end < 0) {
+    const int64_t pos = first + 2 * s_got;
+    block_mt_normals(st, out + pos, n - pos, ring, 6);
+  }
+}
 __global__ void rng_philox_kernel(RngState *st, double *out, int64_t n) {
   const uint64_t key = st->philox_key, base = st->philox_ctr;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -387,6 +502,8 @@ void preload_capi_kernels() {
                       (const void *)row_sort_kernel,    (const void *)row_of_kernel,
                       (const void *)gather_t_kernel,    (const void *)slice_sort_kernel,
                       (const void *)slice_fill_kernel,  (const void *)rng_mt_kernel,
+                      (const void *)rng_mt_states_kernel, (const void *)rng_mt_count_kernel,
+                      (const void *)rng_mt_emit_kernel, (const void *)rng_mt_finish_kernel,
                       (const void *)rng_philox_kernel,  (const void *)rng_philox_advance};
   for (const void *k : ks)
     preload(k);
@@ -1072,14 +1189,46 @@ int krans_rng_seed(const krans_rng *r, uint32_t *seed) {
   return KRANS_OK;
 }
 
+// Draws from here on run on all SMs; below, one block's single launch is quicker.
+static constexpr int64_t kMtLong = 8192, kMtPiece = (int64_t)1 << 22;
 int krans_rng_normal(krans_rng *r, krans_vec *out) {
   KR_CHECK_ARG(r && out, "krans_rng_normal: NULL argument");
   krans_ctx *c = r->ctx;
   if (r->mode == KRANS_RNG_PHILOX) {
     rng_philox_kernel<<<grid_for(c, out->n), 256, 0, c->stream>>>(r->d, out->d, out->n);
     rng_philox_advance<<<1, 1, 0, c->stream>>>(r->d, out->n);
+  } else if (out->n < kMtLong) {
+    rng_mt_kernel<<<1, 1024, 0, c->stream>>>(r->d, out->d, out->n);
   } else {
-    rng_mt_kernel<<<1, 256, 0, c->stream>>>(r->d, out->d, out->n);
+    // pieces, so that the words stay within the kept scratch
+    for (int64_t at = 0; at < out->n; at += kMtPiece) {
+      const int64_t n = std::min(kMtPiece, out->n - at);
+      // attempts for n / 2 accepted ones: mean n / 2 / p and six standard
+      // deviations, p = pi / 4; four words each, after the current state
+      const double need = 0.5 * (double)(n + 1), p = 0.78539816339744831;
+      const int64_t tries = (int64_t)(need / p + 6.0 * std::sqrt(need * (1.0 - p)) / p) + 8;
+      const int64_t states = (4 * tries + 623) / 624 + 1;
+      const int blocks = (int)((states * 156 + kMtTry - 1) / kMtTry);
+      Carver lay;
+      lay.take<uint32_t>(states * 624);
+      lay.take<int32_t>(blocks);
+      lay.take<int64_t>(2);
+      WsHold ws;
+      const int rc = ws_take(c, lay.off + 256, &ws, true);
+      if (rc != KRANS_OK)
+        return rc;
+      Carver cv;
+      cv.base = (char *)ws.p;
+      uint32_t *words = cv.take<uint32_t>(states * 624);
+      int32_t *cnt = cv.take<int32_t>(blocks);
+      int64_t *last = cv.take<int64_t>(2);
+      double *saved = reinterpret_cast<double *>(last + 1);
+      rng_mt_states_kernel<<<1, 640, 0, c->stream>>>(r->d, words, states, last);
+      rng_mt_count_kernel<<<blocks, kMtTry, 0, c->stream>>>(r->d, words, states, cnt);
+      rng_mt_emit_kernel<<<blocks, kMtTry, 0, c->stream>>>(r->d, words, states, cnt, out->d + at, n, last, saved);
+      rng_mt_finish_kernel<<<1, 1024, 0, c->stream>>>(r->d, words, states, cnt, blocks, out->d + at, n, last, saved);
+      ws_give(c, &ws);
+    }
   }
   KR_CUDA(cudaGetLastError());
   return KRANS_OK;

@@ -919,103 +919,106 @@ KR_DEV uint32_t mt_temper(uint32_t y) {
   return y;
 }
 
-// Block-cooperative MT19937 regeneration of 624 words: src -> dst. The
-// recurrence new[i] = f(old[i], old[i+1], new-or-old[(i+397) mod 624]) is
-// evaluated in four dependency waves ([0,227), [227,454), [454,623), 623).
-KR_DEV void mt_regen_block(const uint32_t *src, uint32_t *dst) {
-  const int t = threadIdx.x;
-  auto f = [&](int i, uint32_t a, uint32_t b, uint32_t c) {
-    const uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
-    uint32_t v = c ^ (y >> 1);
-    if (y & 1u)
-      v ^= 0x9908b0dfu;
-    dst[i] = v;
-  };
-  for (int i = t; i < 227; i += blockDim.x)
-    f(i, src[i], src[i + 1], src[i + 397]);
-  __syncthreads();
-  for (int i = 227 + t; i < 454; i += blockDim.x)
-    f(i, src[i], src[i + 1], dst[i - 227]);
-  __syncthreads();
-  for (int i = 454 + t; i < 623; i += blockDim.x)
-    f(i, src[i], src[i + 1], dst[i - 227]);
-  __syncthreads();
-  if (t == 0)
-    f(623, src[623], dst[0], dst[396]);
-  __syncthreads();
+KR_DEV uint32_t mt_twist(uint32_t a, uint32_t b) {
+  return (((a & 0x80000000u) | (b & 0x7fffffffu)) >> 1) ^ (b & 1u ? 0x9908b0dfu : 0u);
 }
+// Word i of the state that follows `src`. The recurrence new[i] = x[i + 397] ^
+// twist(old[i], old[i + 1]) reads a new word from i = 227 on; those are written
+// out in terms of old words (one twist more from 227 on, two from 454 on), so all
+// words are independent. Loads and twists that word i does not need are made on
+// some other word and dropped, so that the loads go out together.
+KR_DEV uint32_t mt_next_word(const uint32_t *src, int i) {
+  const int j = i >= 227 ? i - 227 : 0, k = i >= 454 ? i - 454 : 0;
+  const uint32_t far = src[i < 227 ? i + 397 : i < 454 ? i + 170 : i - 57];
+  const uint32_t a0 = src[i], a1 = src[i < 623 ? i + 1 : 0], b0 = src[j], b1 = src[j + 1], c0 = src[k], c1 = src[k + 1];
+  const uint32_t new0 = src[397] ^ mt_twist(src[0], src[1]); // follows the last old word
+  uint32_t v = far ^ mt_twist(a0, i < 623 ? a1 : new0);
+  v ^= i >= 227 ? mt_twist(b0, b1) : 0u;
+  v ^= i >= 454 ? mt_twist(c0, c1) : 0u;
+  return v;
+}
+// MT19937 regeneration of 624 words by a block: src -> dst, no barrier inside
+KR_DEV void mt_regen_block(const uint32_t *src, uint32_t *dst) {
+  for (int i = threadIdx.x; i < 624; i += blockDim.x)
+    dst[i] = mt_next_word(src, i);
+}
+
+// One polar attempt from four words (two 53-bit canonicals): the point (x, y)
+// and its squared radius; true if it is accepted.
+KR_DEV bool polar_attempt(const uint32_t *w, double &x, double &y, double &r2) {
+  const double a = (double)mt_temper(w[0]), b = (double)mt_temper(w[1]);
+  const double c = (double)mt_temper(w[2]), d = (double)mt_temper(w[3]);
+  double u1 = __dadd_rn(a, __dmul_rn(b, 4294967296.0)) * 0x1p-64;
+  double u2 = __dadd_rn(c, __dmul_rn(d, 4294967296.0)) * 0x1p-64;
+  if (u1 >= 1.0)
+    u1 = 0x1.fffffffffffffp-1;
+  if (u2 >= 1.0)
+    u2 = 0x1.fffffffffffffp-1;
+  x = __dadd_rn(__dmul_rn(2.0, u1), -1.0);
+  y = __dadd_rn(__dmul_rn(2.0, u2), -1.0);
+  r2 = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
+  return !(r2 > 1.0 || r2 == 0.0);
+}
+// an accepted point's scale: the normals are y times it, then x times it
+KR_DEV double polar_scale(double r2) { return sqrt(-2.0 * log(r2) / r2); }
 
 // One block draws the next n normals of an MT19937 + polar stream, exactly
 // as std::normal_distribution<double> consumes std::mt19937 in libstdc++:
 // each polar attempt takes four 32-bit words (two 53-bit canonicals); an
 // accepted attempt yields y*m then x*m, and an unused x*m is carried over.
-// Needs blockDim.x >= 160.
-KR_DEV void block_mt_normals(RngState *st, double *out, int64_t n) {
-  __shared__ uint32_t smt[2][624];
-  __shared__ int s_wsum[8];
+// `ring` holds nblk states of 624 words in shared memory; a round generates
+// them one after the other and takes one attempt per thread from all of them
+// (needs blockDim.x >= 156 nblk). Bound by the barriers between dependent
+// states and by one SM's FP64 rate in log and square root.
+KR_DEV void block_mt_normals(RngState *st, double *out, int64_t n, uint32_t *ring, int nblk) {
+  __shared__ int s_wsum[KR_MAX_WARPS];
   __shared__ int s_last;
   __shared__ double s_saved;
   __shared__ int s_has_saved;
-  int cur = 0;
-  for (int i = threadIdx.x; i < 624; i += blockDim.x)
-    smt[0][i] = st->mt[i];
-  int idx = st->idx;
-  if (threadIdx.x == 0) {
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = (blockDim.x + 31) >> 5;
+  for (int i = t; i < 624; i += blockDim.x)
+    ring[i] = st->mt[i];
+  int idx = st->idx; // first unused word of the ring
+  if (t == 0) {
     s_has_saved = st->has_saved;
     s_saved = st->saved;
+    s_last = -1;
   }
   __syncthreads();
   int64_t pos = 0;
   if (n > 0 && s_has_saved) {
-    if (threadIdx.x == 0)
+    if (t == 0)
       out[0] = s_saved;
     pos = 1;
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (t == 0)
       s_has_saved = 0;
   }
   __syncthreads();
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  while (pos < n) {
-    if (idx >= 624) {
-      mt_regen_block(smt[cur], smt[cur ^ 1]);
-      cur ^= 1;
+  for (bool first = true; pos < n; first = false) {
+    // the states after the last one; it becomes the first of the ring
+    if (!first) {
+      mt_regen_block(ring + (nblk - 1) * 624, ring);
       idx = 0;
+      __syncthreads();
     }
-    const int navail = (624 - idx) >> 2;
-    bool acc = false;
+    for (int b = 1; b < nblk; b++) {
+      mt_regen_block(ring + (b - 1) * 624, ring + b * 624);
+      __syncthreads();
+    }
+    const int navail = (nblk * 624 - idx) >> 2;
     double x = 0.0, y = 0.0, r2 = 0.0;
-    if (t < navail) {
-      const uint32_t *w = smt[cur] + idx + 4 * t;
-      const double a = (double)mt_temper(w[0]), b = (double)mt_temper(w[1]);
-      const double c = (double)mt_temper(w[2]), d = (double)mt_temper(w[3]);
-      double u1 = __dadd_rn(a, __dmul_rn(b, 4294967296.0)) * 0x1p-64;
-      double u2 = __dadd_rn(c, __dmul_rn(d, 4294967296.0)) * 0x1p-64;
-      if (u1 >= 1.0)
-        u1 = 0x1.fffffffffffffp-1;
-      if (u2 >= 1.0)
-        u2 = 0x1.fffffffffffffp-1;
-      x = __dadd_rn(__dmul_rn(2.0, u1), -1.0);
-      y = __dadd_rn(__dmul_rn(2.0, u2), -1.0);
-      r2 = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
-      acc = !(r2 > 1.0 || r2 == 0.0);
-    }
+    const bool acc = t < navail && polar_attempt(ring + idx + 4 * t, x, y, r2);
     const unsigned bal = __ballot_sync(0xffffffffu, acc);
-    if (lane == 0 && wid < 8)
+    if (lane == 0)
       s_wsum[wid] = __popc(bal);
-    if (t == 0)
-      s_last = -1;
     __syncthreads();
-    int before = __popc(bal & ((1u << lane) - 1u));
-    int total = 0;
-    for (int w = 0; w < 5; w++) {
-      if (w < wid)
-        before += s_wsum[w];
-      total += s_wsum[w];
-    }
+    const int mine = lane < nw ? s_wsum[lane] : 0;
+    const int before = __reduce_add_sync(0xffffffffu, lane < wid ? mine : 0) + __popc(bal & ((1u << lane) - 1u));
+    const int total = __reduce_add_sync(0xffffffffu, mine);
     const int64_t need = (n - pos + 1) >> 1; // pairs still needed
     if (acc && before < need) {
-      const double mult = sqrt(-2.0 * log(r2) / r2);
+      const double mult = polar_scale(r2);
       const int64_t p = pos + 2 * (int64_t)before;
       out[p] = __dmul_rn(y, mult);
       if (p + 1 < n) {
@@ -1032,15 +1035,17 @@ KR_DEV void block_mt_normals(RngState *st, double *out, int64_t n) {
       idx += 4 * (s_last + 1);
       pos = n;
     } else {
-      idx += 4 * navail;
+      idx = nblk * 624;
       pos += 2 * (int64_t)total;
     }
-    __syncthreads();
   }
-  for (int i = threadIdx.x; i < 624; i += blockDim.x)
-    st->mt[i] = smt[cur][i];
-  if (threadIdx.x == 0) {
-    st->idx = idx;
+  // the state that holds the last used word (an exhausted state stays, as the
+  // next draw regenerates it), and the next word in it
+  const int last = idx > 624 ? (idx - 1) / 624 : 0;
+  for (int i = t; i < 624; i += blockDim.x)
+    st->mt[i] = ring[last * 624 + i];
+  if (t == 0) {
+    st->idx = idx - last * 624;
     st->has_saved = s_has_saved;
     st->saved = s_saved;
   }
@@ -1085,8 +1090,10 @@ template <class Team> KR_DEV void team_random_normal(Team &tm, RngState *st, dou
       st->philox_ctr = base + (uint64_t)n;
     tm.publish();
   } else {
+    // the ring takes the space of team_multidot's partials (3 states on 512 threads)
+    static_assert(sizeof(TeamShared::dots) >= 3 * 624 * 4, "ring of MT19937 states");
     if (tm.lead_cta())
-      block_mt_normals(st, out, n);
+      block_mt_normals(st, out, n, reinterpret_cast<uint32_t *>(tm.sh->dots), 3);
     tm.publish();
   }
 }
