@@ -9,8 +9,8 @@
 //    ordering (all disjoint rotations of a round applied at once);
 //  - Householder tridiagonalisation + implicit QL for symmetric matrices;
 //  - Cholesky and a triangular inverse.
-// Orders up to 32 run on warp 0 with warp barriers (block barriers dominate
-// such tiny problems); larger ones use the whole block.
+// Tiny orders run on warp 0 with warp barriers (block barriers dominate there);
+// larger ones use the whole block.
 // Matrices are column-major in global memory owned by the solve.
 #pragma once
 
@@ -242,37 +242,174 @@ KR_DEV double blk_allsum(double v, double *red) {
 }
 
 #define KR_EIG_MAX 512
+#define KR_EIG_WARP 4 // pencils up to this order stay on one warp
 
-// Thread groups of the eigensolver: the whole block, or warp 0 alone (small
+// Thread groups of the eigensolver: the whole block, or warp 0 alone (tiny
 // pencils, where block barriers dominate: the same steps with warp barriers).
 struct EigBlock {
+  static constexpr bool kTwoRoles = true; // warp 0 runs the recurrence, the others apply the rotations
   KR_DEV static int tid() { return threadIdx.x; }
   KR_DEV static int size() { return blockDim.x; }
   KR_DEV static void sync() { __syncthreads(); }
   KR_DEV static double allsum(double v, double *red) { return blk_allsum(v, red); }
 };
 struct EigWarp { // called by warp 0 only
+  static constexpr bool kTwoRoles = false;
   KR_DEV static int tid() { return threadIdx.x & 31; }
   KR_DEV static int size() { return 32; }
   KR_DEV static void sync() { __syncwarp(); }
   KR_DEV static double allsum(double v, double *) { return warp_sum(v); }
 };
 
+// r = sqrt(f^2 + g^2), cs = g / r, sn = f / r (cs, sn unchanged when r = 0).
+// One reciprocal square root and three products, where f^2 + g^2 is far from
+// over- and underflow, instead of a hypot and two divisions: this is the serial
+// chain of the QL sweeps. Each result is within 2 ulp.
+KR_DEV double rotation(double f, double g, double &cs, double &sn) {
+  const double r2 = fma(f, f, g * g);
+  if (r2 > 1e-280 && r2 < 1e280) {
+    const double inv = rsqrt(r2);
+    sn = f * inv;
+    cs = g * inv;
+    return r2 * inv;
+  }
+  const double r = hypot(f, g);
+  if (r != 0.0) {
+    sn = f / r;
+    cs = g / r;
+  }
+  return r;
+}
+
+// One sweep's rotations of sym_eig_ql: rotation i (m > i >= lo) mixes columns i
+// and i + 1; m = lo: nothing to apply.
+struct QlSweep {
+  int m, lo;
+  int state; // 0: go on, 1: all eigenvalues found, 2: an eigenvalue needed more than 60 sweeps
+};
+
+// The next sweep of implicit QL on (d, e), by one warp: finds the block to work
+// on (all lanes), runs the sweep (lane 0) and stores its rotations in c, s. l and
+// iter carry the eigenvalue sought and its sweeps so far.
+KR_DEV QlSweep ql_sweep(int n, double tn, double *d, double *e, double *c, double *s, int &l, int &iter) {
+  const int lane = threadIdx.x & 31;
+  for (; l < n; l++, iter = 0) {
+    int m = n - 1; // first negligible e from l on
+    for (int base = l; base < n - 1; base += 32) {
+      const int i = base + lane;
+      bool small = false;
+      if (i < n - 1) {
+        const double dd = fabs(d[i]) + fabs(d[i + 1]), ei = fabs(e[i]);
+        small = ei <= 2.2204460492503131e-16 * dd || ei <= 2.2204460492503131e-16 * tn;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, small);
+      if (hit) {
+        m = base + __ffs(hit) - 1;
+        break;
+      }
+    }
+    if (m == l)
+      continue;
+    if (iter >= 60)
+      return QlSweep{l, l, 2};
+    int lo = l;
+    if (lane == 0) {
+      double cs = 1.0, sn = 1.0, pp = 0.0, ei = e[m - 1], di1 = d[m], di = d[m - 1];
+      double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
+      g = di1 - d[l] + e[l] / (g + copysign(hypot(g, 1.0), g));
+      bool early = false;
+      for (int i = m - 1; i >= l; i--) {
+        // the next step's entries, before this step's stores
+        const double en = i > l ? e[i - 1] : 0.0, dn = i > l ? d[i - 1] : 0.0;
+        const double f = sn * ei, b = cs * ei;
+        double r = rotation(f, g, cs, sn);
+        e[i + 1] = r;
+        if (r == 0.0) {
+          d[i + 1] = di1 - pp;
+          e[m] = 0.0;
+          lo = i + 1;
+          early = true;
+          break;
+        }
+        g = di1 - pp;
+        r = (di - g) * sn + 2.0 * cs * b;
+        pp = sn * r;
+        d[i + 1] = g + pp;
+        g = cs * r - b;
+        c[i] = cs;
+        s[i] = sn;
+        ei = en;
+        di1 = di;
+        di = dn;
+      }
+      if (!early) {
+        d[l] -= pp;
+        e[l] = g;
+        e[m] = 0.0;
+      }
+    }
+    lo = __shfl_sync(0xffffffffu, lo, 0);
+    __syncwarp();
+    iter++;
+    return QlSweep{m, lo, 0};
+  }
+  return QlSweep{0, 0, 1};
+}
+
+// The rotations of a sweep applied to the rows tid, tid + bd, ... of Z. Eight
+// columns are loaded ahead at a time (each is read before the rotation that
+// overwrites it, as in the plain loop, so the values are the same) to keep
+// eight loads in flight per row.
+KR_DEV void ql_apply(int n, const QlSweep &q, const double *c, const double *s, double *Z, int tid, int bd) {
+  const int m = q.m, lo = q.lo;
+  if (m == lo)
+    return;
+  for (int row = tid; row < n; row += bd) {
+    double xr = Z[row + (size_t)m * n];
+    int i0 = m - 1;
+    for (; i0 - 7 >= lo; i0 -= 8) {
+      double zi[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        zi[u] = Z[row + (size_t)(i0 - u) * n];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int i = i0 - u;
+        const double cs = c[i], sn = s[i];
+        Z[row + (size_t)(i + 1) * n] = sn * zi[u] + cs * xr;
+        xr = cs * zi[u] - sn * xr;
+      }
+    }
+    for (int i = i0; i >= lo; i--) {
+      const double zi = Z[row + (size_t)i * n];
+      const double cs = c[i], sn = s[i];
+      Z[row + (size_t)(i + 1) * n] = sn * zi + cs * xr;
+      xr = cs * zi - sn * xr;
+    }
+    Z[row + (size_t)lo * n] = xr;
+  }
+}
+
 // Symmetric eigendecomposition of A (n x n, column-major, ld n; both
 // triangles referenced, destroyed) on a thread group: Householder reduction
 // to tridiagonal form with the orthogonal factor accumulated explicitly, then
 // the implicit QL algorithm with shifts for the tridiagonal matrix (Golub &
 // Van Loan, Matrix Computations, 4th ed., 8.3.1 and 8.3.3; QL as in Bowdler,
-// Martin, Reinsch and Wilkinson, Numer. Math. 11 (1968) 293-306). One thread
+// Martin, Reinsch and Wilkinson, Numer. Math. 11 (1968) 293-306). One lane
 // runs the scalar recurrence of each QL sweep into shared arrays of rotations;
-// all threads then apply the sweep to the rows of Z in parallel (the rows are
-// independent). w ascending (ties keep index order), Z columns = eigenvectors.
-// Returns 0, or nonzero if n > KR_EIG_MAX or an eigenvalue needed more than 60
-// sweeps (the caller then falls back to Jacobi).
-template <class G, int NMAX> KR_DEV int sym_eig_ql(int n, double *A, double *w, double *Z, int *ord) {
-  __shared__ double s_d[NMAX], s_e[NMAX], s_c[NMAX], s_s[NMAX];
+// the rows of Z take them in parallel (the rows are independent). A block runs
+// the two side by side: warp 0 is a sweep ahead, the other warps apply the one
+// before (the recurrence does not read Z).
+// w ascending (ties keep index order), Z columns = eigenvectors. Returns 0, or
+// nonzero if n > KR_EIG_MAX or an eigenvalue needed more than 60 sweeps (the
+// caller then falls back to Jacobi).
+template <class G, int NMAX> KR_DEV int sym_eig_ql(int n, double *A, double *w, double *Z, int *ord,
+                                                       double *tri) {
+  __shared__ double s_cs[2][2][NMAX]; // rotations of two sweeps
+  double *const s_d = tri, *const s_e = tri + NMAX; // the tridiagonal matrix
+  double *const s_c = s_cs[0][0], *const s_s = s_cs[0][1];
   __shared__ double s_red[KR_MAX_WARPS];
-  __shared__ int s_m, s_lo, s_fail;
+  __shared__ QlSweep s_sweep[2];
   __shared__ double s_tn;
   const int tid = G::tid(), bd = G::size(), lane = tid & 31, wid = tid >> 5, nw = bd >> 5;
   if (n > NMAX || n < 1)
@@ -340,7 +477,6 @@ template <class G, int NMAX> KR_DEV int sym_eig_ql(int n, double *A, double *w, 
     }
     s_d[n - 1] = A[(n - 1) + (size_t)(n - 1) * n];
     s_e[n - 1] = 0.0;
-    s_fail = 0;
     double tn = 0.0; // ||T||_inf: the deflation floor eps ||T|| (absolute accuracy)
     for (int i = 0; i < n; i++)
       tn = fmax(tn, fabs(s_d[i]) + fabs(s_e[i]) + (i ? fabs(s_e[i - 1]) : 0.0));
@@ -368,96 +504,34 @@ template <class G, int NMAX> KR_DEV int sym_eig_ql(int n, double *A, double *w, 
     G::sync();
   }
   // ---- 3) implicit QL on (d, e), rotations applied to the rows of Z
-  for (int l = 0; l < n; l++) {
-    for (int iter = 0;; iter++) {
-      if (tid == 0) {
-        int m = l;
-        for (; m < n - 1; m++) {
-          const double dd = fabs(s_d[m]) + fabs(s_d[m + 1]);
-          if (fabs(s_e[m]) <= 2.2204460492503131e-16 * dd || fabs(s_e[m]) <= 2.2204460492503131e-16 * s_tn)
-            break;
-        }
-        s_m = m;
-        s_lo = m;
-        if (m != l) {
-          if (iter >= 60) {
-            s_fail = 1;
-          } else {
-            double g = (s_d[l + 1] - s_d[l]) / (2.0 * s_e[l]);
-            double r = hypot(g, 1.0);
-            g = s_d[m] - s_d[l] + s_e[l] / (g + copysign(r, g));
-            double sn = 1.0, cs = 1.0, pp = 0.0;
-            int i = m - 1;
-            bool early = false;
-            for (; i >= l; i--) {
-              const double f = sn * s_e[i], b = cs * s_e[i];
-              r = hypot(f, g);
-              s_e[i + 1] = r;
-              if (r == 0.0) {
-                s_d[i + 1] -= pp;
-                s_e[m] = 0.0;
-                early = true;
-                break;
-              }
-              sn = f / r;
-              cs = g / r;
-              g = s_d[i + 1] - pp;
-              r = (s_d[i] - g) * sn + 2.0 * cs * b;
-              pp = sn * r;
-              s_d[i + 1] = g + pp;
-              g = cs * r - b;
-              s_c[i] = cs;
-              s_s[i] = sn;
-            }
-            s_lo = early ? i + 1 : l;
-            if (!early) {
-              s_d[l] -= pp;
-              s_e[l] = g;
-              s_e[m] = 0.0;
-            }
-          }
-        }
+  int l = 0, iter = 0, fail = 0;
+  if constexpr (G::kTwoRoles) {
+    // step k: warp 0 computes sweep k, the other warps apply sweep k - 1
+    for (int k = 0;; k++) {
+      if (wid == 0) {
+        const QlSweep q = ql_sweep(n, s_tn, s_d, s_e, s_cs[k & 1][0], s_cs[k & 1][1], l, iter);
+        if (lane == 0)
+          s_sweep[k & 1] = q;
+      } else if (k > 0) {
+        ql_apply(n, s_sweep[(k - 1) & 1], s_cs[(k - 1) & 1][0], s_cs[(k - 1) & 1][1], Z, tid - 32, bd - 32);
       }
       G::sync();
-      const int m = s_m, lo = s_lo, fl = s_fail;
-      G::sync(); // all have read before thread 0 writes the next sweep
-      if (m == l || fl)
+      const int state = s_sweep[k & 1].state; // rewritten two steps on, behind the next barrier
+      if (state) {
+        fail = state == 2;
         break;
-      // rotation i mixes columns i and i+1 of every row, for i = m-1 down to
-      // lo; eight columns are loaded ahead at a time (each is read before the
-      // rotation that overwrites it, as in the plain loop, so the values are
-      // the same) to keep eight loads in flight per row
-      for (int row = tid; row < n; row += bd) {
-        double xr = Z[row + (size_t)m * n];
-        int i0 = m - 1;
-        for (; i0 - 7 >= lo; i0 -= 8) {
-          double zi[8];
-#pragma unroll
-          for (int u = 0; u < 8; u++)
-            zi[u] = Z[row + (size_t)(i0 - u) * n];
-#pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const int i = i0 - u;
-            const double cs = s_c[i], sn = s_s[i];
-            Z[row + (size_t)(i + 1) * n] = sn * zi[u] + cs * xr;
-            xr = cs * zi[u] - sn * xr;
-          }
-        }
-        for (int i = i0; i >= lo; i--) {
-          const double zi = Z[row + (size_t)i * n];
-          const double cs = s_c[i], sn = s_s[i];
-          Z[row + (size_t)(i + 1) * n] = sn * zi + cs * xr;
-          xr = cs * zi - sn * xr;
-        }
-        Z[row + (size_t)lo * n] = xr;
       }
+    }
+  } else {
+    for (;;) {
+      const QlSweep q = ql_sweep(n, s_tn, s_d, s_e, s_c, s_s, l, iter);
+      fail = q.state == 2;
+      if (q.state)
+        break;
+      ql_apply(n, q, s_c, s_s, Z, tid, bd);
       G::sync();
     }
-    if (s_fail)
-      break;
-    G::sync();
   }
-  const int fail = s_fail;
   G::sync();
   if (fail)
     return 1;
@@ -486,13 +560,17 @@ template <class G, int NMAX> KR_DEV int sym_eig_ql(int n, double *A, double *w, 
   return 0;
 }
 
-// The block's entry: warp 0 alone for n <= 32, else the whole block. Every
-// thread of the block calls it and gets the same return value.
-KR_DEV int block_sym_eig_ql(int n, double *A, double *w, double *Z, int *ord) {
-  if (n <= 32) {
+// The block's entry: warp 0 alone for n <= KR_EIG_WARP, else the whole block (from
+// n = 6 on the second role pays for the block barriers: n = 12 takes 73 us on the
+// block and 108 on one warp, n = 30 294 and 564; a block that only took turns
+// needed 881 us at n = 36 and 52.5 ms at n = 288, and needs 398 us and 24.8 ms). Every
+// thread of the block calls it and gets the same return value. `tri` is shared
+// memory for 2 KR_EIG_MAX doubles.
+KR_DEV int block_sym_eig_ql(int n, double *A, double *w, double *Z, int *ord, double *tri) {
+  if (n <= KR_EIG_WARP) {
     __shared__ int s_rc;
     if (threadIdx.x < 32) {
-      const int rc = sym_eig_ql<EigWarp, 32>(n, A, w, Z, ord);
+      const int rc = sym_eig_ql<EigWarp, KR_EIG_WARP>(n, A, w, Z, ord, tri);
       if (threadIdx.x == 0)
         s_rc = rc;
     }
@@ -501,7 +579,7 @@ KR_DEV int block_sym_eig_ql(int n, double *A, double *w, double *Z, int *ord) {
     __syncthreads();
     return rc;
   }
-  return sym_eig_ql<EigBlock, KR_EIG_MAX>(n, A, w, Z, ord);
+  return sym_eig_ql<EigBlock, KR_EIG_MAX>(n, A, w, Z, ord, tri);
 }
 
 // In-place Cholesky of the lower triangle of A (n x n, ld n). Returns 0 on

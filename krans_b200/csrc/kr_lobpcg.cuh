@@ -575,7 +575,8 @@ template <class Team> struct LobpcgSolver {
     for (int e = threadIdx.x; e < p * p; e += blockDim.x)
       d.Tm[e] = d.Cm[e];
     __syncthreads();
-    if (block_sym_eig_ql(p, d.Tm, d.th, d.Q, d.eig_ord) != 0)
+    static_assert(sizeof(TeamShared::dots) >= 2 * KR_EIG_MAX * 8, "tridiagonal matrix of the eigensolver");
+    if (block_sym_eig_ql(p, d.Tm, d.th, d.Q, d.eig_ord, tm.sh->dots) != 0)
       block_jacobi_eig(p, d.Cm, d.th, d.Q, d.eig_cs, d.eig_pq, d.eig_ord);
     __shared__ int s_bad;
     if (threadIdx.x == 0)
