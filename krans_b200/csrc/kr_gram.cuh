@@ -1,8 +1,8 @@
 // Tall-skinny products of the block solver, on the FP64 tensor cores:
 //   team_tn_panels:     S = Z^T Z with G = Z^T (AZ), or C = A^T B: shared-memory
 //                       panels, for long, wide blocks
-//   team_gemm_tn_direct, team_gram2_direct: the same for short or narrow
-//                       blocks, one warp per output tile
+//   team_tn_direct:     the same for short or narrow blocks, one warp per output
+//                       tile
 //   team_gemm_nn:       out (-)= Z * Y[roff:roff+zc, 0:q] (n x q), shared-memory
 //                       chunks (team_combine, team_combine_sub)
 // Sums run in a fixed order that depends only on the team size, so results
@@ -20,140 +20,180 @@ KR_DEV void dmma_8x8x4(double &d0, double &d1, double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// C = A^T B for tall-skinny A (n x a) and B (n x b), column-major with
-// leading dim ld; C is a x b with leading dim a. DMMA 8x8 tiles, one warp per
-// tile; each block reduces its fixed row range into a private partial, then
-// the partials are summed in block order (deterministic for a team size).
-template <class Team>
-KR_DEV void team_gemm_tn_direct(Team &tm, int64_t n, const double *A, int a, const double *B, int b, int64_t ld,
-                         double *C, double *part) {
-  const int ta = (a + 7) / 8, tb = (b + 7) / 8, ntiles = ta * tb;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int ncta = tm.ncta(), rank = tm.cta_rank();
-  const int64_t per = (n + ncta - 1) / ncta;
-  const int64_t r0 = imin64((int64_t)rank * per, n), r1 = imin64(r0 + per, n);
-  double *my = part + (size_t)rank * a * b;
-  for (int t = wid; t < ntiles; t += nw) {
-    const int bi = t % ta, bj = t / ta;
-    const int ia = bi * 8 + (lane >> 2), jb = bj * 8 + (lane >> 2);
-    const bool va = ia < a, vb = jb < b;
-    const double *pa = A + (int64_t)(va ? ia : 0) * ld;
-    const double *pb = B + (int64_t)(vb ? jb : 0) * ld;
-    double c0 = 0.0, c1 = 0.0, e0 = 0.0, e1 = 0.0;
-    int64_t base = r0;
-    for (; base + 8 <= r1; base += 8) { // two independent accumulators
-      const int64_t r = base + (lane & 3);
-      const double x0 = va ? pa[r] : 0.0, y0 = vb ? pb[r] : 0.0;
-      const double x1 = va ? pa[r + 4] : 0.0, y1 = vb ? pb[r + 4] : 0.0;
-      dmma_8x8x4(c0, c1, x0, y0);
-      dmma_8x8x4(e0, e1, x1, y1);
+// f(e, sum over the team's blocks of part[rank * stride + e]) for e < count,
+// with two sums when `two` (the second at offset `second`). Few blocks: a thread
+// per element, blocks in order. Many: a warp per element, each lane over its
+// share of the blocks and a butterfly (one thread summing 148 partials waits
+// out 148 loads).
+template <class Team, class F>
+KR_DEV void team_sum_ranks(Team &tm, int64_t count, const double *part, size_t stride, size_t second, F f) {
+  const int ncta = tm.ncta();
+  if (ncta < 32) {
+    for (int64_t e = tm.tid(); e < count; e += tm.nthreads()) {
+      double s = 0.0, g = 0.0;
+      for (int r = 0; r < ncta; r++) {
+        s += __ldcg(part + (size_t)r * stride + e);
+        if (second)
+          g += __ldcg(part + (size_t)r * stride + second + e);
+      }
+      f(e, s, g);
     }
-    for (; base < r1; base += 4) {
-      const int64_t r = base + (lane & 3);
-      const bool in = r < r1;
-      const double x0 = (in && va) ? pa[r] : 0.0, y0 = (in && vb) ? pb[r] : 0.0;
-      dmma_8x8x4(c0, c1, x0, y0);
-    }
-    c0 += e0;
-    c1 += e1;
-    const int ci = bi * 8 + (lane >> 2), cj = bj * 8 + 2 * (lane & 3);
-    if (ci < a) {
-      if (cj < b)
-        my[ci + (size_t)cj * a] = c0;
-      if (cj + 1 < b)
-        my[ci + (size_t)(cj + 1) * a] = c1;
-    }
+    return;
   }
-  tm.sync();
-  const int64_t nt = tm.nthreads();
-  for (int64_t e = tm.tid(); e < (int64_t)a * b; e += nt) {
-    double s = 0.0;
-    for (int r = 0; r < ncta; r++)
-      s += __ldcg(part + (size_t)r * a * b + e);
-    C[e] = s;
+  const int lane = threadIdx.x & 31;
+  for (int64_t e = tm.warp_id(); e < count; e += tm.nwarps()) {
+    double s = 0.0, g = 0.0;
+    for (int r = lane; r < ncta; r += 32) {
+      s += __ldcg(part + (size_t)r * stride + e);
+      if (second)
+        g += __ldcg(part + (size_t)r * stride + second + e);
+    }
+    s = warp_sum(s);
+    if (second)
+      g = warp_sum(g);
+    if (lane == 0)
+      f(e, s, g);
   }
-  tm.sync();
 }
 
+// Rows [r0, r1) of an 8 x 8 tile of X^T Y (and of X^T W when TWO) by one warp,
+// operands straight from global memory; xa, yb, wb: this lane's column, or
+// nullptr past the last one. Four steps of four rows are loaded together. The
+// MMA lane layout of m8n8k4: A(row = lane >> 2, k = lane & 3), B(k = lane & 3,
+// col = lane >> 2), C rows lane >> 2, columns 2 (lane & 3) and the next.
+template <bool TWO>
+KR_DEV void warp_tn_tile(int64_t r0, int64_t r1, const double *xa, const double *yb, const double *wb, double (&s)[2],
+                         double (&g)[2]) {
+  constexpr int U = 4;
+  const int k = threadIdx.x & 3;
+  double cs[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, cg[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  for (int64_t base = r0; base < r1; base += 4 * U) { // warp-uniform trip count
+    double x[U], y[U], w[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int64_t r = base + 4 * u + k;
+      const bool in = r < r1;
+      x[u] = in && xa ? xa[r] : 0.0;
+      y[u] = in && yb ? yb[r] : 0.0;
+      if constexpr (TWO)
+        w[u] = in && wb ? wb[r] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      dmma_8x8x4(cs[u & 1][0], cs[u & 1][1], x[u], y[u]);
+      if constexpr (TWO)
+        dmma_8x8x4(cg[u & 1][0], cg[u & 1][1], x[u], w[u]);
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    s[h] = cs[0][h] + cs[1][h];
+    g[h] = cg[0][h] + cg[1][h];
+  }
+}
 
-// S = Z^T Z and G = Z^T (AZ) (p x p) in one pass, one warp per 8x8 upper
-// tile with DMMA, operands straight from global memory; each block reduces
-// its fixed row range into a private partial (2 p^2 doubles per block in
-// `part`), summed in block order. Like the reference's form_gram
-// (LOBPCGSolver.cpp:67-80), which sets S(i,j) = S(j,i) = Z_i.Z_j and
-// G(i,j) = G(j,i) = Z_i.(AZ)_j for i <= j, only the upper triangles are
-// formed and then mirrored. Used for short or narrow blocks.
-template <class Team>
-KR_DEV void team_gram2_direct(Team &tm, int64_t n, const double *Z, const double *AZ, int64_t ld, int p,
-                       double *S, double *G, double *part) {
-  const int nt8 = (p + 7) / 8;                       // 8x8 tiles per dimension
-  const int ntiles = nt8 * (nt8 + 1) / 2;            // upper triangle incl. diagonal
+// The direct forms, for short or narrow blocks: each block reduces its fixed
+// row range into a private partial, 8 x 8 tiles by warps; with fewer tiles than
+// warps the rows are split among the warps too, whose pieces are added in order
+// in shared memory. The blocks' partials are summed in a fixed order. Bound by the
+// latency of dependent steps of 4 to 16 rows (a block of 148 has 338 of 50021
+// rows); the Gram pairs of that LOBPCG solve (36 and 12 columns) took 9.8 ms in
+// all and take 4.5, its orthonormalisations 53 and 41 ms.
+//   SYM: S = Z^T Z and G = Z^T W (p x p): like the reference's form_gram
+//        (LOBPCGSolver.cpp:67-80), which sets S(i,j) = S(j,i) = Z_i.Z_j and
+//        G(i,j) = G(j,i) = Z_i.(AZ)_j for i <= j, only the upper triangles are
+//        formed and then mirrored; `part` holds 2 p^2 doubles a block
+//   else: S = Z^T W (p x q); p q doubles a block
+template <bool SYM, class Team>
+KR_DEV void team_tn_direct(Team &tm, int64_t n, const double *Z, int p, const double *W, int q, int64_t ld, double *S,
+                           double *G, double *part) {
+  constexpr int TILE = SYM ? 128 : 64; // doubles of a tile's piece
+  const int tp = (p + 7) / 8, tq = (q + 7) / 8, ntiles = SYM ? tp * (tp + 1) / 2 : tp * tq;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int ncta = tm.ncta(), rank = tm.cta_rank();
-  // fixed row range of this block
   const int64_t per = (n + ncta - 1) / ncta;
   const int64_t r0 = imin64((int64_t)rank * per, n), r1 = imin64(r0 + per, n);
-  double *myS = part + (size_t)rank * 2 * p * p;
-  double *myG = myS + (size_t)p * p;
-  // a warp owns one 8x8 tile at a time; the MMA lane layout of m8n8k4:
-  // A(row=lane>>2, k=lane&3), B(k=lane&3, col=lane>>2), C rows lane>>2,
-  // cols 2*(lane&3) and 2*(lane&3)+1.
-  for (int t = wid; t < ntiles; t += nw) {
-    // decode upper-triangular tile index t -> (bi <= bj)
-    int bi = 0, rem = t;
-    while (rem >= nt8 - bi) {
-      rem -= nt8 - bi;
-      bi++;
-    }
-    const int bj = bi + rem;
-    const int ia = bi * 8 + (lane >> 2), jb = bj * 8 + (lane >> 2);
-    const bool va = ia < p, vb = jb < p;
-    const double *za = Z + (int64_t)(va ? ia : 0) * ld;
-    const double *zb = Z + (int64_t)(vb ? jb : 0) * ld;
-    const double *azb = AZ + (int64_t)(vb ? jb : 0) * ld;
-    double s0 = 0.0, s1 = 0.0, g0 = 0.0, g1 = 0.0;
-    for (int64_t base = r0; base < r1; base += 4) { // warp-uniform trip count
-      const int64_t r = base + (lane & 3);
-      const bool in = r < r1;
-      const double a = (in && va) ? za[r] : 0.0;
-      const double b = (in && vb) ? zb[r] : 0.0;
-      const double ab = (in && vb) ? azb[r] : 0.0;
-      dmma_8x8x4(s0, s1, a, b);
-      dmma_8x8x4(g0, g1, a, ab);
-    }
-    const int ci = bi * 8 + (lane >> 2), cj = bj * 8 + 2 * (lane & 3);
-    if (ci < p) {
-      if (cj < p) {
-        myS[ci + (size_t)cj * p] = s0;
-        myG[ci + (size_t)cj * p] = g0;
+  const size_t stride = (SYM ? 2 : 1) * (size_t)p * q;
+  double *my = part + (size_t)rank * stride;
+  double *pieces = tm.sh->dots; // (slab, tile) pieces, ntiles nslab <= pieces that fit
+  constexpr int fit = KR_MDOT * KR_RED_LD / TILE;
+  const int nslab = max(1, min(nw, fit) / ntiles);
+  const int64_t slab_rows = kr_round_up((r1 - r0 + nslab - 1) / nslab, 16);
+  for (int t = wid; t < ntiles * nslab; t += nw) {
+    const int tile = t % ntiles, slab = t / ntiles;
+    int bi = tile % tp, bj = tile / tp;
+    if (SYM) { // upper-triangular tile index -> bi <= bj
+      bi = 0;
+      int rem = tile;
+      while (rem >= tp - bi) {
+        rem -= tp - bi;
+        bi++;
       }
-      if (cj + 1 < p) {
-        myS[ci + (size_t)(cj + 1) * p] = s1;
-        myG[ci + (size_t)(cj + 1) * p] = g1;
+      bj = bi + rem;
+    }
+    const int ia = bi * 8 + (lane >> 2), jb = bj * 8 + (lane >> 2);
+    const double *xa = ia < p ? Z + (int64_t)ia * ld : nullptr;
+    const double *yb = jb < q ? (SYM ? Z : W) + (int64_t)jb * ld : nullptr;
+    const double *wb = SYM && jb < q ? W + (int64_t)jb * ld : nullptr;
+    const int64_t s0 = imin64(r0 + slab * slab_rows, r1), s1 = imin64(s0 + slab_rows, r1);
+    double s[2], g[2];
+    warp_tn_tile<SYM>(s0, s1, xa, yb, wb, s, g);
+    const int ci = lane >> 2, cj = 2 * (lane & 3);
+    if (nslab > 1) {
+      double *pc = pieces + t * TILE;
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        pc[ci + 8 * (cj + h)] = s[h];
+        if (SYM)
+          pc[64 + ci + 8 * (cj + h)] = g[h];
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int i = bi * 8 + ci, j = bj * 8 + cj + h;
+        if (i < p && j < q) {
+          my[i + (size_t)j * p] = s[h];
+          if (SYM)
+            my[(size_t)p * q + i + (size_t)j * p] = g[h];
+        }
       }
     }
   }
+  if (nslab > 1) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < p * q; e += blockDim.x) {
+      const int i = e % p, j = e / p, bi = i / 8, bj = j / 8;
+      if (SYM && bi > bj)
+        continue;
+      const int tile = SYM ? bi * tp - bi * (bi - 1) / 2 + (bj - bi) : bj * tp + bi;
+      double s = 0.0, g = 0.0;
+      for (int k = 0; k < nslab; k++) {
+        const double *pc = pieces + (k * ntiles + tile) * TILE + (i & 7) + 8 * (j & 7);
+        s += pc[0];
+        if (SYM)
+          g += pc[64];
+      }
+      my[e] = s;
+      if (SYM)
+        my[(size_t)p * q + e] = g;
+    }
+  }
   tm.sync();
-  // sum the block partials in block order; fill both triangles
-  const int64_t nt = tm.nthreads();
-  for (int64_t e = tm.tid(); e < (int64_t)p * p; e += nt) {
+  team_sum_ranks(tm, (int64_t)p * q, part, stride, SYM ? (size_t)p * q : 0, [&](int64_t e, double s, double g) {
+    if (!SYM) {
+      S[e] = s;
+      return;
+    }
     const int j = (int)(e / p), i = (int)(e % p);
     if (i > j)
-      continue;
-    double s = 0.0, g = 0.0;
-    for (int b = 0; b < ncta; b++) {
-      const double *ps = part + (size_t)b * 2 * p * p;
-      s += __ldcg(ps + e);
-      g += __ldcg(ps + (size_t)p * p + e);
-    }
+      return;
     S[i + (size_t)j * p] = s;
     S[j + (size_t)i * p] = s;
     G[i + (size_t)j * p] = g;
     G[j + (size_t)i * p] = g;
-  }
+  });
   tm.sync();
 }
-
 
 #define KR_TN_ROWS 131072 // rows from which the panel form of the A^T B products runs
 #define KR_TN_COLS 32     // and columns
@@ -363,7 +403,7 @@ KR_DEV void team_gemm_tn(Team &tm, int64_t n, const double *A, int a, const doub
   if (n >= KR_TN_ROWS && (a >= KR_TN_COLS || b >= KR_TN_COLS))
     team_tn_panels<false>(tm, n, A, a, B, b, ld, C, nullptr, part);
   else
-    team_gemm_tn_direct(tm, n, A, a, B, b, ld, C, part);
+    team_tn_direct<false>(tm, n, A, a, B, b, ld, C, nullptr, part);
 }
 
 // ---- Z * Y products (combine_columns, LOBPCGSolver.cpp:122-134) -----------

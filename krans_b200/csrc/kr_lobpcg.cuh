@@ -458,7 +458,7 @@ template <class Team> struct LobpcgSolver {
     if (n >= KR_TN_ROWS && p >= KR_TN_COLS) {
       team_tn_panels<true>(tm, n, Zb, p, AZb, p, ldn, d.S, d.G, d.gram_part); // both in one pass
     } else {
-      team_gram2_direct(tm, n, Zb, AZb, ldn, p, d.S, d.G, d.gram_part); // both in one pass
+      team_tn_direct<true>(tm, n, Zb, p, AZb, p, ldn, d.S, d.G, d.gram_part); // both in one pass
     }
     t_ph[1] += globaltimer_ns() - t0;
     gram_flops += 2.0 * 2.0 * (double)n * p * p;
