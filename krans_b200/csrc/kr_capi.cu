@@ -182,7 +182,40 @@ int pick_lanes(int64_t rows, int64_t nnz) {
   return 32;
 }
 
-// two-stage deterministic reduction: partial per block, then one block sums
+// Deterministic dot product in one launch: a partial per block, and the block
+// that finishes last sums them in index order. `out` may be pinned host memory,
+// so that a scalar the host waits for takes one launch and no copy (a caller's own
+// Golub-Kahan step of 1000 unknowns, seven scalars among its twelve calls: 157 us
+// with two launches and a copy each, 127 us so).
+__global__ void __launch_bounds__(256) dot_kernel(int64_t n, const double *x, const double *y, double *part,
+                                                  unsigned *done, double *out, int take_sqrt) {
+  __shared__ TeamShared sh;
+  __shared__ bool s_last;
+  int buf = 0;
+  double v[1] = {0.0};
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    v[0] += x[i] * y[i];
+  block_sum<1>(&sh, buf, v);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = v[0];
+    __threadfence();
+    s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last)
+    return;
+  __threadfence();
+  v[0] = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+    v[0] += __ldcg(part + i);
+  block_sum<1>(&sh, buf, v);
+  if (threadIdx.x == 0) {
+    out[0] = take_sqrt ? sqrt(v[0]) : v[0];
+    *done = 0; // for the next launch on the stream
+  }
+}
+// the same in two launches without a counter, for krans_vec_dot_noalloc: partial per block, then one block sums
 __global__ void __launch_bounds__(256) dot_partial_kernel(int64_t n, const double *x, const double *y,
                                                           double *part) {
   __shared__ TeamShared sh;
@@ -494,7 +527,8 @@ void preload(const void *kernel) {
 }
 
 void preload_capi_kernels() {
-  const void *ks[] = {(const void *)dot_partial_kernel, (const void *)sum_partials_kernel,
+  const void *ks[] = {(const void *)dot_kernel,         (const void *)dot_partial_kernel,
+                      (const void *)sum_partials_kernel,
                       (const void *)axpy_kernel,        (const void *)scale_kernel,
                       (const void *)scale_by_inv_norm_kernel, (const void *)fill_kernel,
                       (const void *)to_f32_kernel,      (const void *)col_count_kernel,
@@ -590,6 +624,8 @@ int krans_ctx_create(int device, size_t hbm_budget_bytes, krans_ctx **out) {
     e = cudaMalloc(&c->d_scalar, 64 * sizeof(double));
   if (e == cudaSuccess)
     e = cudaMalloc(&c->d_partials, (size_t)c->partial_blocks * sizeof(double));
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(c->d_scalar, 0, 64 * sizeof(double), c->stream); // scalars, and the block counter of dot_kernel
   if (e != cudaSuccess) {
     int rc = cuda_fail(e, "context setup", __FILE__, __LINE__);
     krans_ctx_destroy(c);
@@ -1023,15 +1059,17 @@ int krans_vec_download(const krans_vec *v, double *host, int64_t n) {
   return KRANS_OK;
 }
 
+static void launch_dot(krans_ctx *c, int64_t n, const double *x, const double *y, int take_sqrt, double *out) {
+  const int g = std::min<int>(grid_for(c, n), c->partial_blocks);
+  dot_kernel<<<g, 256, 0, c->stream>>>(n, x, y, c->d_partials, reinterpret_cast<unsigned *>(c->d_scalar + 1), out,
+                                       take_sqrt);
+}
 static int reduce_to_host(krans_ctx *c, int64_t n, const double *x, const double *y, int take_sqrt,
                           double *out) {
-  const int g = std::min<int>(grid_for(c, n), c->partial_blocks);
-  dot_partial_kernel<<<g, 256, 0, c->stream>>>(n, x, y, c->d_partials);
-  sum_partials_kernel<<<1, 256, 0, c->stream>>>(g, c->d_partials, c->d_scalar, take_sqrt);
+  launch_dot(c, n, x, y, take_sqrt, c->h_scalar); // pinned: the device writes it directly
   KR_CUDA(cudaGetLastError());
-  KR_CUDA(cudaMemcpyAsync(c->h_scalar, c->d_scalar, 8, cudaMemcpyDeviceToHost, c->stream));
   KR_CUDA(cudaStreamSynchronize(c->stream));
-  *out = c->h_scalar[0];
+  *out = *(volatile double *)c->h_scalar;
   return KRANS_OK;
 }
 
@@ -1064,9 +1102,7 @@ int krans_vec_scale(krans_vec *v, double alpha) {
 int krans_vec_normalize(krans_vec *v) {
   KR_CHECK_ARG(v, "NULL argument");
   krans_ctx *c = v->ctx;
-  const int g = std::min<int>(grid_for(c, v->n), c->partial_blocks);
-  dot_partial_kernel<<<g, 256, 0, c->stream>>>(v->n, v->d, v->d, c->d_partials);
-  sum_partials_kernel<<<1, 256, 0, c->stream>>>(g, c->d_partials, c->d_scalar, 1);
+  launch_dot(c, v->n, v->d, v->d, 1, c->d_scalar);
   scale_by_inv_norm_kernel<<<grid_for(c, v->n), 256, 0, c->stream>>>(v->n, c->d_scalar, v->d);
   KR_CUDA(cudaGetLastError());
   return KRANS_OK;

@@ -4,8 +4,8 @@
 // only from their own pre-planned pool and treat any other allocation as a
 // bug, and code paths that must not synchronize the device (cudaFree and, in
 // many configurations, cudaMalloc implicitly synchronize). For them this entry
-// point computes x.y with the same two reduction kernels as krans_vec_dot,
-// but takes its scratch (one partial sum per thread block) from a
+// point computes x.y with two reduction kernels in krans_vec_dot's order of
+// summation, but takes its scratch (one partial sum per thread block) from a
 // file-scope device array instead of a context allocation.
 //
 // The array is KRANS_NOALLOC_DOT_MAX_BLOCKS doubles (128 KiB) and every GPU
