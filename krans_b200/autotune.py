@@ -15,7 +15,12 @@ tune() searches them one at a time (coordinate descent, each knob over a
 short list of candidates around the built-in value, in the order above) on
 probe batches drawn from the batched workload's generator with seeds the
 benchmark does not use, keeping a candidate only when it is faster by more
-than the noise margin. The winners are written to
+than the noise margin. The probes are full batches (throughput: more work than
+teams) and, for each, a short one of a quarter of the requests and a tenth of
+the largest size, where the slowest request's team decides (a table tuned on
+full batches alone left such a batch to two-block teams while the big
+clusters idled: 835 ms, and 399 ms with a lower pair_max at the same
+throughput of full batches). The winners are written to
 krans_b200/tuning/<device>.json together with every trial; Context() applies
 the table of its device when one exists.
 
@@ -35,7 +40,7 @@ DEFAULTS = {"cluster_min": 16384, "pair_max": 120000, "cluster_size": 8, "lanes"
 CANDIDATES = [
     ("cluster_size", [8, 4]),
     ("cluster_min", [16384, 8192, 32768]),
-    ("pair_max", [120000, 60000, 250000]),
+    ("pair_max", [120000, 60000, 40000, 30000, 250000]),
     ("lanes[1]", [2, 1, 4]),   # mean row length in (3, 8]: incidence transposes (degree ~6)
     ("lanes[0]", [1, 2]),      # mean row length <= 3: shift operators, incidence rows
 ]
@@ -146,21 +151,22 @@ def tune(ctx, batch: int = 256, probes: int = 1, seed: int = 7000) -> Dict:
         return float(np.sqrt(max(A2.sum(axis=0).max(), A2.sum(axis=1).max())))
 
     sets = []
-    for b in range(probes):
-        insts = G.batch_instances(batch, seed=seed + b, kernel=False)
+    shapes = [s for b in range(probes) for s in ((batch, seed + b, 2e5), (max(1, batch // 4), seed + 500 + b, 2e4))]
+    for count, sd, n_hi in shapes:
+        insts = G.batch_instances(count, seed=sd, n_hi=n_hi, kernel=False)
         mats = [CudaCsrMatrixAdapter.from_scipy(ctx, i.A, fp32=True) for i in insts]
         opts = [CyclicLanczosOptions(k=i.k, tol_abs=1e-12 * L(i.A), tol_rel=0.0, cg_maxit=1000,
                                      precision=Precision.MIXED) for i in insts]
         sets.append((mats, opts))
 
     def evaluate(knobs):
+        # geometric mean over the probes, so that the short ones count as much as the full ones
         apply(ctx, knobs)
-        n, ms = 0, 0.0
+        logs = []
         for mats, opts in sets:
             reqs = [SolveRequest(M, o, seed=1 + j, rng_mode="philox") for j, (M, o) in enumerate(zip(mats, opts))]
-            ms += solve_batch(ctx, reqs)
-            n += len(reqs)
-        return n / (ms / 1e3)
+            logs.append(np.log(len(reqs) / (solve_batch(ctx, reqs) / 1e3)))
+        return float(np.exp(np.mean(logs)))
 
     evaluate(DEFAULTS)  # warm-up (module load, first touch of the matrices)
     best, best_v, trials = search(evaluate, DEFAULTS)
@@ -171,7 +177,7 @@ def tune(ctx, batch: int = 256, probes: int = 1, seed: int = 7000) -> Dict:
             "probe": {"workload": "batched uneven null-space solves (shift and incidence, n log-uniform in "
                                   "[1e3, 2e5]), mixed precision, tol_abs = 1e-12 L", "batch": batch,
                       "probes": probes, "seed": seed},
-            "metric": "solves/s of the probe batches (device time)", "knobs": best,
+            "metric": "geometric mean of the probe batches' solves/s (device time)", "knobs": best,
             "best_solves_per_s": best_v, "default_solves_per_s": trials[0]["solves_per_s"], "trials": trials}
 
 
