@@ -269,30 +269,43 @@ __global__ void col_count_kernel(int64_t nnz, const int32_t *ci, int32_t *cnt) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x)
     atomicAdd(cnt + ci[k], 1);
 }
-// exclusive scan of cnt[0..n) into out[0..n]; single block, chunked
+// exclusive scan of cnt[0..n) into out[0..n]; single block, 8 consecutive values
+// per thread and round: sums by warp shuffles, two barriers a round (1024 values
+// and 22 barriers a round: the device's part of creating a 200003-column incidence
+// matrix took 402 us, and takes 251)
 __global__ void __launch_bounds__(1024) scan_kernel(int64_t n, const int32_t *cnt, int32_t *out) {
-  __shared__ int32_t s[1024];
-  __shared__ int32_t carry;
-  if (threadIdx.x == 0)
-    carry = 0;
-  __syncthreads();
-  for (int64_t base = 0; base < n; base += 1024) {
-    const int64_t i = base + threadIdx.x;
-    const int32_t v = i < n ? cnt[i] : 0;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-      const int32_t t = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0;
-      __syncthreads();
-      s[threadIdx.x] += t;
-      __syncthreads();
+  constexpr int V = 8;
+  __shared__ int32_t s_warp[2][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int32_t carry = 0;
+  int buf = 0;
+  for (int64_t base = 0; base < n; base += 1024 * V, buf ^= 1) {
+    const int64_t i0 = base + (int64_t)threadIdx.x * V;
+    int32_t v[V], sum = 0;
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      v[k] = i0 + k < n ? cnt[i0 + k] : 0;
+      sum += v[k];
     }
-    if (i < n)
-      out[i] = carry + s[threadIdx.x] - v;
+    int32_t run = sum; // inclusive over the warp
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t t = __shfl_up_sync(0xffffffffu, run, o);
+      run += lane >= o ? t : 0;
+    }
+    if (lane == 31)
+      s_warp[buf][wid] = run;
     __syncthreads();
-    if (threadIdx.x == 1023)
-      carry += s[1023];
-    __syncthreads();
+    const int32_t w = s_warp[buf][lane];
+    const int32_t before = __reduce_add_sync(0xffffffffu, lane < wid ? w : 0);
+    const int32_t total = __reduce_add_sync(0xffffffffu, w);
+    int32_t at = carry + before + run - sum;
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      if (i0 + k < n)
+        out[i0 + k] = at;
+      at += v[k];
+    }
+    carry += total; // the next round writes the other buffer
   }
   if (threadIdx.x == 0)
     out[n] = carry;
@@ -395,6 +408,44 @@ __global__ void slice_fill_kernel(int64_t slices, const int32_t *off, const int3
         sv32[k] = (float)x;
     }
   }
+}
+
+// first entry of row [b, e) in column c or beyond (columns ascending)
+KR_DEV int32_t first_from(const int32_t *ci, int32_t b, int32_t e, int64_t c) {
+  while (b < e) {
+    const int32_t m = b + (e - b) / 2;
+    if (ci[m] < c)
+      b = m + 1;
+    else
+      e = m;
+  }
+  return b;
+}
+// entries of every row in column part [c0, c1)
+__global__ void part_count_kernel(int64_t rows, const int32_t *rp, const int32_t *ci, int64_t c0, int64_t c1,
+                                  int32_t *cnt) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t b = first_from(ci, rp[r], rp[r + 1], c0);
+    cnt[r] = first_from(ci, b, rp[r + 1], c1) - b;
+  }
+}
+// the part's entries; `at`: entries of the earlier parts, added to its row pointers
+__global__ void part_fill_kernel(int64_t rows, const int32_t *rp, const int32_t *ci, const double *v, int64_t c0,
+                                 const int32_t *prp, int32_t *pci, double *pv, float *pv32) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t b = first_from(ci, rp[r], rp[r + 1], c0), k0 = prp[r], len = prp[r + 1] - k0;
+    for (int32_t j = 0; j < len; j++) {
+      pci[k0 + j] = ci[b + j];
+      pv[k0 + j] = v[b + j];
+      if (pv32)
+        pv32[k0 + j] = (float)v[b + j];
+    }
+  }
+}
+__global__ void part_shift_kernel(int64_t n, const int32_t *by, int32_t *rp) { // rp[0..n) += *by
+  const int32_t d = *by;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    rp[i] += d;
 }
 
 __global__ void __launch_bounds__(1024) rng_mt_kernel(RngState *st, double *out, int64_t n) {
@@ -535,7 +586,9 @@ void preload_capi_kernels() {
                       (const void *)scan_kernel,        (const void *)scatter_kernel,
                       (const void *)row_sort_kernel,    (const void *)row_of_kernel,
                       (const void *)gather_t_kernel,    (const void *)slice_sort_kernel,
-                      (const void *)slice_fill_kernel,  (const void *)rng_mt_kernel,
+                      (const void *)slice_fill_kernel,  (const void *)part_count_kernel,
+                      (const void *)part_fill_kernel,   (const void *)part_shift_kernel,
+                      (const void *)rng_mt_kernel,
                       (const void *)rng_mt_states_kernel, (const void *)rng_mt_count_kernel,
                       (const void *)rng_mt_emit_kernel, (const void *)rng_mt_finish_kernel,
                       (const void *)rng_philox_kernel,  (const void *)rng_philox_advance};
@@ -787,6 +840,50 @@ extern "C" int krans_selftest_barrier_timeout(krans_ctx *ctx, double timeout_ms,
   return KRANS_OK;
 }
 
+// Columns from which x outgrows what L2 keeps of it beside the streamed operand
+// (gathers a second from x of 34 / 67 / 134 MB: 170 / 146 / 84 billion), and the
+// columns a part's piece of x should have at most.
+static constexpr int64_t kCutCols = 12582912, kPartCols = 6291456;
+
+// A^T cut into column parts (SpmvParts), queued on the context's stream. Without
+// room for it the operand stays whole: it is a second copy, for speed alone.
+static void cut_transpose(krans_ctx *ctx, krans_mat *A, int32_t *cnt) {
+  SpmvParts P;
+  const int64_t rows = A->n, cols = A->m, nnz = A->nnz;
+  P.parts = (int)std::min<int64_t>(kMaxParts, (cols + kPartCols - 1) / kPartCols);
+  if (cols < kCutCols || nnz < rows * P.parts) // fewer than an entry a row and part: y would cost more than x
+    return;
+  Carver lay;
+  auto carve = [&](Carver &c) {
+    for (int q = 0; q < P.parts; q++)
+      P.rp[q] = c.take<int32_t>(rows + 1);
+    P.ci = c.take<int32_t>(nnz);
+    P.v64 = c.take<double>(nnz);
+    P.v32 = A->vT32 ? c.take<float>(nnz) : nullptr;
+  };
+  carve(lay);
+  P.bytes = lay.off + 256;
+  if (dev_alloc(ctx, (void **)&P.base, P.bytes) != KRANS_OK) {
+    set_error("%s", "");
+    cudaGetLastError();
+    return;
+  }
+  Carver c;
+  c.base = P.base;
+  carve(c);
+  cudaStream_t s = ctx->stream;
+  const int g = grid_for(ctx, rows);
+  for (int q = 0; q < P.parts; q++) {
+    const int64_t c0 = cols * q / P.parts, c1 = cols * (q + 1) / P.parts;
+    part_count_kernel<<<g, 256, 0, s>>>(rows, A->rpT, A->ciT, c0, c1, cnt);
+    scan_kernel<<<1, 1024, 0, s>>>(rows, cnt, P.rp[q]);
+    if (q > 0) // after the entries of the parts before it
+      part_shift_kernel<<<g, 256, 0, s>>>(rows + 1, P.rp[q - 1] + rows, P.rp[q]);
+    part_fill_kernel<<<g, 256, 0, s>>>(rows, A->rpT, A->ciT, A->vT, c0, P.rp[q], P.ci, P.v64, P.v32);
+  }
+  A->partsT = P;
+}
+
 int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const int32_t *row_ptr,
                      const int32_t *col_idx, const double *values, int flags, krans_mat **out) {
   KR_CHECK_ARG(ctx && out, "krans_csr_create: NULL argument");
@@ -935,6 +1032,7 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
       fill(m, A->rp, A->ci, A->v, A->sl);
     if (slT)
       fill(n, A->rpT, A->ciT, A->vT, A->slT);
+    cut_transpose(ctx, A, cnt);
   } else if (e == cudaSuccess) {
     e = cudaMemsetAsync(A->rpT, 0, sz_rpT, s);
   }
@@ -967,6 +1065,7 @@ int krans_csr_destroy(krans_mat *A) {
   if (!A)
     return KRANS_OK;
   dev_free(A->ctx, A->base, A->bytes);
+  dev_free(A->ctx, A->partsT.base, A->partsT.bytes);
   delete A;
   return KRANS_OK;
 }

@@ -76,6 +76,22 @@ struct krans_ctx {
   int solo_cluster[3] = {-1, -1, -1};
 };
 
+namespace kr {
+// An operand cut by columns for the standalone SpMV (kr_spmv.cu): part q holds
+// every row's entries in columns [cols q / parts, cols (q + 1) / parts), in
+// storage order, as CSR of its own.
+constexpr int kMaxParts = 8;
+struct SpmvParts {
+  int parts = 0; // 0: not cut
+  int32_t *rp[kMaxParts] = {};
+  int32_t *ci = nullptr;
+  double *v64 = nullptr;
+  float *v32 = nullptr;
+  char *base = nullptr;
+  size_t bytes = 0;
+};
+} // namespace kr
+
 struct krans_mat {
   krans_ctx *ctx = nullptr;
   int64_t m = 0, n = 0, nnz = 0;
@@ -86,6 +102,7 @@ struct krans_mat {
   int32_t ulen = 0, ulenT = 0; // uniform row length of A / A^T (0 = not uniform)
   kr::SlicedView sl{}, slT{};  // sorted slices of A / A^T for the solvers (slices = 0: not kept)
   krans_spmv_tuning tune{}, tuneT{}; // standalone SpMV kernel of A / A^T (zero: automatic)
+  kr::SpmvParts partsT;              // A^T cut by columns, where its x is larger than L2
   char *base = nullptr;         // one device allocation holding every stored array
   size_t bytes = 0;
 };
@@ -113,10 +130,12 @@ struct SpmvOperand {
   int lanes;
   int32_t ulen;
   krans_spmv_tuning tune;
+  const SpmvParts *cut; // or nullptr
 };
 inline SpmvOperand spmv_operand(const krans_mat *A, int trans) {
-  return trans ? SpmvOperand{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, A->lanesT, A->ulenT, A->tuneT}
-               : SpmvOperand{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, A->lanes, A->ulen, A->tune};
+  return trans ? SpmvOperand{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, A->lanesT, A->ulenT, A->tuneT,
+                             A->partsT.parts ? &A->partsT : nullptr}
+               : SpmvOperand{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, A->lanes, A->ulen, A->tune, nullptr};
 }
 // y = op x on `s` (kr_spmv.cu); fp32: FP32 values and sums
 cudaError_t spmv_launch(const SpmvOperand &A, bool fp32, const double *x, double *y, int sms, cudaStream_t s);
