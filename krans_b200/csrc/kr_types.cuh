@@ -18,8 +18,8 @@
 namespace kr {
 
 struct GridBarrierState {
-  unsigned int count;
-  unsigned int gen;
+  unsigned int count; // blocks that have arrived, over all barriers (zero at launch)
+  unsigned int spare;
   int error; // sticky: once set, barriers return at once and solvers unwind
   int pad;
   uint64_t timeout_ns; // longest wait at one barrier; 0 = the default (kBarrierTimeoutNs)
