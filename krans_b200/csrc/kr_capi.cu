@@ -1332,11 +1332,15 @@ int krans_rng_normal(krans_rng *r, krans_vec *out) {
   if (r->mode == KRANS_RNG_PHILOX) {
     rng_philox_kernel<<<grid_for(c, out->n), 256, 0, c->stream>>>(r->d, out->d, out->n);
     rng_philox_advance<<<1, 1, 0, c->stream>>>(r->d, out->n);
-  } else if (out->n < kMtLong) {
-    rng_mt_kernel<<<1, 1024, 0, c->stream>>>(r->d, out->d, out->n);
   } else {
+    // one block draws what is short, what finds no room for scratch, and what is
+    // being captured (scratch taken during a capture would belong to the graph)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    KR_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+    const bool whole = out->n < kMtLong || cap != cudaStreamCaptureStatusNone;
     // pieces, so that the words stay within the kept scratch
-    for (int64_t at = 0; at < out->n; at += kMtPiece) {
+    int64_t at = 0;
+    for (; !whole && at < out->n; at += std::min(kMtPiece, out->n - at)) {
       const int64_t n = std::min(kMtPiece, out->n - at);
       // attempts for n / 2 accepted ones: mean n / 2 / p and six standard
       // deviations, p = pi / 4; four words each, after the current state
@@ -1349,9 +1353,11 @@ int krans_rng_normal(krans_rng *r, krans_vec *out) {
       lay.take<int32_t>(blocks);
       lay.take<int64_t>(2);
       WsHold ws;
-      const int rc = ws_take(c, lay.off + 256, &ws, true);
-      if (rc != KRANS_OK)
-        return rc;
+      if (ws_take(c, lay.off + 256, &ws, true) != KRANS_OK) {
+        set_error("%s", "");
+        cudaGetLastError();
+        break;
+      }
       Carver cv;
       cv.base = (char *)ws.p;
       uint32_t *words = cv.take<uint32_t>(states * 624);
@@ -1364,6 +1370,8 @@ int krans_rng_normal(krans_rng *r, krans_vec *out) {
       rng_mt_finish_kernel<<<1, 1024, 0, c->stream>>>(r->d, words, states, cnt, blocks, out->d + at, n, last, saved);
       ws_give(c, &ws);
     }
+    if (at < out->n)
+      rng_mt_kernel<<<1, 1024, 0, c->stream>>>(r->d, out->d + at, out->n - at);
   }
   KR_CUDA(cudaGetLastError());
   return KRANS_OK;

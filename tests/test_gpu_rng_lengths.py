@@ -16,3 +16,12 @@ def test_normals_over_lengths(ctx, oracle, lengths):
     ref = oracle.Rng(77)
     for n in lengths:
         np.testing.assert_allclose(vf.create_random_of_size(n).data(), ref.normal(n), rtol=1e-14, atol=0)
+
+
+def test_normals_without_room_for_scratch(ctx, oracle):
+    """A budget that holds the vector (160 kB) but not the words of a whole-GPU draw (240 kB): one block draws."""
+    import krans_b200 as kb
+    vf = kb.CudaVectorFactory(kb.Context(0, hbm_budget=300_000), 1, seed=78)
+    ref = oracle.Rng(78)
+    x = vf.create_random_of_size(20001)
+    np.testing.assert_allclose(x.data(), ref.normal(20001), rtol=1e-14, atol=0)
