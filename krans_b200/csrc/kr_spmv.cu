@@ -316,7 +316,7 @@ static cudaError_t spmv_launch_t(const SpmvOperand &A, const VT *val, const doub
     spmv_lanes_kernel<VT><<<g, kSpmvThreads, 0, s>>>(A.rows, A.rp, A.ci, val, x, y, A.lanes);
     return cudaGetLastError();
   }
-  if (A.cut && A.tune.kernel == KRANS_SPMV_AUTO) {
+  if (A.cut && A.tune.kernel == KRANS_SPMV_AUTO && A.tune.rows_per_block == 0) {
     // One column part after the other, each with its piece of x in L2. The sums
     // go on from part to part in storage order, so the result is the same.
     const VT *pv = sizeof(VT) == 8 ? (const VT *)A.cut->v64 : (const VT *)A.cut->v32;
