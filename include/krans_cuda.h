@@ -422,8 +422,8 @@ int krans_solve_batch(krans_ctx *ctx, int64_t count, const krans_request *reqs,
  *   lanes[6]      threads per row of the solvers' SpMV for operands whose mean
  *                 row length is <= 3, <= 8, <= 16, <= 32, <= 64, > 64
  *                 (1, 2, 4, 8, 16, 32); powers of two up to 32. Operands whose
- *                 rows all hold exactly 1, 2 or 4 entries use one thread per
- *                 row whatever the table says.
+ *                 rows hold at most 64 entries each are read one row per
+ *                 lane whatever the table says.
  * The lanes apply to every solve of the context (single and batched); a
  * request's rounding depends on them, so results are reproducible for a
  * given table. */
