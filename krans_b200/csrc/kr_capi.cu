@@ -1337,10 +1337,12 @@ int krans_rng_normal(krans_rng *r, krans_vec *out) {
     // being captured (scratch taken during a capture would belong to the graph)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     KR_CUDA(cudaStreamIsCapturing(c->stream, &cap));
-    const bool whole = out->n < kMtLong || cap != cudaStreamCaptureStatusNone;
-    // pieces, so that the words stay within the kept scratch
+    const bool one = cap != cudaStreamCaptureStatusNone;
+    // Pieces, so that the words stay within the kept scratch. A rest shorter than
+    // kMtLong is one block's too: a piece has pairs to draw, also where it starts
+    // with a carried value (one of a single value would need none).
     int64_t at = 0;
-    for (; !whole && at < out->n; at += std::min(kMtPiece, out->n - at)) {
+    for (; !one && out->n - at >= kMtLong; at += std::min(kMtPiece, out->n - at)) {
       const int64_t n = std::min(kMtPiece, out->n - at);
       // attempts for n / 2 accepted ones: mean n / 2 / p and six standard
       // deviations, p = pi / 4; four words each, after the current state
