@@ -85,7 +85,7 @@ bool ws_release(krans_ctx *ctx) {
   return true;
 }
 
-int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, bool stream_ordered) {
+int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, WsOwn own) {
   *w = WsHold{};
   if (bytes <= kWsKeep) {
     std::lock_guard<std::mutex> lk(ctx->ws_mu);
@@ -111,10 +111,16 @@ int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, bool stream_ordered) {
       }
     }
   }
-  const int rc = stream_ordered ? dev_alloc_async(ctx, &w->p, bytes, ctx->stream) : dev_alloc(ctx, &w->p, bytes);
+  if (own == WsOwn::kUncounted) {
+    KR_CUDA(cudaMallocAsync(&w->p, bytes, ctx->stream));
+    w->mode = WsHold::kOwnUncounted;
+    return KRANS_OK;
+  }
+  const bool async = own == WsOwn::kStream;
+  const int rc = async ? dev_alloc_async(ctx, &w->p, bytes, ctx->stream) : dev_alloc(ctx, &w->p, bytes);
   if (rc == KRANS_OK) {
     w->bytes = bytes;
-    w->mode = stream_ordered ? WsHold::kOwnAsync : WsHold::kOwn;
+    w->mode = async ? WsHold::kOwnAsync : WsHold::kOwn;
   }
   return rc;
 }
@@ -127,6 +133,8 @@ void ws_give(krans_ctx *ctx, WsHold *w) {
     dev_free(ctx, w->p, w->bytes);
   } else if (w->mode == WsHold::kOwnAsync) {
     dev_free_async(ctx, w->p, w->bytes, ctx->stream);
+  } else if (w->mode == WsHold::kOwnUncounted) {
+    cudaFreeAsync(w->p, ctx->stream);
   }
   *w = WsHold{};
 }
@@ -983,7 +991,7 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   WsHold scr;
   const size_t sz_w = up((size_t)(std::max(m, n) / 32 + 1) * 4); // slice widths, one operand at a time
   const size_t sz_scr = up(sz_rpT) + 3 * up(sz_ci) + sz_w;
-  rc = ws_take(ctx, sz_scr, &scr, true);
+  rc = ws_take(ctx, sz_scr, &scr, WsOwn::kUncounted); // gone when this returns: the budget is for what stays
   if (rc != KRANS_OK) {
     krans_csr_destroy(A);
     return rc;
@@ -1355,7 +1363,7 @@ int krans_rng_normal(krans_rng *r, krans_vec *out) {
       lay.take<int32_t>(blocks);
       lay.take<int64_t>(2);
       WsHold ws;
-      if (ws_take(c, lay.off + 256, &ws, true) != KRANS_OK) {
+      if (ws_take(c, lay.off + 256, &ws, WsOwn::kStream) != KRANS_OK) {
         set_error("%s", "");
         cudaGetLastError();
         break;

@@ -155,11 +155,15 @@ constexpr size_t kWsKeep = (size_t)256 << 20;
 struct WsHold {
   void *p = nullptr;
   size_t bytes = 0;
-  enum { kNone, kKept, kOwn, kOwnAsync } mode = kNone;
+  enum { kNone, kKept, kOwn, kOwnAsync, kOwnUncounted } mode = kNone;
 };
-// stream_ordered: an allocation of the call's own is freed in stream order (the
-// caller need not have waited for its kernels)
-int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, bool stream_ordered = false);
+// What a call that does not get the kept scratch allocates for itself
+enum class WsOwn {
+  kDevice,    // cudaMalloc; the caller has waited for its kernels when it gives it back
+  kStream,    // freed in stream order (it need not have waited)
+  kUncounted, // the same, and the budget does not count it
+};
+int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, WsOwn own = WsOwn::kDevice);
 void ws_give(krans_ctx *ctx, WsHold *w);
 bool ws_release(krans_ctx *ctx); // frees idle scratch; true if there was any
 // Stream-ordered forms (cudaMallocAsync / cudaFreeAsync on `s`): neither
