@@ -44,22 +44,16 @@ static int budget_fail(krans_ctx *ctx, size_t bytes) {
   return KRANS_ERR_OUT_OF_MEMORY;
 }
 
+static bool give_back(krans_ctx *ctx);
 int dev_alloc(krans_ctx *ctx, void **p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0)
     bytes = 256;
-  if (over_budget(ctx, bytes) && !(ws_release(ctx) && !over_budget(ctx, bytes)))
+  if (over_budget(ctx, bytes))
     return budget_fail(ctx, bytes);
   cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && ws_release(ctx)) {
-    // back from the stream-ordered pool to the device
-    cudaGetLastError();
-    cudaStreamSynchronize(ctx->stream);
-    cudaMemPool_t pool;
-    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess)
-      cudaMemPoolTrimTo(pool, 0);
+  if (e == cudaErrorMemoryAllocation && give_back(ctx))
     e = cudaMalloc(p, bytes);
-  }
   if (e != cudaSuccess)
     return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
   ctx->in_use.fetch_add(bytes);
@@ -77,7 +71,7 @@ static void ws_drop(krans_ctx *ctx) {
   ctx->ws_bytes = 0;
 }
 
-bool ws_release(krans_ctx *ctx) {
+static bool ws_release(krans_ctx *ctx) { // true if there was idle scratch
   std::lock_guard<std::mutex> lk(ctx->ws_mu);
   if (!ctx->ws || ctx->ws_busy)
     return false;
@@ -85,16 +79,33 @@ bool ws_release(krans_ctx *ctx) {
   return true;
 }
 
+// When the device has no room: what the context holds beyond its callers' own
+// allocations goes back, from the stream-ordered pool to the device. False if
+// there was nothing.
+static bool give_back(krans_ctx *ctx) {
+  cudaGetLastError(); // the failed allocation's
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+    return false;
+  if (!ws_release(ctx))
+    return false;
+  cudaStreamSynchronize(ctx->stream);
+  cudaMemPool_t pool;
+  if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, 0);
+  return true;
+}
+
 int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, WsOwn own) {
   *w = WsHold{};
-  if (bytes <= kWsKeep) {
+  if (!ctx->budget && bytes <= kWsKeep) {
     std::lock_guard<std::mutex> lk(ctx->ws_mu);
     if (!ctx->ws_busy) {
       if (ctx->ws_bytes < bytes) {
         // grown by half again, so that a run of growing calls reallocates a few times only
         const size_t want = std::min(kWsKeep, std::max(bytes + bytes / 2, (size_t)1 << 20));
         ws_drop(ctx);
-        if (!over_budget(ctx, want) && cudaMallocAsync((void **)&ctx->ws, want, ctx->stream) == cudaSuccess) {
+        if (cudaMallocAsync((void **)&ctx->ws, want, ctx->stream) == cudaSuccess) {
           ctx->ws_bytes = want;
           ctx->in_use.fetch_add(want);
         } else {
@@ -155,6 +166,8 @@ int dev_alloc_async(krans_ctx *ctx, void **p, size_t bytes, cudaStream_t s) {
   if (over_budget(ctx, bytes))
     return budget_fail(ctx, bytes);
   cudaError_t e = cudaMallocAsync(p, bytes, s);
+  if (e == cudaErrorMemoryAllocation && give_back(ctx))
+    e = cudaMallocAsync(p, bytes, s);
   if (e != cudaSuccess)
     return cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
   ctx->in_use.fetch_add(bytes);

@@ -149,8 +149,9 @@ void dev_free(krans_ctx *ctx, void *p, size_t bytes);
 // another (a nested solve, another thread) gets an allocation of its own. What a
 // call has queued may still use it after ws_give: the next holder queues on the
 // same stream. At most kWsKeep bytes are kept; a call that needs more, or finds
-// the budget or the device short, allocates for itself, and dev_alloc gives idle
-// scratch back before it fails.
+// the device short, allocates for itself, and idle scratch goes back to the
+// device before an allocation fails. A context with a budget keeps none: it
+// would count against calls that fit beside what the callers themselves hold.
 constexpr size_t kWsKeep = (size_t)256 << 20;
 struct WsHold {
   void *p = nullptr;
@@ -165,7 +166,6 @@ enum class WsOwn {
 };
 int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, WsOwn own = WsOwn::kDevice);
 void ws_give(krans_ctx *ctx, WsHold *w);
-bool ws_release(krans_ctx *ctx); // frees idle scratch; true if there was any
 // Stream-ordered forms (cudaMallocAsync / cudaFreeAsync on `s`): neither
 // waits for kernels running on other streams, unlike cudaFree, which waits
 // for the whole device. The served paths use them so that releasing one

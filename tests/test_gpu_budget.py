@@ -24,3 +24,31 @@ def test_creation_scratch_is_outside_the_budget():
     M = kb.CudaCsrMatrixAdapter(ctx, n, n, *_ring(n))  # the device transpose takes another 2.8 MB meanwhile
     assert ctx.memory_in_use() <= _plain_bytes(n, n, 2 * n)
     del M
+
+
+def test_batch_after_a_solve_under_a_budget():
+    """The smallest budget that holds a batch also holds it after a single solve and a block product."""
+    import krans_b200 as kb
+    from krans_b200.serving import SolveRequest, solve_batch
+    n = 3000
+    opt = kb.CyclicLanczosOptions(k=1, tol_abs=1e-12, tol_rel=0.0, cg_maxit=200, max_restarts=2, grad_max_iters=10)
+
+    def runs(budget, before):
+        ctx = kb.Context(0, hbm_budget=budget)
+        try:
+            M = kb.CudaCsrMatrixAdapter(ctx, n, n, *_ring(n))
+            if before:
+                held = ctx.memory_in_use()
+                kb.find_nullspace_cyclic_lanczos(M, kb.CudaVectorFactory(ctx, n, seed=1), opt)
+                assert ctx.memory_in_use() == held  # the basis and the factory are gone, nothing is kept
+            solve_batch(ctx, [SolveRequest(M, opt, seed=1 + i, keep_basis=False) for i in range(3)])
+            return True
+        except kb.KransError:
+            return False
+
+    lo, hi = 0, 64 << 20
+    assert runs(hi, False)
+    while hi - lo > 1024:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if runs(mid, False) else (mid, hi)
+    assert runs(hi, True)
