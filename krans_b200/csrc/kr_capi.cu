@@ -96,6 +96,27 @@ static bool give_back(krans_ctx *ctx) {
   return true;
 }
 
+SpeedCopy::~SpeedCopy() {
+  cudaFreeAsync(base, ctx->stream);
+  release_bytes(ctx, bytes);
+}
+// Room for a second copy, or nullptr
+static std::unique_ptr<SpeedCopy> copy_alloc(krans_ctx *ctx, size_t bytes) {
+  char *p = nullptr;
+  if (ctx->budget)
+    return nullptr;
+  if (cudaMallocAsync((void **)&p, bytes, ctx->stream) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  ctx->in_use.fetch_add(bytes);
+  auto c = std::make_unique<SpeedCopy>();
+  c->ctx = ctx;
+  c->base = p;
+  c->bytes = bytes;
+  return c;
+}
+
 int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, WsOwn own) {
   *w = WsHold{};
   if (!ctx->budget && bytes <= kWsKeep) {
@@ -866,8 +887,7 @@ extern "C" int krans_selftest_barrier_timeout(krans_ctx *ctx, double timeout_ms,
 // columns a part's piece of x should have at most.
 static constexpr int64_t kCutCols = 12582912, kPartCols = 6291456;
 
-// A^T cut into column parts (SpmvParts), queued on the context's stream. Without
-// room for it the operand stays whole: it is a second copy, for speed alone.
+// A^T cut into column parts (SpmvParts), queued on the context's stream.
 static void cut_transpose(krans_ctx *ctx, krans_mat *A, int32_t *cnt) {
   SpmvParts P;
   const int64_t rows = A->n, cols = A->m, nnz = A->nnz;
@@ -883,14 +903,11 @@ static void cut_transpose(krans_ctx *ctx, krans_mat *A, int32_t *cnt) {
     P.v32 = A->vT32 ? c.take<float>(nnz) : nullptr;
   };
   carve(lay);
-  P.bytes = lay.off + 256;
-  if (dev_alloc(ctx, (void **)&P.base, P.bytes) != KRANS_OK) {
-    set_error("%s", "");
-    cudaGetLastError();
+  auto copy = copy_alloc(ctx, lay.off + 256);
+  if (!copy)
     return;
-  }
   Carver c;
-  c.base = P.base;
+  c.base = copy->base;
   carve(c);
   cudaStream_t s = ctx->stream;
   const int g = grid_for(ctx, rows);
@@ -902,7 +919,8 @@ static void cut_transpose(krans_ctx *ctx, krans_mat *A, int32_t *cnt) {
       part_shift_kernel<<<g, 256, 0, s>>>(rows + 1, P.rp[q - 1] + rows, P.rp[q]);
     part_fill_kernel<<<g, 256, 0, s>>>(rows, A->rpT, A->ciT, A->vT, c0, P.rp[q], P.ci, P.v64, P.v32);
   }
-  A->partsT = P;
+  copy->cut = P;
+  A->cut = std::move(copy);
 }
 
 int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const int32_t *row_ptr,
@@ -951,12 +969,7 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   // (a CG iteration at 4000 columns 12.8 -> 10.9 us, at 100000 36 -> 29 us)
   const bool sl = nnz > 0 && !(uni && L == 2) && szA.longest <= kSliceMaxLen;
   const bool slT = nnz > 0 && !(uniT && LT == 2) && szT.longest <= kSliceMaxLen;
-  auto slice_bytes = [&](int64_t rows, const SliceSize &z) {
-    const size_t slots = (size_t)((rows + 31) / 32) * 32, e = (size_t)(nnz + z.padding());
-    return up(slots * 4) + up((slots / 32 + 1) * 4) + up(e * 4) + up(e * 8) + (f32 ? up(e * 4) : 0);
-  };
-  const size_t total = up(sz_rp) + 2 * up(sz_ci) + 2 * up(sz_v) + up(sz_rpT) + (f32 ? 2 * up(sz_v32) : 0) +
-                       (sl ? slice_bytes(m, szA) : 0) + (slT ? slice_bytes(n, szT) : 0);
+  const size_t total = up(sz_rp) + 2 * up(sz_ci) + 2 * up(sz_v) + up(sz_rpT) + (f32 ? 2 * up(sz_v32) : 0);
   char *base = nullptr;
   int rc = dev_alloc(ctx, (void **)&base, total);
   if (rc != KRANS_OK)
@@ -984,19 +997,36 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
     A->v32 = (float *)take(sz_v32);
     A->vT32 = (float *)take(sz_v32);
   }
-  auto take_slices = [&](int64_t rows, const SliceSize &z, SlicedView &S) {
-    const size_t nsl = (size_t)((rows + 31) / 32), e = (size_t)(nnz + z.padding());
+  // the slices of both operands, in an allocation of their own
+  auto carve_slices = [&](Carver &c, int64_t rows, const SliceSize &z) {
+    const int64_t nsl = (rows + 31) / 32, e = nnz + z.padding();
+    SlicedView S;
     S.slices = (int32_t)nsl;
-    S.row = (int32_t *)take(nsl * 32 * 4);
-    S.off = (int32_t *)take((nsl + 1) * 4);
-    S.ci = (int32_t *)take(e * 4);
-    S.v64 = (double *)take(e * 8);
-    S.v32 = f32 ? (float *)take(e * 4) : nullptr;
+    S.row = c.take<int32_t>(nsl * 32);
+    S.off = c.take<int32_t>(nsl + 1);
+    S.ci = c.take<int32_t>(e);
+    S.v64 = c.take<double>(e);
+    S.v32 = f32 ? c.take<float>(e) : nullptr;
+    return S;
   };
-  if (sl)
-    take_slices(m, szA, A->sl);
-  if (slT)
-    take_slices(n, szT, A->slT);
+  if (sl || slT) {
+    SlicedView S{}, ST{};
+    auto carve = [&](Carver &c) {
+      if (sl)
+        S = carve_slices(c, m, szA);
+      if (slT)
+        ST = carve_slices(c, n, szT);
+    };
+    Carver lay;
+    carve(lay);
+    if ((A->slices = copy_alloc(ctx, lay.off + 256))) {
+      Carver c;
+      c.base = A->slices->base;
+      carve(c);
+      A->slices->sl = S;
+      A->slices->slT = ST;
+    }
+  }
   // scratch of the device transpose: kept by the context and used in stream
   // order, so releasing it does not wait for the device, and the next matrix's
   // host work overlaps this matrix's transpose kernels
@@ -1049,10 +1079,10 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
           S.slices, off, row, rp, ci, v, const_cast<int32_t *>(S.ci), const_cast<double *>(S.v64),
           const_cast<float *>(S.v32));
     };
-    if (sl)
-      fill(m, A->rp, A->ci, A->v, A->sl);
-    if (slT)
-      fill(n, A->rpT, A->ciT, A->vT, A->slT);
+    if (A->slices && sl)
+      fill(m, A->rp, A->ci, A->v, A->slices->sl);
+    if (A->slices && slT)
+      fill(n, A->rpT, A->ciT, A->vT, A->slices->slT);
     cut_transpose(ctx, A, cnt);
   } else if (e == cudaSuccess) {
     e = cudaMemsetAsync(A->rpT, 0, sz_rpT, s);
@@ -1086,7 +1116,6 @@ int krans_csr_destroy(krans_mat *A) {
   if (!A)
     return KRANS_OK;
   dev_free(A->ctx, A->base, A->bytes);
-  dev_free(A->ctx, A->partsT.base, A->partsT.bytes);
   delete A;
   return KRANS_OK;
 }

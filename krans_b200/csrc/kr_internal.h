@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -87,8 +88,19 @@ struct SpmvParts {
   int32_t *ci = nullptr;
   double *v64 = nullptr;
   float *v32 = nullptr;
+};
+// A second copy of a matrix's entries, kept for speed alone: the sorted slices of
+// A and A^T that the solvers read, or A^T cut by columns. A matrix does without
+// where there is no room, and in a context with a budget, which is for what the
+// callers ask for (a planted FP64 matrix takes 20 bytes an entry, and 47 with its
+// slices).
+struct SpeedCopy {
+  krans_ctx *ctx = nullptr;
   char *base = nullptr;
   size_t bytes = 0;
+  SlicedView sl{}, slT{}; // slices = 0: that operand has none
+  SpmvParts cut;          // parts = 0: not cut
+  ~SpeedCopy();           // frees it in the order of the context's stream
 };
 } // namespace kr
 
@@ -100,9 +112,9 @@ struct krans_mat {
   float *v32 = nullptr, *vT32 = nullptr;
   int lanes = 1, lanesT = 1;
   int32_t ulen = 0, ulenT = 0; // uniform row length of A / A^T (0 = not uniform)
-  kr::SlicedView sl{}, slT{};  // sorted slices of A / A^T for the solvers (slices = 0: not kept)
   krans_spmv_tuning tune{}, tuneT{}; // standalone SpMV kernel of A / A^T (zero: automatic)
-  kr::SpmvParts partsT;              // A^T cut by columns, where its x is larger than L2
+  std::unique_ptr<kr::SpeedCopy> slices; // sorted slices of A / A^T for the solvers
+  std::unique_ptr<kr::SpeedCopy> cut;    // A^T cut by columns, where its x is larger than L2
   char *base = nullptr;         // one device allocation holding every stored array
   size_t bytes = 0;
 };
@@ -134,7 +146,7 @@ struct SpmvOperand {
 };
 inline SpmvOperand spmv_operand(const krans_mat *A, int trans) {
   return trans ? SpmvOperand{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, A->lanesT, A->ulenT, A->tuneT,
-                             A->partsT.parts ? &A->partsT : nullptr}
+                             A->cut ? &A->cut->cut : nullptr}
                : SpmvOperand{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, A->lanes, A->ulen, A->tune, nullptr};
 }
 // y = op x on `s` (kr_spmv.cu); fp32: FP32 values and sums
@@ -216,10 +228,11 @@ constexpr int64_t kServedGridMin = 120000;
 std::atomic<int> &device_servers(int device);
 // A (or its stored transpose) as the solvers' device code sees it
 inline CsrView csr_view(const krans_mat *A, bool trans) {
+  const SlicedView none{};
   if (trans)
     return CsrView{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, tuned_lanes(A->ctx, A->n, A->nnz), A->ulenT,
-                   A->slT};
+                   A->slices ? A->slices->slT : none};
   return CsrView{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, tuned_lanes(A->ctx, A->m, A->nnz), A->ulen,
-                 A->sl};
+                 A->slices ? A->slices->sl : none};
 }
 } // namespace kr

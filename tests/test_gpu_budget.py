@@ -3,6 +3,8 @@
 import numpy as np
 import pytest
 
+from krans_b200 import generators as G
+
 pytestmark = pytest.mark.gpu
 
 
@@ -52,3 +54,16 @@ def test_batch_after_a_solve_under_a_budget():
         mid = (lo + hi) // 2
         lo, hi = (lo, mid) if runs(mid, False) else (mid, hi)
     assert runs(hi, True)
+
+
+def test_creation_without_room_for_slices():
+    """Rows and columns of uneven lengths: the sorted slices do not count against the budget of the arrays."""
+    import krans_b200 as kb
+    A = G.planted_kernel(6000, 4000, 8, kernel=False).A
+    m, n = A.shape
+    ctx = kb.Context(0, hbm_budget=_plain_bytes(m, n, A.nnz) + 8 * (m + n) + 1024)
+    M = kb.CudaCsrMatrixAdapter.from_scipy(ctx, A)
+    x = kb.CudaVectorAdapter.from_numpy(ctx, np.ones(n))
+    y = kb.CudaVectorAdapter(ctx, m)
+    M.multiply(x, y)
+    np.testing.assert_allclose(y.data(), A @ np.ones(n), rtol=1e-12, atol=1e-12)
