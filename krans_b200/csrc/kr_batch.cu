@@ -118,6 +118,8 @@ struct BatchLaunch {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   std::vector<CyclicRequestDev> hreq;
   std::vector<RngState> hrng;
+  std::vector<const krans_mat *> mats;             // of hreq
+  std::vector<std::shared_ptr<SpeedCopy>> slices;  // of the requests, until release()
 
   int classify(const krans_mat *A) const {
     const int64_t sz = A->m + A->n;
@@ -126,7 +128,16 @@ struct BatchLaunch {
     return (npairs > 0 && sz < pair_max) ? 1 : 0;
   }
 
-  // Descriptor and RNG stream of one request (no per-slot pointers yet);
+  // the operands of a request, once the launch's memory is allocated
+  void set_operands(CyclicRequestDev &q, const krans_mat *A) {
+    auto s = hold_slices(A);
+    q.F = csr_view(A, false, s.get());
+    q.B = csr_view(A, true, s.get());
+    if (s)
+      slices.push_back(std::move(s));
+  }
+
+  // Descriptor and RNG stream of one request (no operands and no per-slot pointers yet);
   // *carve = its workspace bytes (0 if trivial).
   int describe(const krans_request &r, CyclicRequestDev &q, RngState &s, size_t *carve) const {
     KR_CHECK_ARG(r.A && r.A->ctx == ctx, "krans_solve_batch: request without a matrix of this context");
@@ -136,8 +147,6 @@ struct BatchLaunch {
                  "krans_solve_batch: mixed precision needs matrices created with KRANS_CSR_FP32");
     const krans_mat *A = r.A;
     memset(&q, 0, sizeof q);
-    q.F = csr_view(A, false);
-    q.B = csr_view(A, true);
     q.o = r.opts;
     q.o.team = KRANS_TEAM_CTA;
     int64_t kt = (r.opts.nullity_known >= 0) ? (int64_t)r.opts.nullity_known : r.opts.k;
@@ -240,12 +249,14 @@ struct BatchLaunch {
     }
     hreq.assign(n, CyclicRequestDev{});
     hrng.assign(n, RngState{});
+    mats.assign(n, nullptr);
     ws_stride = stride_L = stride_M = 256;
     for (int pos = 0; pos < n; pos++) {
       size_t cv = 0;
       const int rc = describe(reqs[order[pos]], hreq[pos], hrng[pos], &cv);
       if (rc != KRANS_OK)
         return rc;
+      mats[pos] = reqs[order[pos]].A;
       if (pos < n_large)
         stride_L = std::max(stride_L, cv);
       else if (pos < n_large + n_mid)
@@ -349,6 +360,7 @@ struct BatchLaunch {
     }
     for (int pos = 0; pos < count; pos++) {
       const int g = slot_of(pos);
+      set_operands(hreq[pos], mats[pos]);
       hreq[pos].res = d_res + g;
       hreq[pos].status = d_status + g;
       hreq[pos].max_resid = d_mr + g;
@@ -468,6 +480,7 @@ struct BatchLaunch {
     if (npub[cl] >= cap[cl] || cv > stride || (cl == 0 && nclusters == 0) || (cl == 1 && npairs == 0))
       return 0;
     const int g = base[cl] + npub[cl];
+    set_operands(q, r.A);
     q.res = d_res + g;
     q.status = d_status + g;
     q.max_resid = d_mr + g;
@@ -565,6 +578,7 @@ struct BatchLaunch {
   // `graveyard` when one is given (cudaFreeHost waits for the whole device;
   // the server frees them once nothing runs), else are freed here.
   void release(std::vector<void *> *graveyard = nullptr) {
+    slices.clear();
     if (ws)
       dev_free_async(ctx, ws, ws_bytes, stream);
     if (meta)
@@ -768,6 +782,10 @@ bool krans_server::admit_lobpcg(uint64_t id, Clock::time_point now) {
   if (ew == cudaSuccess)
     ew = cudaStreamWaitEvent(streams[fs], ctx_ready, 0);
   rc = ew == cudaSuccess ? lobpcg_async_launch(a, streams[fs]) : cuda_fail(ew, "server stream order", __FILE__, __LINE__);
+  if (rc == KRANS_ERR_OUT_OF_MEMORY && !inflight.empty()) {
+    lobpcg_async_release(a, &graveyard);
+    return false; // the launches in flight hold what it lacks, copies of their matrices among it
+  }
   queue.pop_front();
   if (rc != KRANS_OK) {
     lobpcg_async_release(a, &graveyard);
@@ -889,6 +907,14 @@ bool krans_server::admit_cyclic(Clock::time_point now) {
   if (ew == cudaSuccess)
     ew = cudaStreamWaitEvent(streams[fs], ctx_ready, 0);
   rc = ew == cudaSuccess ? f->L.alloc_and_launch(streams[fs]) : cuda_fail(ew, "server stream order", __FILE__, __LINE__);
+  if (rc == KRANS_ERR_OUT_OF_MEMORY && !inflight.empty()) {
+    // as for a LOBPCG request: wait for the launches in flight
+    for (auto it = take.rbegin(); it != take.rend(); ++it)
+      queue.push_front(*it);
+    f->L.release(&graveyard);
+    delete f;
+    return false;
+  }
   if (rc != KRANS_OK) {
     for (auto id2 : take)
       fail(id2, rc, now);

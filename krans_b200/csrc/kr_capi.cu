@@ -87,7 +87,17 @@ static bool give_back(krans_ctx *ctx) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
     return false;
-  if (!ws_release(ctx))
+  bool any = ws_release(ctx);
+  {
+    std::lock_guard<std::mutex> lk(ctx->copies_mu);
+    for (krans_mat *A : ctx->copied)
+      for (auto *c : {&A->slices, &A->cut})
+        if (*c && c->use_count() == 1 && !(*c)->captured) { // nothing but the matrix holds it
+          c->reset();
+          any = true;
+        }
+  }
+  if (!any)
     return false;
   cudaStreamSynchronize(ctx->stream);
   cudaMemPool_t pool;
@@ -101,7 +111,7 @@ SpeedCopy::~SpeedCopy() {
   release_bytes(ctx, bytes);
 }
 // Room for a second copy, or nullptr
-static std::unique_ptr<SpeedCopy> copy_alloc(krans_ctx *ctx, size_t bytes) {
+static std::shared_ptr<SpeedCopy> copy_alloc(krans_ctx *ctx, size_t bytes) {
   char *p = nullptr;
   if (ctx->budget)
     return nullptr;
@@ -110,7 +120,7 @@ static std::unique_ptr<SpeedCopy> copy_alloc(krans_ctx *ctx, size_t bytes) {
     return nullptr;
   }
   ctx->in_use.fetch_add(bytes);
-  auto c = std::make_unique<SpeedCopy>();
+  auto c = std::make_shared<SpeedCopy>();
   c->ctx = ctx;
   c->base = p;
   c->bytes = bytes;
@@ -1108,6 +1118,10 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   // SpMV skip the row pointers and use vector loads
   A->ulen = uni ? (int32_t)L : 0;
   A->ulenT = uniT ? LT : 0;
+  if (A->slices || A->cut) {
+    std::lock_guard<std::mutex> lk(ctx->copies_mu);
+    ctx->copied.push_back(A);
+  }
   *out = A;
   return KRANS_OK;
 }
@@ -1115,6 +1129,11 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
 int krans_csr_destroy(krans_mat *A) {
   if (!A)
     return KRANS_OK;
+  {
+    std::lock_guard<std::mutex> lk(A->ctx->copies_mu);
+    auto &all = A->ctx->copied;
+    all.erase(std::remove(all.begin(), all.end(), A), all.end());
+  }
   dev_free(A->ctx, A->base, A->bytes);
   delete A;
   return KRANS_OK;
@@ -1288,7 +1307,14 @@ int krans_spmv_ex(const krans_mat *A, int trans, int precision, const krans_vec 
   KR_CHECK_ARG(precision != KRANS_PREC_MIXED || A->v32,
                "krans_spmv: matrix has no FP32 values (create with KRANS_CSR_FP32)");
   krans_ctx *c = A->ctx;
-  KR_CUDA(spmv_launch(spmv_operand(A, trans), precision == KRANS_PREC_MIXED, x->d, y->d, c->sms, c->stream));
+  const auto cut = trans ? hold_cut(A) : nullptr;
+  if (cut && !cut->captured) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    KR_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone)
+      cut->captured = true;
+  }
+  KR_CUDA(spmv_launch(spmv_operand(A, trans, cut.get()), precision == KRANS_PREC_MIXED, x->d, y->d, c->sms, c->stream));
   return KRANS_OK;
 }
 

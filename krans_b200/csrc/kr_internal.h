@@ -73,6 +73,8 @@ struct krans_ctx {
   char *ws = nullptr;
   size_t ws_bytes = 0;
   bool ws_busy = false;
+  std::mutex copies_mu;
+  std::vector<krans_mat *> copied; // matrices with second copies
   // blocks of a single solve's cluster: cyclic FP64, cyclic mixed, LOBPCG (-1: not asked yet; under mu)
   int solo_cluster[3] = {-1, -1, -1};
 };
@@ -93,13 +95,17 @@ struct SpmvParts {
 // A and A^T that the solvers read, or A^T cut by columns. A matrix does without
 // where there is no room, and in a context with a budget, which is for what the
 // callers ask for (a planted FP64 matrix takes 20 bytes an entry, and 47 with its
-// slices).
+// slices). Where a later allocation finds no room, the copies that nothing uses go
+// back to the device. What launches work with a copy holds it (hold_slices, hold_cut),
+// from when its own memory is allocated until its kernels are done, or queued on
+// the context's stream.
 struct SpeedCopy {
   krans_ctx *ctx = nullptr;
   char *base = nullptr;
   size_t bytes = 0;
   SlicedView sl{}, slT{}; // slices = 0: that operand has none
   SpmvParts cut;          // parts = 0: not cut
+  std::atomic<bool> captured{false}; // a graph may replay launches that read it: it stays with its matrix
   ~SpeedCopy();           // frees it in the order of the context's stream
 };
 } // namespace kr
@@ -113,8 +119,9 @@ struct krans_mat {
   int lanes = 1, lanesT = 1;
   int32_t ulen = 0, ulenT = 0; // uniform row length of A / A^T (0 = not uniform)
   krans_spmv_tuning tune{}, tuneT{}; // standalone SpMV kernel of A / A^T (zero: automatic)
-  std::unique_ptr<kr::SpeedCopy> slices; // sorted slices of A / A^T for the solvers
-  std::unique_ptr<kr::SpeedCopy> cut;    // A^T cut by columns, where its x is larger than L2
+  // under the context's copies_mu:
+  std::shared_ptr<kr::SpeedCopy> slices; // sorted slices of A / A^T for the solvers
+  std::shared_ptr<kr::SpeedCopy> cut;    // A^T cut by columns, where its x is larger than L2
   char *base = nullptr;         // one device allocation holding every stored array
   size_t bytes = 0;
 };
@@ -144,9 +151,9 @@ struct SpmvOperand {
   krans_spmv_tuning tune;
   const SpmvParts *cut; // or nullptr
 };
-inline SpmvOperand spmv_operand(const krans_mat *A, int trans) {
+inline SpmvOperand spmv_operand(const krans_mat *A, int trans, const SpeedCopy *cut) {
   return trans ? SpmvOperand{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, A->lanesT, A->ulenT, A->tuneT,
-                             A->cut ? &A->cut->cut : nullptr}
+                             cut ? &cut->cut : nullptr}
                : SpmvOperand{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, A->lanes, A->ulen, A->tune, nullptr};
 }
 // y = op x on `s` (kr_spmv.cu); fp32: FP32 values and sums
@@ -226,13 +233,22 @@ constexpr int64_t kSoloLobpcgClusterMin = 4000, kSoloLobpcgGridMin = 40000;
 constexpr int64_t kServedGridMin = 120000;
 // live servers of this process on a device
 std::atomic<int> &device_servers(int device);
-// A (or its stored transpose) as the solvers' device code sees it
-inline CsrView csr_view(const krans_mat *A, bool trans) {
+// the copies as they are now, or nullptr
+inline std::shared_ptr<SpeedCopy> hold_slices(const krans_mat *A) {
+  std::lock_guard<std::mutex> lk(A->ctx->copies_mu);
+  return A->slices;
+}
+inline std::shared_ptr<SpeedCopy> hold_cut(const krans_mat *A) {
+  std::lock_guard<std::mutex> lk(A->ctx->copies_mu);
+  return A->cut;
+}
+// A (or its stored transpose) as the solvers' device code sees it; `slices` as held
+inline CsrView csr_view(const krans_mat *A, bool trans, const SpeedCopy *slices) {
   const SlicedView none{};
   if (trans)
     return CsrView{A->n, A->m, A->nnz, A->rpT, A->ciT, A->vT, A->vT32, tuned_lanes(A->ctx, A->n, A->nnz), A->ulenT,
-                   A->slices ? A->slices->slT : none};
+                   slices ? slices->slT : none};
   return CsrView{A->m, A->n, A->nnz, A->rp, A->ci, A->v, A->v32, tuned_lanes(A->ctx, A->m, A->nnz), A->ulen,
-                 A->slices ? A->slices->sl : none};
+                 slices ? slices->sl : none};
 }
 } // namespace kr

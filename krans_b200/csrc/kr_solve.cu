@@ -55,7 +55,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
                       const krans_cyclic_opts &o, const double *init_right, int64_t k_target,
                       int64_t ncv, std::vector<krans_vec *> &found, RunOut *out,
                       const double *prefill = nullptr, int64_t nprefill = 0, double frob_init = 0.0) {
-  const CsrView F = csr_view(A, trans), B = csr_view(A, !trans);
+  const int64_t rows = trans ? A->n : A->m, cols = trans ? A->m : A->n;
   const bool mixed = o.precision == KRANS_PREC_MIXED;
   if (mixed && !A->v32) {
     set_error("mixed precision needs a matrix created with KRANS_CSR_FP32");
@@ -68,7 +68,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
                "cyclic: precond_aat must be a KRANS_PRECOND_* value, precond_steps in [1, 1000]");
   int team = o.team, csize = 0; // csize: blocks of a cluster team, else 0
   if (team == KRANS_TEAM_AUTO) {
-    const int64_t size = F.rows + F.cols;
+    const int64_t size = rows + cols;
     const bool served = device_servers(ctx->device).load() > 0;
     if (!served && size >= kSoloClusterMin && size < kSoloGridMin) {
       if (ctx->solo_cluster[mixed] < 0)
@@ -81,8 +81,8 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
   const int threads = 512;
   CyclicPlan p;
   memset(&p, 0, sizeof p);
-  p.m = F.rows;
-  p.n = F.cols;
+  p.m = rows;
+  p.n = cols;
   p.k_target = k_target;
   p.ncv = ncv;
   p.ldn = round_up(p.n, 32);
@@ -119,6 +119,8 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
   if (rc != KRANS_OK)
     return rc;
   layout((char *)ws.p);
+  auto slices = hold_slices(A); // until the kernel is done
+  const CsrView F = csr_view(A, trans, slices.get()), B = csr_view(A, !trans, slices.get());
   cudaStream_t s = ctx->stream;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -186,6 +188,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
     e = cudaMemcpyAsync(&out->r, d_res, sizeof(CyclicDevResult), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(s);
+  slices.reset();
   float ms = 0.f;
   if (e == cudaSuccess)
     cudaEventElapsedTime(&ms, e0, e1);

@@ -200,8 +200,6 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
 
   LobpcgDesc d;
   memset(&d, 0, sizeof d);
-  d.F = csr_view(A, false);
-  d.B = csr_view(A, true);
   d.o = o;
   d.k_target = k_target;
   d.bs = bs;
@@ -213,6 +211,9 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
   int rc = ws_take(ctx, bytes, &ws);
   if (rc != KRANS_OK)
     return rc;
+  auto slices = hold_slices(A); // until the kernel is done
+  d.F = csr_view(A, false, slices.get());
+  d.B = csr_view(A, true, slices.get());
   double **d_init = nullptr;
   std::vector<double *> hinit;
   for (int64_t i = 0; i < n_initial; i++)
@@ -254,6 +255,7 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
     e = cudaMemcpyAsync(&R, d.res, sizeof R, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(s);
+  slices.reset();
   float ms = 0.f;
   if (e == cudaSuccess)
     cudaEventElapsedTime(&ms, e0, e1);
@@ -338,6 +340,7 @@ cudaError_t launch_basis_max_residual(const CsrView &F, const double *basis, int
 
 struct LobpcgAsync {
   krans_ctx *ctx = nullptr;
+  std::shared_ptr<SpeedCopy> slices; // until the request is released, its kernels done
   krans_request req;
   LobpcgDesc d;
   int64_t m = 0, n = 0, k_target = 0, bs = 0, pmax = 0;
@@ -424,8 +427,6 @@ int lobpcg_async_plan(krans_ctx *ctx, const krans_request &r, LobpcgAsync **out,
   a->ncta = cluster ? std::min(4, std::max(2, ctx->tune.cluster_size)) : 1;
   LobpcgDesc &d = a->d;
   memset(&d, 0, sizeof d);
-  d.F = csr_view(A, false);
-  d.B = csr_view(A, true);
   d.o = o;
   d.o.team = cluster ? KRANS_TEAM_GRID : KRANS_TEAM_CTA; // informational only
   d.k_target = k_target;
@@ -449,6 +450,9 @@ int lobpcg_async_launch(LobpcgAsync *a, cudaStream_t s) {
   a->stream = s;
   char *p = a->ws;
   LobpcgDesc &d = a->d;
+  a->slices = hold_slices(a->req.A);
+  d.F = csr_view(a->req.A, false, a->slices.get());
+  d.B = csr_view(a->req.A, true, a->slices.get());
   d.rng = nullptr;
   lobpcg_layout(a->m, a->n, a->bs, a->k_target, a->pmax, a->ncta, p, &d);
   p += kr_round_up((int64_t)a->layout_bytes, 256);
