@@ -648,23 +648,53 @@ void preload_capi_kernels() {
     preload(k);
 }
 
-// Room of an operand's sorted slices. A slice is as wide as its longest row;
-// within a window sorted by length, every slice after the first is no wider
-// than the shortest row before it, so the padding of a window is at most 32
-// times its longest row.
-struct SliceSize {
-  int32_t longest = 0;
-  int64_t window_max = 0, sum_max = 0;
-  void row(int64_t i, int32_t len) {
-    if (i % kSliceWindow == 0) {
-      sum_max += window_max;
-      window_max = 0;
-    }
-    window_max = std::max<int64_t>(window_max, len);
-    longest = std::max(longest, len);
+// Whether an operand of `rows` rows keeps sorted slices, and how many entries
+// these hold, padding included (0: none). longest: of its rows; ulen: their
+// length if they are all equal, else 0; len(i): length of row i. An upper bound
+// within twice the entries may stand for the number.
+// Rows of one entry gain nothing (one load in flight per lane: 5400 of them on one
+// block 12.6 us a product, 9.6 with vector loads and four rows in flight), and rows
+// of exactly 2 are read with vector loads as they are; rows of fewer than 2 on
+// average still gain (the transpose of a shift operator: a CG iteration at 4000
+// columns 12.8 -> 10.9 us, at 100000 36 -> 29 us). Padding is read by every product
+// and takes memory: at most 7 entries for each real one (one row of 64 among 256
+// rows of one makes 6: 11.6 us a product on the whole GPU, 25 with lanes).
+template <class Len>
+static int64_t slice_entries(int64_t rows, int64_t nnz, int32_t longest, int32_t ulen, Len len) {
+  if (nnz == 0 || longest < 2 || longest > kSliceMaxLen || ulen == 2)
+    return 0;
+  if (ulen)
+    return (rows + 31) / 32 * 32 * ulen;
+  // Every slice of a window but the first is no wider than the shortest row before
+  // it, so the padding of a window is at most 32 times its longest row. Where that is
+  // close enough it is taken: counting lengths costs 1 ns a row (a creation with 200003
+  // columns takes 3.6 ms).
+  int64_t most = nnz;
+  for (int64_t w0 = 0; w0 < rows; w0 += kSliceWindow) {
+    const int64_t w1 = std::min<int64_t>(rows, w0 + kSliceWindow);
+    int32_t top = 0;
+    for (int64_t i = w0; i < w1; i++)
+      top = std::max(top, len(i));
+    most += 32 * (int64_t)top;
   }
-  int64_t padding() const { return 32 * (sum_max + window_max); }
-};
+  if (most <= 2 * nnz)
+    return most;
+  // a slice is as wide as the row it starts at, in the order of slice_sort_kernel
+  int64_t e = 0;
+  for (int64_t w0 = 0; w0 < rows; w0 += kSliceWindow) {
+    int32_t of_len[2][kSliceMaxLen + 1] = {}; // two counters a length: rows in turn, shorter chains
+    const int64_t w1 = std::min<int64_t>(rows, w0 + kSliceWindow);
+    for (int64_t i = w0; i < w1; i++)
+      of_len[i & 1][len(i)]++;
+    int32_t before = 0; // longer rows
+    for (int32_t l = longest; l > 0; l--) {
+      const int32_t after = before + of_len[0][l] + of_len[1][l];
+      e += 32 * (int64_t)l * ((after + 31) / 32 - (before + 31) / 32);
+      before = after;
+    }
+  }
+  return e <= 8 * nnz ? e : 0;
+}
 
 static int grid_for(krans_ctx *ctx, int64_t n, int threads = 256) {
   int64_t b = (n + threads - 1) / threads;
@@ -902,7 +932,9 @@ static void cut_transpose(krans_ctx *ctx, krans_mat *A, int32_t *cnt) {
   SpmvParts P;
   const int64_t rows = A->n, cols = A->m, nnz = A->nnz;
   P.parts = (int)std::min<int64_t>(kMaxParts, (cols + kPartCols - 1) / kPartCols);
-  if (cols < kCutCols || nnz < rows * P.parts) // fewer than an entry a row and part: y would cost more than x
+  // fewer than an entry a row and part: y would cost more than x; parts as wide as
+  // kCutCols: their pieces of x outgrow L2 too
+  if (cols < kCutCols || cols >= P.parts * kCutCols || nnz < rows * P.parts)
     return;
   Carver lay;
   auto carve = [&](Carver &c) {
@@ -946,12 +978,12 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   // columns (range, per-column counts for the transpose's uniform length)
   const int64_t L = m > 0 ? (int64_t)(row_ptr[1] - row_ptr[0]) : 0;
   bool uni = m > 0 && L > 0 && L <= 8;
-  SliceSize szA, szT; // room that sorted slices of A and of its transpose take
+  int32_t longest = 0, longestT = 0;
   for (int64_t i = 0; i < m; i++) {
     const int32_t len = row_ptr[i + 1] - row_ptr[i];
     KR_CHECK_ARG(len >= 0, "krans_csr_create: row_ptr not monotone");
     uni = uni && len == L;
-    szA.row(i, len);
+    longest = std::max(longest, len);
   }
   std::vector<int32_t> cc((size_t)n, 0);
   for (int64_t k = 0; k < nnz; k++) {
@@ -963,7 +995,7 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   bool uniT = n > 0 && LT > 0 && LT <= 8;
   for (int64_t j = 0; j < n; j++) {
     uniT = uniT && cc[(size_t)j] == LT;
-    szT.row(j, cc[(size_t)j]);
+    longestT = std::max(longestT, cc[(size_t)j]);
   }
   if (!(flags & (KRANS_CSR_FP64 | KRANS_CSR_FP32)))
     flags |= KRANS_CSR_FP64;
@@ -974,11 +1006,9 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
   const size_t sz_v = (size_t)std::max<int64_t>(nnz, 1) * 8, sz_v32 = (size_t)std::max<int64_t>(nnz, 1) * 4;
   // the stored arrays share one allocation (carved at 256-byte offsets)
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  // rows of exactly 2 entries are read with vector loads as they are; rows of
-  // fewer on average (the transpose of a shift operator) still gain from slices
-  // (a CG iteration at 4000 columns 12.8 -> 10.9 us, at 100000 36 -> 29 us)
-  const bool sl = nnz > 0 && !(uni && L == 2) && szA.longest <= kSliceMaxLen;
-  const bool slT = nnz > 0 && !(uniT && LT == 2) && szT.longest <= kSliceMaxLen;
+  const int64_t sl = slice_entries(m, nnz, longest, uni ? (int32_t)L : 0,
+                                   [&](int64_t i) { return row_ptr[i + 1] - row_ptr[i]; });
+  const int64_t slT = slice_entries(n, nnz, longestT, uniT ? LT : 0, [&](int64_t j) { return cc[(size_t)j]; });
   const size_t total = up(sz_rp) + 2 * up(sz_ci) + 2 * up(sz_v) + up(sz_rpT) + (f32 ? 2 * up(sz_v32) : 0);
   char *base = nullptr;
   int rc = dev_alloc(ctx, (void **)&base, total);
@@ -1008,10 +1038,11 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
     A->vT32 = (float *)take(sz_v32);
   }
   // the slices of both operands, in an allocation of their own
-  auto carve_slices = [&](Carver &c, int64_t rows, const SliceSize &z) {
-    const int64_t nsl = (rows + 31) / 32, e = nnz + z.padding();
+  auto carve_slices = [&](Carver &c, int64_t rows, int64_t e, int32_t longest_row) {
+    const int64_t nsl = (rows + 31) / 32;
     SlicedView S;
     S.slices = (int32_t)nsl;
+    S.longest = longest_row;
     S.row = c.take<int32_t>(nsl * 32);
     S.off = c.take<int32_t>(nsl + 1);
     S.ci = c.take<int32_t>(e);
@@ -1023,9 +1054,9 @@ int krans_csr_create(krans_ctx *ctx, int64_t m, int64_t n, int64_t nnz, const in
     SlicedView S{}, ST{};
     auto carve = [&](Carver &c) {
       if (sl)
-        S = carve_slices(c, m, szA);
+        S = carve_slices(c, m, sl, longest);
       if (slT)
-        ST = carve_slices(c, n, szT);
+        ST = carve_slices(c, n, slT, longestT);
     };
     Carver lay;
     carve(lay);

@@ -539,12 +539,14 @@ template <> struct AccOf<float> { using T = float; };
 KR_DEV double2 ldg2(const double *a) { return __ldg(reinterpret_cast<const double2 *>(a)); }
 KR_DEV float2 ldg2(const float *a) { return __ldg(reinterpret_cast<const float2 *>(a)); }
 
-// Thread-per-row SpMV for matrices whose rows all hold exactly 2 entries
-// (incidence, shift and difference operators): no row pointers, vector loads
-// of the (column, value) pairs. `pre` as in csr_mv_pre below.
-template <class Team, class VT, class GX, class Pre, class Epi>
-KR_DEV void team_spmv_uniform2(Team &tm, int64_t rows, const int32_t *__restrict__ ci,
-                               const VT *__restrict__ val, GX gx, Pre pre, Epi epi) {
+// Thread-per-row SpMV for matrices whose rows all hold exactly L = 1 or 2 entries
+// (selections; incidence, shift and difference operators): no row pointers,
+// vector loads of the (column, value) pairs, R rows in flight per thread. `pre`
+// as in csr_mv_pre below.
+template <int L, class Team, class VT, class GX, class Pre, class Epi>
+KR_DEV void team_spmv_uniform(Team &tm, int64_t rows, const int32_t *__restrict__ ci,
+                              const VT *__restrict__ val, GX gx, Pre pre, Epi epi) {
+  static_assert(L == 1 || L == 2, "one or two entries");
   using Acc = typename AccOf<VT>::T;
   using XT = decltype(gx(0));
   using PT = decltype(pre(int64_t(0)));
@@ -552,28 +554,37 @@ KR_DEV void team_spmv_uniform2(Team &tm, int64_t rows, const int32_t *__restrict
   const int64_t nt = tm.nthreads();
   for (int64_t i0 = tm.tid(); i0 < rows; i0 += (int64_t)R * nt) {
     // rows past the end read the last row, so that all loads are unconditional
-    int2 c[R];
-    VT v0[R], v1[R];
+    int32_t c[R][L];
+    VT v[R][L];
     PT pv[R];
 #pragma unroll
     for (int u = 0; u < R; u++) {
       const int64_t i = imin64(i0 + (int64_t)u * nt, rows - 1);
-      c[u] = __ldg(reinterpret_cast<const int2 *>(ci) + i);
-      const auto vv = ldg2(val + 2 * i);
-      v0[u] = vv.x;
-      v1[u] = vv.y;
+      if constexpr (L == 2) {
+        const int2 cc = __ldg(reinterpret_cast<const int2 *>(ci) + i);
+        const auto vv = ldg2(val + 2 * i);
+        c[u][0] = cc.x;
+        c[u][1] = cc.y;
+        v[u][0] = vv.x;
+        v[u][1] = vv.y;
+      } else {
+        c[u][0] = __ldg(ci + i);
+        v[u][0] = __ldg(val + i);
+      }
       pv[u] = pre(i);
     }
-    XT x0[R], x1[R];
+    XT x[R][L];
 #pragma unroll
-    for (int u = 0; u < R; u++) {
-      x0[u] = gx(c[u].x);
-      x1[u] = gx(c[u].y);
-    }
+    for (int u = 0; u < R; u++)
+#pragma unroll
+      for (int j = 0; j < L; j++)
+        x[u][j] = gx(c[u][j]);
 #pragma unroll
     for (int u = 0; u < R; u++) {
       const int64_t i = i0 + (int64_t)u * nt;
-      const Acc s = (Acc)v0[u] * (Acc)x0[u] + (Acc)v1[u] * (Acc)x1[u];
+      Acc s = (Acc)v[u][0] * (Acc)x[u][0];
+      if constexpr (L == 2)
+        s += (Acc)v[u][1] * (Acc)x[u][1];
       if (i < rows)
         epi(i, s, pv[u]);
     }
@@ -760,21 +771,38 @@ template <class VT> KR_DEV const VT *sliced_values(const SlicedView &S) {
     return S.v32;
 }
 
+// Whether a team reads an operand by its slices. Few slices of long rows leave
+// most warps of a wide team idle, where several lanes a row would use them (us a
+// product, slices / lanes: 5400 rows of 1 to 64 entries on the whole GPU 15.1 / 14.3,
+// on 16 blocks 12.3 / 16.8; 1500 rows of 48 on 16 blocks 16.9 / 15.0; 27000 rows of
+// 64 on the whole GPU 20.2 / 22.6; 5400 rows of 16 there 11.5 / 14.8). Rows of about
+// one entry leave a lane one load in flight, and one block has few warps to hide it
+// (a product and its transpose with 5400 entries, 6000 columns: 11.4 / 9.4 on one
+// block, 5.0 / 6.0 on 16).
+template <class Team> KR_DEV bool by_slices(const Team &tm, const CsrView &V) {
+  const int64_t nw = tm.nwarps();
+  if (!V.sl.slices || (V.lanes >= 16 && 4 * (int64_t)V.sl.slices < nw))
+    return false;
+  return nw > KR_MAX_WARPS || V.sl.longest > 8 || 2 * V.nnz >= 3 * V.rows;
+}
+
 // y = V x with VT values, gather gx(col), prologue pre(row, slot) and epilogue
-// epi(row, slot, sum, prologue's value). Rows of exactly 2 entries: vector
-// loads, no row pointers; operands with sorted slices: those; else `lanes`
-// threads per row (slot = row in both).
+// epi(row, slot, sum, prologue's value). Operands with sorted slices: those (see
+// by_slices); rows of exactly 1 or 2 entries: vector loads, no row pointers; else
+// `lanes` threads per row (slot = row in both).
 template <class VT, class Team, class GX, class Pre, class Epi>
 KR_DEV void csr_mv_pre(Team &tm, const CsrView &V, GX gx, Pre pre, Epi epi) {
   using Acc = typename AccOf<VT>::T;
-  if (V.sl.slices) {
+  if (by_slices(tm, V)) {
     team_spmv_sliced(tm, V.sl, sliced_values<VT>(V.sl), gx, pre, epi);
     return;
   }
   auto pre1 = [&](int64_t i) { return pre((int)i, (int)i); };
   auto epi1 = [&](int64_t i, Acc s, decltype(pre(0, 0)) p) { epi((int)i, (int)i, s, p); };
   if (V.ulen == 2)
-    team_spmv_uniform2(tm, V.rows, V.ci, csr_values<VT>(V), gx, pre1, epi1);
+    team_spmv_uniform<2>(tm, V.rows, V.ci, csr_values<VT>(V), gx, pre1, epi1);
+  else if (V.ulen == 1)
+    team_spmv_uniform<1>(tm, V.rows, V.ci, csr_values<VT>(V), gx, pre1, epi1);
   else
     team_spmv_lanes(tm, V.rows, V.rp, V.ci, csr_values<VT>(V), gx, V.lanes, pre1, epi1);
 }

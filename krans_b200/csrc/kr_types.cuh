@@ -44,7 +44,8 @@ struct RngState {
 // + 31, and round r (off[s] <= r < off[s + 1]) holds one entry of each of its
 // rows at 32 r + lane (column 0, value 0 where the row has ended).
 struct SlicedView {
-  int32_t slices; // 0: this operand has none
+  int32_t slices;  // 0: this operand has none
+  int32_t longest; // row
   const int32_t *off, *row, *ci;
   const double *v64;
   const float *v32;

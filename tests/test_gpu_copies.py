@@ -45,3 +45,21 @@ def test_slices_go_back_when_the_device_is_full():
     del hold
     torch.cuda.empty_cache()
     assert frob() == pytest.approx(want, rel=1e-12)
+
+
+def test_slices_without_more_than_seven_padded_entries_for_each_real_one():
+    """One row of 64 entries among 255 empty ones: its slice would be 31 / 32 padding."""
+    import krans_b200 as kb
+    r = np.random.default_rng(4)
+    m, n = 2560, 3500
+    lens = np.where(np.arange(m) % 256 == 7, 64, 0)
+    ip = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    A = sp.csr_matrix((r.standard_normal(ip[-1]), r.integers(0, n, ip[-1]).astype(np.int32), ip), shape=(m, n))
+    ctx = kb.Context(0)
+    before = ctx.memory_in_use()
+    M = kb.CudaCsrMatrixAdapter.from_scipy(ctx, A)
+    plain = sum((b + 255) // 256 * 256 for b in (4 * (m + 1), 4 * (n + 1)) + 2 * (4 * A.nnz, 8 * A.nnz))
+    scratch = 1 << 20  # the context keeps at least as much after a creation
+    # at most 8 entries of 12 bytes in a slice for each one, a row number a slot and a bound a slice, of both operands
+    assert ctx.memory_in_use() - before - plain - scratch <= 2 * 8 * 12 * A.nnz + 5 * (m + n) + 4096
+    del M
