@@ -433,9 +433,13 @@ __host__ __device__ constexpr size_t gemm_nn_smem_bytes() {
 // sums over k in order on the CUDA cores, with no shared memory and no
 // barrier. For the few-column blocks of small solves the tiled form spends
 // two block barriers per 64-row tile on a 64 x 128 output group it barely
-// fills; this form costs none (the caller's barrier publishes the result).
+// fills; this form costs none (the caller's barrier publishes the result). Bound
+// by the latency of a row's loads: those of U = 8 k are issued together in the
+// kernel of its own (36 x 12 at n = 20011: 33.9 -> 18.5 us, at n = 1000003 221 ->
+// 183), one k at a time inside the solver, whose registers are short (eight: 3%
+// slower solves at 4 and 6 columns, 3% faster at 16).
 #define KR_NQ_DIRECT 16
-template <class Team>
+template <int U, class Team>
 KR_DEV void team_gemm_nn_direct(Team &tm, int64_t n, const double *Z, int64_t ld, int zc, const double *Y, int ldy,
                                 int roff, int q, double *out, bool subtract) {
   for (int64_t i = tm.tid(); i < n; i += tm.nthreads()) {
@@ -443,7 +447,22 @@ KR_DEV void team_gemm_nn_direct(Team &tm, int64_t n, const double *Z, int64_t ld
 #pragma unroll
     for (int j = 0; j < KR_NQ_DIRECT; j++)
       acc[j] = 0.0;
-    for (int k = 0; k < zc; k++) {
+    int k = 0;
+    for (; k + U <= zc; k += U) {
+      double z[U];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        z[u] = Z[(int64_t)(k + u) * ld + i];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const double *yk = Y + roff + k + u;
+#pragma unroll
+        for (int j = 0; j < KR_NQ_DIRECT; j++)
+          if (j < q)
+            acc[j] += z[u] * yk[(int64_t)j * ldy];
+      }
+    }
+    for (; k < zc; k++) {
       const double z = Z[(int64_t)k * ld + i];
       const double *yk = Y + roff + k;
 #pragma unroll
@@ -464,7 +483,7 @@ template <class Team>
 KR_DEV void team_gemm_nn(Team &tm, int64_t n, const double *Z, int64_t ld, int zc, const double *Y, int ldy,
                          int roff, int q, double *out, bool subtract) {
   if (q <= KR_NQ_DIRECT) {
-    team_gemm_nn_direct(tm, n, Z, ld, zc, Y, ldy, roff, q, out, subtract);
+    team_gemm_nn_direct<1>(tm, n, Z, ld, zc, Y, ldy, roff, q, out, subtract);
     return;
   }
   extern __shared__ __align__(16) double kr_gemm_smem[];

@@ -26,12 +26,18 @@ __global__ void __launch_bounds__(512) block_gemm_tn_kernel(int64_t n, const dou
   team_gemm_tn(tm, n, A, a, B, b, ld, C, part);
 }
 
+// narrow: the form for few output columns alone, a kernel of its own because it
+// wants more registers than let two blocks of the tiled form onto an SM
+template <bool NARROW>
 __global__ void __launch_bounds__(512) block_combine_kernel(int64_t n, const double *Z, int64_t ld, int zc,
                                                             const double *C, int ldc, int q, double *out,
                                                             GridBarrierState *gb, double *gpart, int *status) {
   __shared__ TeamShared sh;
   TeamGrid tm{&sh, status, gb, gpart, 0, 0};
-  team_gemm_nn(tm, n, Z, ld, zc, C, ldc, 0, q, out, false);
+  if constexpr (NARROW)
+    team_gemm_nn_direct<8>(tm, n, Z, ld, zc, C, ldc, 0, q, out, false);
+  else
+    team_gemm_nn(tm, n, Z, ld, zc, C, ldc, 0, q, out, false);
 }
 
 static int coop_blocks(const void *k, krans_ctx *ctx, size_t smem) {
@@ -67,7 +73,8 @@ static int coop_scratch(krans_ctx *ctx, int blocks, size_t part_doubles, WsHold 
 void preload_gram_kernels() {
   preload((const void *)block_gram_kernel);
   preload((const void *)block_gemm_tn_kernel);
-  preload((const void *)block_combine_kernel);
+  preload((const void *)block_combine_kernel<true>);
+  preload((const void *)block_combine_kernel<false>);
 }
 
 } // namespace kr
@@ -192,8 +199,10 @@ extern "C" int krans_block_combine(krans_ctx *ctx, int64_t n, int64_t zc, int64_
                "krans_block_combine: need n >= 0, 1 <= zc, q <= 4096, ld >= n, ldc >= zc");
   KR_CUDA(cudaSetDevice(ctx->device));
   std::lock_guard<std::mutex> lk(ctx->mu);
-  const void *k = (const void *)block_combine_kernel;
-  const int blocks = coop_blocks(k, ctx, gemm_nn_smem_bytes());
+  const bool narrow = q <= KR_NQ_DIRECT;
+  const void *k = narrow ? (const void *)block_combine_kernel<true> : (const void *)block_combine_kernel<false>;
+  const size_t smem = narrow ? 0 : gemm_nn_smem_bytes();
+  const int blocks = coop_blocks(k, ctx, smem);
   WsHold ws;
   GridBarrierState *gb;
   double *gpart, *pt;
@@ -209,7 +218,7 @@ extern "C" int krans_block_combine(krans_ctx *ctx, int64_t n, int64_t zc, int64_
   void *args[] = {(void *)&n, (void *)&Z, (void *)&ld, (void *)&zci, (void *)&C, (void *)&ldci, (void *)&qi,
                   (void *)&out, (void *)&gb, (void *)&gpart, (void *)&status};
   if (e == cudaSuccess)
-    e = timed_coop(k, blocks, args, gemm_nn_smem_bytes(), s, device_ms);
+    e = timed_coop(k, blocks, args, smem, s, device_ms);
   ws_give(ctx, &ws);
   if (e != cudaSuccess)
     return cuda_fail(e, "krans_block_combine", __FILE__, __LINE__);
