@@ -36,7 +36,7 @@ static void release_bytes(krans_ctx *ctx, size_t bytes) {
   }
 }
 
-static bool over_budget(krans_ctx *ctx, size_t bytes) {
+bool over_budget(const krans_ctx *ctx, size_t bytes) {
   return ctx->budget && ctx->in_use.load() + bytes > ctx->budget;
 }
 static int budget_fail(krans_ctx *ctx, size_t bytes) {

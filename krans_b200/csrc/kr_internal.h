@@ -160,6 +160,7 @@ inline SpmvOperand spmv_operand(const krans_mat *A, int trans, const SpeedCopy *
 cudaError_t spmv_launch(const SpmvOperand &A, bool fp32, const double *x, double *y, int sms, cudaStream_t s);
 int spmv_rows_per_block(int64_t rows, int64_t nnz);
 // allocation with budget accounting
+bool over_budget(const krans_ctx *ctx, size_t bytes); // these on top of what is allocated
 int dev_alloc(krans_ctx *ctx, void **p, size_t bytes);
 void dev_free(krans_ctx *ctx, void *p, size_t bytes);
 // Scratch of one call on the context's stream, kept from call to call: a

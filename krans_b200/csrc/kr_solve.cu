@@ -77,7 +77,7 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
     }
     team = size < (served ? kServedGridMin : kSoloGridMin) ? KRANS_TEAM_CTA : KRANS_TEAM_GRID;
   }
-  const bool grid = team == KRANS_TEAM_GRID;
+  bool grid = team == KRANS_TEAM_GRID;
   const int threads = 512;
   CyclicPlan p;
   memset(&p, 0, sizeof p);
@@ -90,8 +90,6 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
   p.ldb = p.ldn;
   p.cap = ncv / 2 + 2;
   p.ksz = mixed ? 4 : 8;
-  p.grid_blocks = grid ? cyclic_grid_blocks(ctx, mixed, threads) : 1;
-  p.own_basis = grid ? 1 : 0;
   p.block_polish = o.polish_block ? 1 : 0;
   p.precond = o.precond_aat;
   // one allocation: solver workspace, basis, request record and counters
@@ -102,10 +100,12 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
   int32_t *d_status = nullptr;
   int *d_queue = nullptr;
   auto layout = [&](char *base) {
+    p.grid_blocks = grid ? cyclic_grid_blocks(ctx, mixed, threads) : 1;
+    p.own_basis = grid ? 1 : 0;
     Carver c;
     c.base = base;
     slot = c.take<char>((int64_t)cyclic_carve(p, nullptr, nullptr));
-    basis = c.take<double>(std::max<int64_t>(k_target, 1) * p.ldb);
+    basis = c.take<double>(grid ? 1 : std::max<int64_t>(k_target, 1) * p.ldb);
     d_req = c.take<CyclicRequestDev>(1);
     d_res = c.take<CyclicDevResult>(1);
     d_status = c.take<int32_t>(1);
@@ -113,9 +113,16 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
     d_queue = c.take<int>(2);
     return c.off + 256;
   };
-  const size_t bytes = layout(nullptr);
+  // one block needs no room for other blocks' partials, and the basis is still to come
+  const bool smaller = o.team == KRANS_TEAM_AUTO && grid && rows + cols < kServedGridMin;
+  if (smaller && over_budget(ctx, layout(nullptr) + (size_t)(8 * k_target * cols)))
+    grid = false;
   WsHold ws;
-  int rc = ws_take(ctx, bytes, &ws);
+  int rc = ws_take(ctx, layout(nullptr), &ws);
+  if (rc == KRANS_ERR_OUT_OF_MEMORY && smaller && grid) {
+    grid = false;
+    rc = ws_take(ctx, layout(nullptr), &ws);
+  }
   if (rc != KRANS_OK)
     return rc;
   layout((char *)ws.p);

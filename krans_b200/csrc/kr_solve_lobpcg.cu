@@ -87,7 +87,7 @@ static size_t lobpcg_layout(int64_t m, int64_t n, int64_t bs, int64_t k, int64_t
   t.status = c.take<int32_t>(1);
   t.res = c.take<LobpcgDevResult>(1);
   t.gb = c.take<GridBarrierState>(1);
-  t.gpart = c.take<double>(2 * std::max(ncta, 1) * KR_MDOT);
+  t.gpart = c.take<double>(ncta > 1 ? 2 * ncta * KR_MDOT : 1);
   t.flag = c.take<int32_t>(4);
   t.dflag = c.take<double>(4);
   if (d) {
@@ -196,7 +196,7 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
     team = m + n < (served ? kServedGridMin : kSoloLobpcgGridMin) ? KRANS_TEAM_CTA : KRANS_TEAM_GRID;
   }
   const int threads = 512;
-  const int ncta = team == KRANS_TEAM_GRID ? lobpcg_grid_blocks(ctx, threads) : csize ? csize : 1;
+  int ncta = team == KRANS_TEAM_GRID ? lobpcg_grid_blocks(ctx, threads) : csize ? csize : 1;
 
   LobpcgDesc d;
   memset(&d, 0, sizeof d);
@@ -206,9 +206,22 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
   d.guards = guards;
   d.rng = rng->d;
   d.n_initial = n_initial;
-  const size_t bytes = lobpcg_layout(m, n, bs, k_target, pmax, ncta, nullptr, nullptr);
+  auto bytes = [&] { return lobpcg_layout(m, n, bs, k_target, pmax, ncta, nullptr, nullptr); };
+  // one block needs no room for other blocks' partial products, and the basis is still to come
+  const bool smaller = o.team == KRANS_TEAM_AUTO && ncta > 1 && m + n < kServedGridMin;
+  auto one_block = [&] {
+    team = KRANS_TEAM_CTA;
+    csize = 0;
+    ncta = 1;
+  };
+  if (smaller && over_budget(ctx, bytes() + (size_t)(8 * k_target * n)))
+    one_block();
   WsHold ws;
-  int rc = ws_take(ctx, bytes, &ws);
+  int rc = ws_take(ctx, bytes(), &ws);
+  if (rc == KRANS_ERR_OUT_OF_MEMORY && smaller && ncta > 1) {
+    one_block();
+    rc = ws_take(ctx, bytes(), &ws);
+  }
   if (rc != KRANS_OK)
     return rc;
   auto slices = hold_slices(A); // until the kernel is done

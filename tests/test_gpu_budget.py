@@ -67,3 +67,32 @@ def test_creation_without_room_for_slices():
     y = kb.CudaVectorAdapter(ctx, m)
     M.multiply(x, y)
     np.testing.assert_allclose(y.data(), A @ np.ones(n), rtol=1e-12, atol=1e-12)
+
+
+@pytest.mark.parametrize("solver,n", [("lobpcg", 2500), ("lobpcg", 20001), ("cyclic", 50001)])  # cluster, whole GPU
+def test_auto_team_under_the_smallest_budget_of_one_block(solver, n):
+    """KRANS_TEAM_AUTO takes a larger team where there is room for its partial sums, and one block where not."""
+    import krans_b200 as kb
+    inst = G.shift_operator(n, 2, 0.5, kernel=False)
+
+    def runs(budget, team):
+        ctx = kb.Context(0, hbm_budget=budget)
+        try:
+            M = kb.CudaCsrMatrixAdapter.from_scipy(ctx, inst.A)
+            vf = kb.CudaVectorFactory(ctx, n, seed=4)
+            if solver == "lobpcg":
+                kb.find_nullspace_lobpcg(M, vf, kb.LOBPCGOptions(nev=2, block_size=4, max_iters=2, team=team))
+            else:
+                kb.find_nullspace_cyclic_lanczos(M, vf, kb.CyclicLanczosOptions(
+                    k=2, ncv=8, max_restarts=1, cg_maxit=2, grad_max_iters=1, team=team))
+            return True
+        except kb.KransError as e:
+            assert "budget" in str(e)
+            return False
+
+    lo, hi = 0, 256 << 20
+    assert runs(hi, 1)
+    while hi - lo > 4096:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if runs(mid, 1) else (mid, hi)
+    assert runs(hi, 0)
