@@ -439,7 +439,9 @@ template <class Team, class KT> struct CyclicSolver {
   // z = M^-1 r, rz = r.z, p = z, tolerance on sqrt(r.z); otherwise as cg().
   __device__ __noinline__ int64_t cg_pre(const double *rhs, double *u, int64_t maxit, double rel_tol,
                                          double bd_tol, double *rnorm_out) {
-    double *z = d.cgr, *r = d.r_pre, *t = d.cgt, *ts = d.cgts, *us = d.cgus;
+    // the SD steps work in tn too: F^T p is read before the next of them, and the
+    // pass that follows forms it anew from ts
+    double *z = d.cgr, *r = d.r_pre, *t = d.tn, *ts = d.cgts, *us = d.cgus;
     double rr = 0.0;
     team_for(tm, n, [&](int64_t i) { u[i] = 0.0; });
     team_for(tm, m, [&](int64_t i) {

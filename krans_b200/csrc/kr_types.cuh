@@ -95,7 +95,6 @@ struct CyclicDesc {
   double2 *rp;                       // CG with a direction: residual and direction, interleaved (m)
   double *Ap;                        // and F F^T p (m)
   double *r_pre, *dinv, *sd_q, *sd_Oq; // preconditioned CG: residual, Jacobi weights, SD vectors (m)
-  double *cgt;                         // preconditioned CG: F^T p (n; the SD steps work in tn)
   double *alpha, *beta;              // ncv + 2
   double *Tb, *Vt, *sv;              // tiny problem
   int32_t *ord;
@@ -150,10 +149,13 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
   double *y0 = c.take<double>(p.ldn), *v = c.take<double>(p.ldn), *vp = c.take<double>(p.ldn);
   double *best_v = c.take<double>(p.ldn), *tn = c.take<double>(p.ldn);
   double *tmv = c.take<double>(p.ldm), *wm = c.take<double>(p.ldm);
-  double *cgr = c.take<double>(p.ldm);
-  double *cgts = c.take<double>(p.ldn), *cgus = c.take<double>(p.ldn);
-  double2 *rp = c.take<double2>(p.ldm);
-  double *Ap = c.take<double>(p.ldm);
+  // the vectors of the two forms of CG share their place: a call of one keeps
+  // nothing for the other (ldm and ldn are multiples of 32)
+  const int64_t craig = p.ldm + 2 * p.ldn, direction = 3 * p.ldm;
+  double *cgr = c.take<double>(craig > direction ? craig : direction);
+  double *cgts = cgr + p.ldm, *cgus = cgts + p.ldn;
+  double2 *rp = (double2 *)cgr;
+  double *Ap = cgr + 2 * p.ldm;
   double *alpha = c.take<double>(p.ncv + 2), *beta = c.take<double>(p.ncv + 2);
   double *Tb = c.take<double>((p.ncv + 1) * p.ncv), *Vt = c.take<double>(p.ncv * p.ncv);
   double *sv = c.take<double>(p.ncv + 1);
@@ -163,14 +165,13 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
   int32_t *status = c.take<int32_t>(1);
   CyclicDevResult *res = c.take<CyclicDevResult>(1);
   GridBarrierState *gb = c.take<GridBarrierState>(1);
-  double *gpart = c.take<double>(2 * (p.grid_blocks > 1 ? p.grid_blocks : 1) * KR_MDOT);
-  double *r_pre = nullptr, *dinv = nullptr, *sd_q = nullptr, *sd_Oq = nullptr, *cgt = nullptr;
+  double *gpart = c.take<double>(p.grid_blocks > 1 ? 2 * p.grid_blocks * KR_MDOT : 1);
+  double *r_pre = nullptr, *dinv = nullptr, *sd_q = nullptr, *sd_Oq = nullptr;
   if (p.precond) {
     r_pre = c.take<double>(p.ldm);
     dinv = c.take<double>(p.ldm);
     sd_q = c.take<double>(p.ldm);
     sd_Oq = c.take<double>(p.ldm);
-    cgt = c.take<double>(p.ldn);
   }
   double *Vc = nullptr, *Hb = nullptr, *Wb = nullptr, *Rk = nullptr, *Pk = nullptr, *Ak = nullptr, *Tk = nullptr;
   if (p.block_polish) {
@@ -193,7 +194,7 @@ __host__ __device__ inline size_t cyclic_carve(const CyclicPlan &p, char *base, 
     if (p.own_basis) { d->status = status; d->res = res; }
     d->gb = gb; d->gpart = gpart;
     d->Vc = Vc; d->Hb = Hb; d->Wb = Wb; d->Rk = Rk; d->Pk = Pk; d->Ak = Ak; d->Tk = Tk;
-    d->r_pre = r_pre; d->dinv = dinv; d->sd_q = sd_q; d->sd_Oq = sd_Oq; d->cgt = cgt;
+    d->r_pre = r_pre; d->dinv = dinv; d->sd_q = sd_q; d->sd_Oq = sd_Oq;
     d->ldn = p.ldn; d->ldm = p.ldm; d->ldb = p.ldb; d->cap = p.cap;
   }
   return c.off + 256;
