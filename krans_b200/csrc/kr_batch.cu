@@ -277,7 +277,7 @@ struct BatchLaunch {
     // largest small request that fits under the cap
     dyn_smem = 0;
     for (int pos = n_large + n_mid; pos < n; pos++) {
-      const size_t b = cta_cg_smem_bytes(hreq[pos].plan.ldm, hreq[pos].plan.ldn);
+      const size_t b = cta_cg_smem_bytes(hreq[pos].plan, mats[pos]->ulen);
       if (b <= cta_smem_cap())
         dyn_smem = std::max(dyn_smem, b);
     }

@@ -129,9 +129,16 @@ __device__ __noinline__ void run_cta_request(TeamShared *sh, CyclicDesc *dp, con
     // (the solver reaches them through generic pointers)
     uint32_t dyn;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-    if (cta_cg_smem_bytes(rq.plan.ldm, rq.plan.ldn) <= (size_t)dyn) {
-      d.cgr = reinterpret_cast<double *>(kr_dyn_smem);
-      d.tn = reinterpret_cast<double *>(kr_dyn_smem + 8 * rq.plan.ldm);
+    if (cta_cg_smem_bytes(rq.plan, rq.F.ulen) <= (size_t)dyn) {
+      double *sm = reinterpret_cast<double *>(kr_dyn_smem);
+      if (cg_keeps_direction(rq.plan, rq.F.ulen)) {
+        d.rp = reinterpret_cast<double2 *>(sm);
+        d.Ap = sm + 2 * rq.plan.ldm;
+        d.tn = sm + 3 * rq.plan.ldm;
+      } else {
+        d.cgr = sm;
+        d.tn = sm + rq.plan.ldm;
+      }
     }
     rq.res->t_begin = globaltimer_ns();
   }

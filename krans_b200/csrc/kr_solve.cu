@@ -185,8 +185,8 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
         : csize ? launch_cyclic_batch_cluster(mixed, 1, csize, 0, s, d_req, 1, d_queue, slot, 0, nullptr, 0,
                                               d_queue + 1, slot, 0, nullptr, 0)
                 : launch_cyclic_batch_cta(mixed, 1, threads,
-                                       cta_cg_smem_bytes(p.ldm, p.ldn) <= cta_smem_cap()
-                                           ? cta_cg_smem_bytes(p.ldm, p.ldn)
+                                       cta_cg_smem_bytes(p, F.ulen) <= cta_smem_cap()
+                                           ? cta_cg_smem_bytes(p, F.ulen)
                                            : 0,
                                        s, d_req, 1, d_queue, slot, 0, nullptr);
   if (e == cudaSuccess)

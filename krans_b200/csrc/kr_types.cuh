@@ -121,10 +121,14 @@ struct CyclicPlan {
 
 __host__ __device__ inline int64_t kr_round_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 
-// Shared-memory bytes that hold the gathered CG vectors of a one-block solve
-// (residual r, F^T p): 8 ldm + 8 ldn.
-__host__ __device__ inline size_t cta_cg_smem_bytes(int64_t ldm, int64_t ldn) {
-  return (size_t)(8 * ldm + 8 * ldn);
+// Shared-memory bytes that hold the gathered CG vectors of a one-block solve: the
+// residual and F^T p (8 ldm + 8 ldn), or, where CG keeps its direction (see
+// CyclicSolver::cg), residual and direction, F F^T p and F^T p (24 ldm + 8 ldn).
+__host__ __device__ inline bool cg_keeps_direction(const CyclicPlan &p, int32_t ulen) {
+  return ulen != 2 && p.precond == KRANS_PRECOND_NONE;
+}
+__host__ __device__ inline size_t cta_cg_smem_bytes(const CyclicPlan &p, int32_t ulen) {
+  return (size_t)((cg_keeps_direction(p, ulen) ? 24 : 8) * p.ldm + 8 * p.ldn);
 }
 
 struct Carver {
