@@ -306,7 +306,11 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
     set_error("%s", lobpcg_err_msg(R.err_code));
     return KRANS_ERR_RUNTIME;
   }
-  KR_CHECK_ARG(right_out || R.n_right == 0, "krans_solve_lobpcg: right_out is NULL");
+  if (!right_out && R.n_right > 0) {
+    ws_give(ctx, &ws);
+    set_error("krans_solve_lobpcg: right_out is NULL");
+    return KRANS_ERR_INVALID_ARGUMENT;
+  }
   std::vector<double> th((size_t)std::max<int64_t>(R.n_right, 1)), rs((size_t)std::max<int64_t>(R.n_right, 1));
   if (R.n_right > 0) {
     e = cudaMemcpyAsync(th.data(), d.theta_out, 8 * (size_t)R.n_right, cudaMemcpyDeviceToHost, s);

@@ -96,3 +96,20 @@ def test_auto_team_under_the_smallest_budget_of_one_block(solver, n):
         mid = (lo + hi) // 2
         lo, hi = (lo, mid) if runs(mid, 1) else (mid, hi)
     assert runs(hi, 0)
+
+
+def test_workspace_of_a_solve_without_an_output_array():
+    """LOBPCG finds vectors and has nowhere to put them: the error leaves no workspace behind."""
+    import ctypes as C
+    import krans_b200 as kb
+    from krans_b200 import _capi as K
+    n = 1000
+    ctx = kb.Context(0, hbm_budget=64 << 20)
+    M = kb.CudaCsrMatrixAdapter.from_scipy(ctx, G.shift_operator(n, 2, 0.5, kernel=False).A)
+    vf = kb.CudaVectorFactory(ctx, n, seed=4)
+    o = kb.LOBPCGOptions(nev=2, block_size=4, tol_abs=1e-10, tol_rel=0.0).to_c()
+    held = ctx.memory_in_use()
+    rc = ctx.lib.krans_solve_lobpcg(ctx.h, M.h, vf.h, C.byref(o), None, 0, None, None, None,
+                                    C.byref(K.LobpcgResultC()))
+    assert rc == K.KRANS_ERR_INVALID_ARGUMENT
+    assert ctx.memory_in_use() == held
