@@ -112,6 +112,8 @@ __device__ __noinline__ void run_cta_request(TeamShared *sh, CyclicDesc *dp, con
     cyclic_carve(rq.plan, slot, &d);
     d.F = rq.F;
     d.B = rq.B;
+    pick_slices(d.F, blockDim.x / 32);
+    pick_slices(d.B, blockDim.x / 32);
     d.o = rq.o;
     d.k_target = rq.plan.k_target;
     d.ncv = rq.plan.ncv;
@@ -201,6 +203,8 @@ __device__ __noinline__ void run_cluster_request(TeamShared *sh, CyclicDesc *dp,
     cyclic_carve(rq.plan, slot, &d);
     d.F = rq.F;
     d.B = rq.B;
+    pick_slices(d.F, (int64_t)csize * (blockDim.x / 32));
+    pick_slices(d.B, (int64_t)csize * (blockDim.x / 32));
     d.o = rq.o;
     d.k_target = rq.plan.k_target;
     d.ncv = rq.plan.ncv;

@@ -192,7 +192,7 @@ template <class Team, class KT> struct CyclicSolver {
   // u by row; `pending`: with the last iteration's alpha t, which no further
   // first pass applies
   __device__ __noinline__ void cg_result(const double *ts, const double *us, bool pending, double alpha, double *u) {
-    const int32_t *row = by_slices(tm, d.B) ? d.B.sl.row : nullptr;
+    const int32_t *row = d.B.sl.slices ? d.B.sl.row : nullptr;
     team_for(tm, n, [&](int64_t p) { u[row ? row[p] : p] = pending ? us[p] + alpha * ts[p] : us[p]; });
     c.bytes += 24.0 * n;
     tm.sync();

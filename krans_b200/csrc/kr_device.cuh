@@ -6,8 +6,10 @@
 //              one per block, synchronised with __syncthreads).
 //   TeamGrid - every block of a cooperative launch (one large solve on the
 //              whole GPU, synchronised with a bounded grid barrier).
+//   TeamCluster - the blocks of a thread-block cluster (solves in between).
 // All reductions use a fixed tree whose shape depends only on the team size,
-// so a solve gives bit-identical results alone and inside a batch.
+// and a batch picks its teams by m + n alone, so a request gives bit-identical
+// results in any batch. A single solve picks its own team: other rounding.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -771,29 +773,14 @@ template <class VT> KR_DEV const VT *sliced_values(const SlicedView &S) {
     return S.v32;
 }
 
-// Whether a team reads an operand by its slices. Few slices of long rows leave
-// most warps of a wide team idle, where several lanes a row would use them (us a
-// product, slices / lanes: 5400 rows of 1 to 64 entries on the whole GPU 15.1 / 14.3,
-// on 16 blocks 12.3 / 16.8; 1500 rows of 48 on 16 blocks 16.9 / 15.0; 27000 rows of
-// 64 on the whole GPU 20.2 / 22.6; 5400 rows of 16 there 11.5 / 14.8). Rows of about
-// one entry leave a lane one load in flight, and one block has few warps to hide it
-// (a product and its transpose with 5400 entries, 6000 columns: 11.4 / 9.4 on one
-// block, 5.0 / 6.0 on 16).
-template <class Team> KR_DEV bool by_slices(const Team &tm, const CsrView &V) {
-  const int64_t nw = tm.nwarps();
-  if (!V.sl.slices || (V.lanes >= 16 && 4 * (int64_t)V.sl.slices < nw))
-    return false;
-  return nw > KR_MAX_WARPS || V.sl.longest > 8 || 2 * V.nnz >= 3 * V.rows;
-}
-
 // y = V x with VT values, gather gx(col), prologue pre(row, slot) and epilogue
 // epi(row, slot, sum, prologue's value). Operands with sorted slices: those (see
-// by_slices); rows of exactly 1 or 2 entries: vector loads, no row pointers; else
+// pick_slices); rows of exactly 1 or 2 entries: vector loads, no row pointers; else
 // `lanes` threads per row (slot = row in both).
 template <class VT, class Team, class GX, class Pre, class Epi>
 KR_DEV void csr_mv_pre(Team &tm, const CsrView &V, GX gx, Pre pre, Epi epi) {
   using Acc = typename AccOf<VT>::T;
-  if (by_slices(tm, V)) {
+  if (V.sl.slices) {
     team_spmv_sliced(tm, V.sl, sliced_values<VT>(V.sl), gx, pre, epi);
     return;
   }

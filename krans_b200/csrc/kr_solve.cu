@@ -144,6 +144,8 @@ static int run_cyclic(krans_ctx *ctx, const krans_mat *A, bool trans, krans_rng 
     cyclic_carve(p, slot, &d);
     d.F = F;
     d.B = B;
+    pick_slices(d.F, (int64_t)p.grid_blocks * (threads / 32));
+    pick_slices(d.B, (int64_t)p.grid_blocks * (threads / 32));
     d.o = o;
     d.k_target = k_target;
     d.ncv = ncv;

@@ -227,6 +227,8 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
   auto slices = hold_slices(A); // until the kernel is done
   d.F = csr_view(A, false, slices.get());
   d.B = csr_view(A, true, slices.get());
+  pick_slices(d.F, (int64_t)ncta * (threads / 32));
+  pick_slices(d.B, (int64_t)ncta * (threads / 32));
   double **d_init = nullptr;
   std::vector<double *> hinit;
   for (int64_t i = 0; i < n_initial; i++)
@@ -470,6 +472,8 @@ int lobpcg_async_launch(LobpcgAsync *a, cudaStream_t s) {
   a->slices = hold_slices(a->req.A);
   d.F = csr_view(a->req.A, false, a->slices.get());
   d.B = csr_view(a->req.A, true, a->slices.get());
+  pick_slices(d.F, (int64_t)a->ncta * 16); // blocks of 512 threads
+  pick_slices(d.B, (int64_t)a->ncta * 16);
   d.rng = nullptr;
   lobpcg_layout(a->m, a->n, a->bs, a->k_target, a->pmax, a->ncta, p, &d);
   p += kr_round_up((int64_t)a->layout_bytes, 256);

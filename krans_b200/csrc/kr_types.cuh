@@ -65,6 +65,22 @@ struct CsrView {
   SlicedView sl;
 };
 
+// Leaves a team of `nwarps` warps without the slices of an operand that it reads
+// better by rows. Few slices of long rows leave most warps of a wide team idle, where
+// several lanes a row would use them (us a product, slices / lanes: 5400 rows of 1 to
+// 64 entries on the whole GPU 15.1 / 14.3, on 16 blocks 12.3 / 16.8; 1500 rows of 48 on
+// 16 blocks 16.9 / 15.0; 27000 rows of 64 on the whole GPU 20.2 / 22.6; 5400 rows of 16
+// there 11.5 / 14.8). Rows of about one entry leave a lane one load in flight, and one
+// block has few warps to hide it (a product and its transpose with 5400 entries, 6000
+// columns: 11.4 / 9.4 on one block, 5.0 / 6.0 on 16). Decided where a request meets its
+// team: asked in every product, it cost a batch of small requests 4%.
+__host__ __device__ inline void pick_slices(CsrView &V, int64_t nwarps) {
+  const bool few = V.lanes >= 16 && 4 * (int64_t)V.sl.slices < nwarps;
+  const bool flat = nwarps <= 32 && V.sl.longest <= 8 && 2 * V.nnz < 3 * V.rows;
+  if (few || flat)
+    V.sl.slices = 0;
+}
+
 struct CyclicDevResult {
   int64_t n_found;
   int64_t restarts, krylov_steps_total, cg_solves, cg_maxit_hits, spmv, spmvT;
