@@ -782,9 +782,9 @@ bool krans_server::admit_lobpcg(uint64_t id, Clock::time_point now) {
   if (ew == cudaSuccess)
     ew = cudaStreamWaitEvent(streams[fs], ctx_ready, 0);
   rc = ew == cudaSuccess ? lobpcg_async_launch(a, streams[fs]) : cuda_fail(ew, "server stream order", __FILE__, __LINE__);
-  if (rc == KRANS_ERR_OUT_OF_MEMORY && !inflight.empty()) {
+  if (rc == KRANS_ERR_OUT_OF_MEMORY && !ctx->budget && !inflight.empty()) {
     lobpcg_async_release(a, &graveyard);
-    return false; // the launches in flight hold what it lacks, copies of their matrices among it
+    return false; // the device is full: the launches in flight hold copies of their matrices (none with a budget)
   }
   queue.pop_front();
   if (rc != KRANS_OK) {
@@ -907,7 +907,7 @@ bool krans_server::admit_cyclic(Clock::time_point now) {
   if (ew == cudaSuccess)
     ew = cudaStreamWaitEvent(streams[fs], ctx_ready, 0);
   rc = ew == cudaSuccess ? f->L.alloc_and_launch(streams[fs]) : cuda_fail(ew, "server stream order", __FILE__, __LINE__);
-  if (rc == KRANS_ERR_OUT_OF_MEMORY && !inflight.empty()) {
+  if (rc == KRANS_ERR_OUT_OF_MEMORY && !ctx->budget && !inflight.empty()) {
     // as for a LOBPCG request: wait for the launches in flight
     for (auto it = take.rbegin(); it != take.rend(); ++it)
       queue.push_front(*it);

@@ -45,15 +45,32 @@ static int budget_fail(krans_ctx *ctx, size_t bytes) {
 }
 
 static bool give_back(krans_ctx *ctx);
+// Both forms of a device allocation: once more if the context had something to
+// give back. An error is the caller's to report: the next launch's check must
+// not find it.
+cudaError_t dev_malloc(krans_ctx *ctx, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && give_back(ctx))
+    e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess)
+    cudaGetLastError();
+  return e;
+}
+static cudaError_t stream_malloc(krans_ctx *ctx, void **p, size_t bytes, cudaStream_t s) {
+  cudaError_t e = cudaMallocAsync(p, bytes, s);
+  if (e == cudaErrorMemoryAllocation && give_back(ctx))
+    e = cudaMallocAsync(p, bytes, s);
+  if (e != cudaSuccess)
+    cudaGetLastError();
+  return e;
+}
 int dev_alloc(krans_ctx *ctx, void **p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0)
     bytes = 256;
   if (over_budget(ctx, bytes))
     return budget_fail(ctx, bytes);
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && give_back(ctx))
-    e = cudaMalloc(p, bytes);
+  const cudaError_t e = dev_malloc(ctx, p, bytes);
   if (e != cudaSuccess)
     return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
   ctx->in_use.fetch_add(bytes);
@@ -79,9 +96,16 @@ static bool ws_release(krans_ctx *ctx) { // true if there was idle scratch
   return true;
 }
 
+static uint64_t pool_bytes(krans_ctx *ctx, cudaMemPoolAttr what) {
+  uint64_t v = 0;
+  if (!ctx->pool || cudaMemPoolGetAttribute(ctx->pool, what, &v) != cudaSuccess)
+    return 0;
+  return v;
+}
+
 // When the device has no room: what the context holds beyond its callers' own
-// allocations goes back, from the stream-ordered pool to the device. False if
-// there was nothing.
+// allocations goes back, from the context's pool to the device. False if there
+// was nothing.
 static bool give_back(krans_ctx *ctx) {
   cudaGetLastError(); // the failed allocation's
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -97,12 +121,10 @@ static bool give_back(krans_ctx *ctx) {
           any = true;
         }
   }
-  if (!any)
+  if (!any && pool_bytes(ctx, cudaMemPoolAttrReservedMemCurrent) <= pool_bytes(ctx, cudaMemPoolAttrUsedMemCurrent))
     return false;
   cudaStreamSynchronize(ctx->stream);
-  cudaMemPool_t pool;
-  if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess)
-    cudaMemPoolTrimTo(pool, 0);
+  cudaMemPoolTrimTo(ctx->pool, 0);
   return true;
 }
 
@@ -115,7 +137,7 @@ static std::shared_ptr<SpeedCopy> copy_alloc(krans_ctx *ctx, size_t bytes) {
   char *p = nullptr;
   if (ctx->budget)
     return nullptr;
-  if (cudaMallocAsync((void **)&p, bytes, ctx->stream) != cudaSuccess) {
+  if (cudaMallocFromPoolAsync((void **)&p, bytes, ctx->pool, ctx->stream) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
@@ -136,7 +158,7 @@ int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, WsOwn own) {
         // grown by half again, so that a run of growing calls reallocates a few times only
         const size_t want = std::min(kWsKeep, std::max(bytes + bytes / 2, (size_t)1 << 20));
         ws_drop(ctx);
-        if (cudaMallocAsync((void **)&ctx->ws, want, ctx->stream) == cudaSuccess) {
+        if (cudaMallocFromPoolAsync((void **)&ctx->ws, want, ctx->pool, ctx->stream) == cudaSuccess) {
           ctx->ws_bytes = want;
           ctx->in_use.fetch_add(want);
         } else {
@@ -154,7 +176,7 @@ int ws_take(krans_ctx *ctx, size_t bytes, WsHold *w, WsOwn own) {
     }
   }
   if (own == WsOwn::kUncounted) {
-    KR_CUDA(cudaMallocAsync(&w->p, bytes, ctx->stream));
+    KR_CUDA(stream_malloc(ctx, &w->p, bytes, ctx->stream));
     w->mode = WsHold::kOwnUncounted;
     return KRANS_OK;
   }
@@ -196,9 +218,7 @@ int dev_alloc_async(krans_ctx *ctx, void **p, size_t bytes, cudaStream_t s) {
     bytes = 256;
   if (over_budget(ctx, bytes))
     return budget_fail(ctx, bytes);
-  cudaError_t e = cudaMallocAsync(p, bytes, s);
-  if (e == cudaErrorMemoryAllocation && give_back(ctx))
-    e = cudaMallocAsync(p, bytes, s);
+  const cudaError_t e = stream_malloc(ctx, p, bytes, s);
   if (e != cudaSuccess)
     return cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
   ctx->in_use.fetch_add(bytes);
@@ -481,7 +501,7 @@ __global__ void part_count_kernel(int64_t rows, const int32_t *rp, const int32_t
     cnt[r] = first_from(ci, b, rp[r + 1], c1) - b;
   }
 }
-// the part's entries; `at`: entries of the earlier parts, added to its row pointers
+// the part's entries, where its row pointers say (they count the entries of the earlier parts too)
 __global__ void part_fill_kernel(int64_t rows, const int32_t *rp, const int32_t *ci, const double *v, int64_t c0,
                                  const int32_t *prp, int32_t *pci, double *pv, float *pv32) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
@@ -752,6 +772,17 @@ int krans_ctx_create(int device, size_t hbm_budget_bytes, krans_ctx **out) {
     return KRANS_ERR_RUNTIME;
   }
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    e = cudaMemPoolCreate(&c->pool, &props);
+  }
+  if (e == cudaSuccess) {
+    uint64_t never = ~0ull; // given back by hand
+    e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &never);
+  }
   if (e == cudaSuccess)
     e = cudaMallocHost(&c->h_scalar, 64 * sizeof(double));
   c->partial_blocks = c->sms * 8;
@@ -792,6 +823,10 @@ int krans_ctx_destroy(krans_ctx *ctx) {
     cudaFree(ctx->d_scalar);
   if (ctx->d_partials)
     cudaFree(ctx->d_partials);
+  if (ctx->stream)
+    cudaStreamSynchronize(ctx->stream); // the scratch is free
+  if (ctx->pool)
+    cudaMemPoolDestroy(ctx->pool);
   if (ctx->stream)
     cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -1165,7 +1200,13 @@ int krans_csr_destroy(krans_mat *A) {
     auto &all = A->ctx->copied;
     all.erase(std::remove(all.begin(), all.end(), A), all.end());
   }
-  dev_free(A->ctx, A->base, A->bytes);
+  krans_ctx *ctx = A->ctx;
+  const bool copies = A->slices || A->cut;
+  A->slices.reset();
+  A->cut.reset();
+  dev_free(ctx, A->base, A->bytes); // waits for the device
+  if (copies && cudaStreamSynchronize(ctx->stream) == cudaSuccess) // which tells the pool that the copies are free
+    cudaMemPoolTrimTo(ctx->pool, (size_t)pool_bytes(ctx, cudaMemPoolAttrUsedMemCurrent) + kPoolKeep);
   delete A;
   return KRANS_OK;
 }

@@ -70,6 +70,7 @@ struct krans_ctx {
   std::mutex mu;
   // Kept scratch of the calls that work on the context's stream (see ws_take)
   std::mutex ws_mu;
+  cudaMemPool_t pool = nullptr; // of the kept scratch and of the second copies of matrices (see kPoolKeep)
   char *ws = nullptr;
   size_t ws_bytes = 0;
   bool ws_busy = false;
@@ -162,6 +163,7 @@ int spmv_rows_per_block(int64_t rows, int64_t nnz);
 // allocation with budget accounting
 bool over_budget(const krans_ctx *ctx, size_t bytes); // these on top of what is allocated
 int dev_alloc(krans_ctx *ctx, void **p, size_t bytes);
+cudaError_t dev_malloc(krans_ctx *ctx, void **p, size_t bytes); // without the budget
 void dev_free(krans_ctx *ctx, void *p, size_t bytes);
 // Scratch of one call on the context's stream, kept from call to call: a
 // cudaMalloc and cudaFree per call cost 0.3 ms and more (the three block products
@@ -173,6 +175,12 @@ void dev_free(krans_ctx *ctx, void *p, size_t bytes);
 // device before an allocation fails. A context with a budget keeps none: it
 // would count against calls that fit beside what the callers themselves hold.
 constexpr size_t kWsKeep = (size_t)256 << 20;
+// The kept scratch and the second copies come from a pool of the context's own. The
+// device's default pool gives freed memory back at the next wait of a stream,
+// whoever's: the first product after a matrix of 16.8M rows was destroyed took 48
+// ms. This one keeps kPoolKeep unused bytes, gives back what is above when a matrix
+// is destroyed, and all of it when the device is full.
+constexpr size_t kPoolKeep = (size_t)64 << 20;
 struct WsHold {
   void *p = nullptr;
   size_t bytes = 0;

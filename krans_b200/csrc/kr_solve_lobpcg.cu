@@ -236,7 +236,7 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
   cudaStream_t s = ctx->stream;
   cudaError_t e = cudaSuccess;
   if (n_initial > 0) {
-    e = cudaMalloc(&d_init, sizeof(double *) * (size_t)n_initial);
+    e = dev_malloc(ctx, (void **)&d_init, sizeof(double *) * (size_t)n_initial);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(d_init, hinit.data(), sizeof(double *) * (size_t)n_initial, cudaMemcpyHostToDevice, s);
   }
@@ -255,7 +255,7 @@ extern "C" int krans_solve_lobpcg(krans_ctx *ctx, const krans_mat *A, krans_rng 
   if (e == cudaSuccess)
     e = cudaEventRecord(e0, s);
   if (e == cudaSuccess && team != KRANS_TEAM_GRID) {
-    e = cudaMalloc(&d_desc, sizeof(LobpcgDesc));
+    e = dev_malloc(ctx, (void **)&d_desc, sizeof(LobpcgDesc));
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(d_desc, &d, sizeof d, cudaMemcpyHostToDevice, s);
   }

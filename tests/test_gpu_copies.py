@@ -63,3 +63,20 @@ def test_slices_without_more_than_seven_padded_entries_for_each_real_one():
     # at most 8 entries of 12 bytes in a slice for each one, a row number a slot and a bound a slice, of both operands
     assert ctx.memory_in_use() - before - plain - scratch <= 2 * 8 * 12 * A.nnz + 5 * (m + n) + 4096
     del M
+
+
+def test_destroyed_matrices_leave_a_bounded_pool():
+    """What the context's pool keeps unused after a matrix is gone: its scratch and 64 MB, not the copies."""
+    import torch
+    import krans_b200 as kb
+    ctx = kb.Context(0)
+    m, n = 1_500_000, 1_000_000
+    A = _ragged(m, n, 9)  # 12M entries: 290 MB of slices, 300 MB of arrays, 145 MB of scratch grown by half
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    M = kb.CudaCsrMatrixAdapter.from_scipy(ctx, A)
+    during = torch.cuda.mem_get_info()[0]
+    assert before - during > (500 << 20)
+    del M
+    assert before - torch.cuda.mem_get_info()[0] <= ctx.memory_in_use() + (64 << 20) + (96 << 20)
