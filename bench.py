@@ -130,12 +130,10 @@ def measured_peak():
 
 
 # DRAM bytes (read + write) per algorithmic byte of the batched launch, taken
-# from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# batched kernel on a 64-instance batch of this workload, whose matrices
-# exceed L2. `traffic` scales it to this launch. The capture was made before
-# the CG of the incidence and shift operators carried F^T p only, and before
-# the sorted slices: an estimate for the present kernels.
-DRAM_PER_ALGO_BYTE = 1.607e12 / 3.966e12
+# from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum, one pass)
+# of the batched kernels on 64 instances of this workload's kinds with n up to
+# 1e5, whose matrices exceed L2 together. `traffic` scales it to this launch.
+DRAM_PER_ALGO_BYTE = 0.3739e12 / 2.2687e12
 
 
 # ---------------------------------------------------------------------------

@@ -59,7 +59,9 @@ int krans_abi_sizes(int64_t *out, int capacity);
 
 /* ---- context --------------------------------------------------------------- */
 /* Opens `device`, creates the context's stream. hbm_budget_bytes = 0 means
- * no budget beyond the device's free memory. */
+ * no budget beyond the device's free memory. A budget counts what the calls ask
+ * for; scratch between calls and second copies of matrices for speed are kept
+ * only without one, and go back when the device is full. */
 int krans_ctx_create(int device, size_t hbm_budget_bytes, krans_ctx **out);
 int krans_ctx_destroy(krans_ctx *ctx);
 int krans_ctx_synchronize(krans_ctx *ctx);
@@ -231,7 +233,10 @@ int krans_rng_seed(const krans_rng *r, uint32_t *seed);
 #define KRANS_PREC_FP64 0  /* plain FP64 throughout */
 #define KRANS_PREC_MIXED 1 /* FP32 SpMV + Krylov recurrence, FP64 reorth/tiny/polish */
 
-#define KRANS_TEAM_AUTO 0 /* pick by problem size */
+/* Teams sum in other orders, so a solve's results differ by rounding from team to
+ * team: name the team where they must not. */
+#define KRANS_TEAM_AUTO 0 /* pick by problem size; one block below m + n = 120000 while a server lives on the
+                             device, and where there is no room for a larger team's partial sums */
 #define KRANS_TEAM_CTA 1  /* one thread block runs the solve */
 #define KRANS_TEAM_GRID 2 /* the whole GPU runs the solve (cooperative launch) */
 
@@ -422,8 +427,10 @@ int krans_solve_batch(krans_ctx *ctx, int64_t count, const krans_request *reqs,
  *   lanes[6]      threads per row of the solvers' SpMV for operands whose mean
  *                 row length is <= 3, <= 8, <= 16, <= 32, <= 64, > 64
  *                 (1, 2, 4, 8, 16, 32); powers of two up to 32. Operands whose
- *                 rows hold at most 64 entries each are read one row per
- *                 lane whatever the table says.
+ *                 rows hold at most 64 entries each are mostly read one row per
+ *                 lane, from a second copy of their entries, whatever the table
+ *                 says: not where the copy would be mostly padding, where there
+ *                 is no room for it, or in a context with a budget.
  * The lanes apply to every solve of the context (single and batched); a
  * request's rounding depends on them, so results are reproducible for a
  * given table. */
