@@ -513,10 +513,14 @@ struct BatchLaunch {
   }
 
   // stop a published request: its team sees the status word at its next
-  // check and unwinds (copied on `ctl`, beside the running kernel)
+  // check and unwinds (copied on `ctl`, beside the running kernel, but after the
+  // launch's set-up, which clears the words: a request cancelled as soon as its
+  // launch was queued would run to its end)
   int cancel_slot(int g, cudaStream_t ctl) const {
     static const int32_t cancelled = KRANS_ERR_CANCELLED;
-    cudaError_t e = cudaMemcpyAsync(d_status + g, &cancelled, 4, cudaMemcpyHostToDevice, ctl);
+    cudaError_t e = cudaStreamWaitEvent(ctl, ev0, 0);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(d_status + g, &cancelled, 4, cudaMemcpyHostToDevice, ctl);
     return e == cudaSuccess ? KRANS_OK : cuda_fail(e, "cancel request", __FILE__, __LINE__);
   }
 
